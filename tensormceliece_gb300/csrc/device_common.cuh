@@ -1,5 +1,5 @@
 // Device primitives shared by the encapsulation and decapsulation kernels:
-// Keccak-f[1600] / SHAKE256 (thread-per-request), GF(2^m) log/antilog helpers.
+// Keccak-f[1600] on one lane, two lanes or a warp, the KEM hash, GF(2^m) log/antilog helpers.
 #pragma once
 #include <stdint.h>
 #include <cuda_runtime.h>
@@ -91,140 +91,209 @@ __device__ __forceinline__ void keccak_f1600(uint64_t A[25]) {
   }
 }
 
-// SHAKE256 of a message of compile-time length LEN bytes whose 8-byte
-// little-endian lanes are produced by lane(i) (bytes past LEN must read as 0).
-// Rate 17 lanes, domain byte 0x1F, final bit 0x80. Writes the first 32
-// output bytes as 4 lanes.
-template <int LEN, typename LaneFn>
-__device__ __forceinline__ void shake256_32(uint64_t out[4], LaneFn lane) {
-  constexpr int nfull = LEN / 136;           // full blocks
-  constexpr int rem = LEN - nfull * 136;     // bytes in the final block
-  uint64_t s[25];
-#pragma unroll
-  for (int i = 0; i < 25; i++) s[i] = 0;
+// Keccak-f[1600] on two neighbouring lanes: lane 2s + h of a warp holds the
+// low (h = 0) or high (h = 1) 32 bits of all 25 words of state s, so a rotation
+// takes the other half from the neighbour (one shuffle) and every other step is
+// lane-local. All 32 lanes must call. A lone permutation is bound by its own
+// instruction stream (180 ALU instructions a round at one per two cycles): the
+// pair form issues half of them per lane. 10 permutations measured on one GPU:
+// 38 us against 54 us for the one-lane form up to 4096 states, 172 against
+// 196 us for 65536 (a finer grain over the four schedulers of each SM). The
+// 29 shuffles a round run in their own pipe. Rotations by IMAD (multiply by a
+// power of two) instead of funnel shifts were slower in either form.
+__device__ __forceinline__ void keccak_f1600_pair(uint32_t (&A)[25], int half) {
+  constexpr int off[25] = {0,  1,  62, 28, 27, 36, 44, 6,  55, 20, 3,  10, 43,
+                           25, 39, 41, 45, 15, 21, 8,  18, 2,  61, 56, 14};
 #pragma unroll 1
-  for (int b = 0; b < nfull; b++) {
+  for (int round = 0; round < 24; ++round) {
+    uint32_t C[5], R[5], B[25];
 #pragma unroll
-    for (int i = 0; i < 17; i++) s[i] ^= lane(b * 17 + i);
-    keccak_f1600(s);
+    for (int x = 0; x < 5; x++) C[x] = A[x] ^ A[x + 5] ^ A[x + 10] ^ A[x + 15] ^ A[x + 20];
+#pragma unroll
+    for (int x = 0; x < 5; x++) R[x] = __funnelshift_l(__shfl_xor_sync(0xffffffffu, C[x], 1), C[x], 1);
+#pragma unroll
+    for (int y = 0; y < 5; y++)
+#pragma unroll
+      for (int x = 0; x < 5; x++) {
+        const uint32_t v = A[x + 5 * y] ^ C[(x + 4) % 5] ^ R[(x + 1) % 5];
+        const int r = off[x + 5 * y];
+        uint32_t w = v;
+        if (r) {
+          const uint32_t o = __shfl_xor_sync(0xffffffffu, v, 1);
+          w = r < 32 ? __funnelshift_l(o, v, r) : __funnelshift_l(v, o, r - 32);
+        }
+        B[y + 5 * ((2 * x + 3 * y) % 5)] = w;
+      }
+#pragma unroll
+    for (int y = 0; y < 5; y++)
+#pragma unroll
+      for (int x = 0; x < 5; x++)
+        A[x + 5 * y] = B[x + 5 * y] ^ (~B[(x + 1) % 5 + 5 * y] & B[(x + 2) % 5 + 5 * y]);
+    const uint64_t rc = c_keccak_rc[round];
+    A[0] ^= half ? (uint32_t)(rc >> 32) : (uint32_t)rc;
   }
-#pragma unroll
-  for (int i = 0; i < 17; i++) {
-    if (8 * i < rem) s[i] ^= lane(nfull * 17 + i);
-    if (i == rem / 8) s[i] ^= 0x1Full << (8 * (rem % 8));
-  }
-  s[16] ^= 0x8000000000000000ull;
-  keccak_f1600(s);
-#pragma unroll
-  for (int i = 0; i < 4; i++) out[i] = s[i];
 }
 
-// ---------------------------------------------------------------- KEM hash preimage
-// 8 bytes of a little-endian word stream from byte offset off >= 0.
-template <typename WordFn>
-__device__ __forceinline__ uint64_t stream_u64(WordFn word, int off) {
-  const int w = off >> 2, sh = 8 * (off & 3);
-  uint64_t v = (uint64_t)word(w) | ((uint64_t)word(w + 1) << 32);
-  if (sh) v = (v >> sh) | ((uint64_t)word(w + 2) << (64 - sh));
-  return v;
-}
-
-// Lane i (bytes 8i .. 8i+7) of the session-key preimage b || e || c, where e
-// has EB bytes given as 32-bit words by eword and c is given as 32-bit words
-// by cword (zero past its length). Lanes inside e or inside c are funnels of
-// three words; only the lane holding the e/c boundary is assembled bytewise.
-template <int EB, typename EWord, typename CWord>
-__device__ __forceinline__ uint64_t kem_preimage_lane(int i, uint32_t b, EWord eword, CWord cword) {
-  const int o = 8 * i;
-  if (o == 0) return (uint64_t)b | (stream_u64(eword, 0) << 8);
-  if (o + 7 <= EB) return stream_u64(eword, o - 1);
-  if (o >= 1 + EB) return stream_u64(cword, o - 1 - EB);
-  uint64_t v = 0;
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const int x = o + k - 1;  // byte of e || c
-    const uint32_t byte = x < EB ? (eword(x >> 2) >> (8 * (x & 3))) : (cword((x - EB) >> 2) >> (8 * ((x - EB) & 3)));
-    v |= (uint64_t)(byte & 0xFFu) << (8 * k);
-  }
-  return v;
-}
-
-// SHAKE256 (first 32 output bytes) of the KEM preimage b || e || c of PRE
-// bytes, e of EB bytes, for the 32 requests of a warp (one per lane; every
-// lane of the warp must call). erow is this lane's e as 32-bit words (zero
-// past EB up to the next word); cword gives c as words (zero past c).
-// The e words of each 136-byte absorb block are loaded for the whole warp as
-// 35 independent loads per lane (word j of every request, and words 32..34 of
-// the lane's own request), issued before the previous block is permuted so
-// they land under the permutation, and handed over through shared memory
-// (stage: 32 x 35 words, odd stride: no bank conflicts; rows: 32 pointers).
-// Lanes outside e (the first, the e/c boundary, c) use kem_preimage_lane.
-constexpr int kStageStride = 35;
-template <int EB, int PRE, typename CWord>
-__device__ __forceinline__ void kem_hash_staged(uint64_t out[4], uint32_t b, const uint32_t *erow, CWord cword,
-                                                uint32_t *stage, const uint32_t **rows) {
-  constexpr int EW = (EB + 3) / 4;
-  constexpr int NB = PRE / 136 + 1;  // full blocks and the final (padded) one
-  const int lane = threadIdx.x & 31;
-  auto eword = [&](int w) -> uint32_t { return erow[w]; };
-  rows[lane] = erow;
-  __syncwarp();
-  auto w_lo_of = [](int blk) { return blk > 0 ? (136 * blk - 1) >> 2 : 0; };
-  uint32_t pf[32], pf2[3];
-  auto prefetch = [&](int blk) {
-    const int w_lo = w_lo_of(blk);
-#pragma unroll
-    for (int r = 0; r < 32; r++) {
-      const int w = w_lo + lane;
-      pf[r] = w < EW ? rows[r][w] : 0u;
+// Keccak-f[1600] on a whole warp: lane x + 5y holds word (x, y) (lanes 25..31
+// repeat lane 0). The lowest latency per permutation (10 in 30 us against 38 us
+// for the pair form and 54 us for the one-lane form), at 6 times their
+// instructions per state: for launches that leave most of the GPU idle.
+struct KeccakWarp {
+  int s1, s2, s3, s4;  // the other words of this word's column
+  int xm, xp;          // a word of columns x - 1 and x + 1
+  int g0, g1, g2;      // before pi: the words that become (x, y), (x + 1, y), (x + 2, y)
+  int rot;             // rho offset
+  bool first;          // word (0, 0)
+  __device__ explicit KeccakWarp(int lane) {
+    const int l = lane < 25 ? lane : 0, x = l % 5, y = l / 5;
+    s1 = x + 5 * ((y + 1) % 5);
+    s2 = x + 5 * ((y + 2) % 5);
+    s3 = x + 5 * ((y + 3) % 5);
+    s4 = x + 5 * ((y + 4) % 5);
+    xm = (x + 4) % 5 + 5 * y;
+    xp = (x + 1) % 5 + 5 * y;
+    g0 = source(x, y);
+    g1 = source((x + 1) % 5, y);
+    g2 = source((x + 2) % 5, y);
+    // rho's walk: (1, 0), then (x, y) -> (y, 2x + 3y), offsets (t + 1)(t + 2) / 2
+    rot = 0;
+    int wx = 1, wy = 0;
+    for (int t = 0; t < 24; t++) {
+      if (wx == x && wy == y) rot = ((t + 1) * (t + 2) / 2) & 63;
+      const int nx = wy, ny = (2 * wx + 3 * wy) % 5;
+      wx = nx;
+      wy = ny;
     }
+    first = l == 0;
+  }
+  // the word that pi moves to (X, Y): (x, y) -> (y, 2x + 3y), so y = X and x = (Y - 3X) / 2 mod 5
+  static __device__ int source(int X, int Y) { return ((Y - 3 * X + 15) * 3) % 5 + 5 * X; }
+  __device__ __forceinline__ void permute(uint64_t &a) const {
+    const int r = rot & 31;
+    const bool swap = rot >= 32;
+#pragma unroll 1
+    for (int round = 0; round < 24; ++round) {
+      const uint64_t C = a ^ sh(a, s1) ^ sh(a, s2) ^ sh(a, s3) ^ sh(a, s4);
+      const uint64_t cm = sh(C, xm), cp = sh(C, xp);
+      const uint64_t v = a ^ cm ^ rotl64(cp, 1);
+      const uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32), p = swap ? hi : lo, q = swap ? lo : hi;
+      const uint64_t b = (uint64_t)__funnelshift_l(q, p, r) | ((uint64_t)__funnelshift_l(p, q, r) << 32);
+      a = sh(b, g0) ^ (~sh(b, g1) & sh(b, g2));
+      if (first) a ^= c_keccak_rc[round];
+    }
+  }
+  static __device__ __forceinline__ uint64_t sh(uint64_t v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+};
+
+// ---------------------------------------------------------------- KEM hash
+// The hash preimage is b || e || c: 32-bit word j of it is the funnel of words
+// j - 1 and j of the stream e || c (word -1: b in its top byte). A source Src
+// gives the stream of one request:
+//   e(w)  word w of e (bits past EB bytes are zero)
+//   c(w)  word w of c (zero past c)
+// Words are loaded a block of 34 ahead of the permutation that absorbs them.
+template <int EB, typename Src>
+__device__ __forceinline__ uint32_t kem_stream_word(const Src &src, int w) {
+  constexpr int EW = EB / 4;
+  static_assert(EB % 4 == 0 || EB % 4 == 2, "e ends on a half word");
+  if (w < EW) return src.e(w);
+  if (EB % 4 == 0) return src.c(w - EW);
+  if (w == EW) return src.e(w) | (src.c(0) << 16);
+  return (src.c(w - EW - 1) >> 16) | (src.c(w - EW) << 16);
+}
+
+template <int EB, typename Src>
+__device__ __forceinline__ uint2 kem_stream_pair(const Src &src, int w) {
+  return make_uint2(kem_stream_word<EB>(src, w), kem_stream_word<EB>(src, w + 1));
+}
+
+// e alone (the plaintext-confirmation hash)
+struct EncOnlySrc {
+  const uint32_t *er;
+  __device__ uint32_t e(int w) const { return er[w]; }
+  __device__ uint32_t c(int) const { return 0u; }
+};
+
+// SHAKE256 (first 32 output bytes) of b || e || c, PRE bytes, two lanes per
+// request (keccak_f1600_pair; every lane of the warp must call): lane half h
+// returns the output's 32-bit words 2i + h in out[i].
+template <int EB, int PRE, typename Src>
+__device__ __forceinline__ void kem_hash_pair(uint32_t (&out)[4], uint32_t b, const Src &src, int half) {
+  constexpr int NB = PRE / 136 + 1, rem = PRE % 136;
+  uint32_t A[25];
 #pragma unroll
-    for (int e = 0; e < 3; e++) {
-      const int w = w_lo + 32 + e;
-      pf2[e] = w < EW ? erow[w] : 0u;
+  for (int i = 0; i < 25; i++) A[i] = 0;
+  uint32_t cur[17];  // this lane's words 2i + half of the block
+  auto load = [&](int blk) {
+    if (34 * (blk + 1) <= EB / 4) {
+#pragma unroll
+      for (int i = 0; i < 17; i++) cur[i] = src.e(34 * blk + 2 * i + half);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 17; i++) cur[i] = kem_stream_word<EB>(src, 34 * blk + 2 * i + half);
     }
   };
-  prefetch(0);
-  uint64_t s[25];
-#pragma unroll
-  for (int i = 0; i < 25; i++) s[i] = 0;
+  load(0);
+  uint32_t prev = b << 24;  // the neighbour's last word (of use to half 0: its word 2i - 1)
 #pragma unroll 1
   for (int blk = 0; blk < NB; blk++) {
-    const int x0 = 136 * blk;
-    const int w_lo = w_lo_of(blk);
-    const bool in_e = x0 - 1 < EB;
-    if (in_e) {
-#pragma unroll
-      for (int r = 0; r < 32; r++) stage[r * kStageStride + lane] = pf[r];
-#pragma unroll
-      for (int e = 0; e < 3; e++) stage[lane * kStageStride + 32 + e] = pf2[e];
-      __syncwarp();
-      if (blk + 1 < NB && 136 * (blk + 1) - 1 < EB) prefetch(blk + 1);
-    }
-    const int rem = (blk == NB - 1) ? PRE % 136 : 136;  // preimage bytes in this block
-    const uint32_t *mine = stage + lane * kStageStride;
 #pragma unroll
     for (int i = 0; i < 17; i++) {
-      const int L = 17 * blk + i, o = 8 * L;
-      uint64_t v = 0;
-      if (8 * i < rem) {
-        if (o > 0 && o + 7 <= EB) {
-          const int rel = (o - 1) - 4 * w_lo, q = rel >> 2, sh = 8 * (rel & 3);
-          v = (uint64_t)mine[q] | ((uint64_t)mine[q + 1] << 32);
-          if (sh) v = (v >> sh) | ((uint64_t)mine[q + 2] << (64 - sh));
-        } else {
-          v = kem_preimage_lane<EB>(L, b, eword, cword);
-        }
-      }
-      if (blk == NB - 1 && i == rem / 8) v ^= 0x1Full << (8 * (rem % 8));
-      s[i] ^= v;
+      const uint32_t o = __shfl_xor_sync(0xffffffffu, cur[i], 1);
+      A[i] ^= __funnelshift_l(half ? o : prev, cur[i], 8);
+      prev = o;
     }
-    if (blk == NB - 1) s[16] ^= 0x8000000000000000ull;
-    keccak_f1600(s);
-    __syncwarp();  // every lane has read the staged words before they are replaced
+    if (blk + 1 < NB) {
+      load(blk + 1);
+    } else {
+      if (half == (rem % 8) / 4) A[rem / 8] ^= 0x1Fu << (8 * (rem % 4));
+      if (half) A[16] ^= 0x80000000u;
+    }
+    keccak_f1600_pair(A, half);
   }
 #pragma unroll
-  for (int i = 0; i < 4; i++) out[i] = s[i];
+  for (int i = 0; i < 4; i++) out[i] = A[i];
+}
+
+// The same with a warp per request (KeccakWarp): lane i < 4 returns the output's 64-bit word i.
+template <int EB, int PRE, typename Src>
+__device__ __forceinline__ uint64_t kem_hash_warp(uint32_t b, const Src &src, int lane) {
+  constexpr int NB = PRE / 136 + 1, rem = PRE % 136;
+  const KeccakWarp kw(lane);
+  uint64_t a = 0;
+  uint2 cur = lane < 17 ? kem_stream_pair<EB>(src, 2 * lane) : make_uint2(0u, 0u);
+  uint32_t carry = b << 24;
+#pragma unroll 1
+  for (int blk = 0; blk < NB; blk++) {
+    uint32_t prev = __shfl_up_sync(0xffffffffu, cur.y, 1);
+    if (lane == 0) prev = carry;
+    carry = __shfl_sync(0xffffffffu, cur.y, 16);
+    if (lane < 17) {
+      a ^= (uint64_t)__funnelshift_l(prev, cur.x, 8) | ((uint64_t)__funnelshift_l(cur.x, cur.y, 8) << 32);
+      if (blk + 1 < NB) {
+        cur = kem_stream_pair<EB>(src, 34 * (blk + 1) + 2 * lane);
+      } else {
+        if (lane == rem / 8) a ^= 0x1Full << (8 * (rem % 8));
+        if (lane == 16) a ^= 0x8000000000000000ull;
+      }
+    }
+    kw.permute(a);
+  }
+  return a;
+}
+
+// Stores the 4 words 2i + h of a 32-byte output (v[i], lane half h) at any byte alignment.
+__device__ __forceinline__ void store_hash_words(uint8_t *dst, const uint32_t (&v)[4], int half) {
+  if ((reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
+    uint32_t *d = reinterpret_cast<uint32_t *>(dst);
+#pragma unroll
+    for (int i = 0; i < 4; i++) d[2 * i + half] = v[i];
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int k = 0; k < 4; k++) dst[4 * (2 * i + half) + k] = (uint8_t)(v[i] >> (8 * k));
+  }
 }
 
 // ---------------------------------------------------------------- GF(2^m)

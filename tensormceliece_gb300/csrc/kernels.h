@@ -8,10 +8,11 @@ namespace gmc {
 
 constexpr int kSampleWarpsPerSM = 8;     // sampler: resident warps per SM (lanes fetch requests)
 constexpr int kSampleThreadsMax = 128;  // sampler block size is a launch parameter (32, 64 or 128)
-// hash kernels (thread per request, one wave): 64-thread blocks spread a
-// 65536-request launch as 6-7 blocks per SM (128-thread blocks: 3-4, so a
-// third of the SMs carried a block more than the rest)
+// hash kernels: 64-thread blocks, 32 requests each (two lanes per request), 14
+// of them resident per SM, so that 65536 requests run in one wave of 13-14
+// blocks per SM
 constexpr int kTailThreads = 64;
+constexpr int kTailBlocksPerSM = 14;
 constexpr int kBMWarps = 14;    // Berlekamp-Massey kernel: default and largest warps per block (32 requests per warp)
 constexpr int kBMCtWarps = 8;   // its constant-time form: largest warps per block
 constexpr int kBMLatWarps = 28;  // Berlekamp-Massey latency form: largest warps per block (one request per warp)
@@ -104,6 +105,8 @@ cudaError_t launch_gf2_gemm_tc(const GemmKeys &keys, const Segs &segs, int rows_
 cudaError_t launch_gf2_gemm_b1(const GemmKeys &keys, const Segs &segs, int lda, int rows_pad, const uint32_t *X,
                                int ldx, int kw_pad, uint32_t *Out, int ldo, int out_words, cudaStream_t st);
 Segs one_segment(long long n);
+// hash kernels: whether a launch takes a warp per request (kernels_enc.cu)
+bool hash_warp_form(const Segs &segs);
 
 // Encapsulation: seeds / C / K rows in padded row space; E, Ens, S have
 // seg_rows(segs) rows. pk_bad_mask bit s: segment s's public key has

@@ -1200,75 +1200,102 @@ __global__ void __launch_bounds__(kRootWarps * 32, 2) dec_root_kernel(const uint
 }
 
 // ---------------------------------------------------------------- tail
+// K = SHAKE256(b || (e or s) || c), s the key's n/8 bytes (stored zero-padded
+// to whole 16-byte units). The choice is a mask, not an address
+// (mc:crypto_kem/348864/vec/kem_dec.c:51-55): every word is (e & mask) |
+// (s & ~mask), with both read by the same loads whatever the outcome.
+// Two lanes per request or a warp per request, as finalize_kernel. 8192128,
+// 65536 requests: 198 us against 241 us with one lane per request; one
+// request 31 us against 86 us.
 template <int SET, bool PC>
-__global__ void __launch_bounds__(kTailThreads) dec_tail_kernel(const uint32_t *__restrict__ E, int lde,
-                                                                const int *__restrict__ okin,
-                                                                const uint8_t *__restrict__ Cin, const DecKeys keys,
-                                                                uint8_t *__restrict__ K, int *__restrict__ rc,
-                                                                const Segs segs) {
+struct DecHashSrc {
   using p = P<SET>;
-  constexpr int SB = p::synd_bytes, CB = SB + (PC ? 32 : 0);  // C0 bytes, ciphertext bytes
-  __shared__ uint32_t stage[kTailThreads / 32][32 * kStageStride];
-  __shared__ const uint32_t *rows[kTailThreads / 32][32];
-  const long long N = seg_rows(segs);
-  const long long op = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long opc = op < N ? op : N - 1;  // every lane of a warp takes part in the staged hash
-  int seg;
-  const bool live = seg_live(segs, op, &seg);
-  const DecKeyDev &key = keys.k[seg_find(segs, opc)];
-  bool ok = okin[opc] != 0;
-  const uint8_t *c = Cin + opc * CB;
-  if constexpr (PC) {
-    // plaintext confirmation (mc:crypto_kem/348864pc/vec/kem_dec.c:43-48): SHAKE256(2 || e, 32) of the
-    // decoded e must equal C1 (its value when decoding failed does not change the outcome)
-    auto none = [](int) -> uint32_t { return 0u; };
-    uint64_t cf[4];
-    kem_hash_staged<p::e_bytes, 1 + p::e_bytes>(cf, 2u, E + opc * lde, none, stage[threadIdx.x >> 5],
-                                                rows[threadIdx.x >> 5]);
-    uint32_t diff = 0;
-#pragma unroll
-    for (int j = 0; j < 32; j++) diff |= (uint32_t)c[SB + j] ^ ((uint32_t)(cf[j >> 3] >> (8 * (j & 7))) & 0xFFu);
-    ok = ok && diff == 0;
-  }
-  // b || (e or s) || c, s the key's n/8 bytes (stored zero-padded to whole words). The choice is a
-  // mask, not an address (mc:crypto_kem/348864/vec/kem_dec.c:51-55): the warp rewrites each of its
-  // 32 rows as (e & mask) | (s & ~mask), reading both e and s with the same coalesced loads whatever
-  // the outcome, and every lane hashes its own (blended) row.
-  {
-    const unsigned okmask = __ballot_sync(0xffffffffu, ok);
-    const long long g0 = opc - (threadIdx.x & 31);  // the warp's first row (clamped rows repeat N-1)
-    for (int r = 0; r < 32; r++) {
-      const long long row = g0 + r < N ? g0 + r : N - 1;
-      const uint32_t m = ((okmask >> r) & 1u) ? 0xFFFFFFFFu : 0u;
-      const uint32_t *sr = reinterpret_cast<const uint32_t *>(keys.k[seg_find(segs, row)].s);
-      uint32_t *er = const_cast<uint32_t *>(E) + row * lde;
-      for (int w = threadIdx.x & 31; w < p::ew; w += 32) er[w] = (er[w] & m) | (sr[w] & ~m);
-    }
-    __syncwarp();
-  }
-  const uint32_t *erow = E + opc * lde;
-  // word loads when every ciphertext row is 4-byte aligned (the buffer and the row length), else bytes
-  const bool c_words = (CB % 4 == 0) && ((reinterpret_cast<uintptr_t>(Cin) & 3) == 0);
-  auto cword = [&](int w) -> uint32_t {
-    if (c_words) return 4 * w < CB ? reinterpret_cast<const uint32_t *>(c)[w] : 0u;
+  static constexpr int CB = p::synd_bytes + (PC ? 32 : 0);
+  const uint32_t *er, *sr;
+  const uint8_t *ct;
+  uint32_t mask;
+  bool words;  // ciphertext rows on 4-byte boundaries
+  __device__ uint32_t pick(uint32_t e, uint32_t s) const { return (e & mask) | (s & ~mask); }
+  __device__ uint32_t e(int w) const { return pick(er[w], sr[w]); }
+  __device__ uint32_t c(int w) const {
+    if (4 * w >= CB) return 0u;
+    if (words) return reinterpret_cast<const uint32_t *>(ct)[w];
     uint32_t v = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++)
-      if (4 * w + k < CB) v |= (uint32_t)c[4 * w + k] << (8 * k);
+      if (4 * w + k < CB) v |= (uint32_t)ct[4 * w + k] << (8 * k);
     return v;
-  };
-  uint64_t h[4];
-  kem_hash_staged<p::e_bytes, p::pre_bytes + (PC ? 32 : 0)>(h, ok ? 1u : 0u, erow, cword, stage[threadIdx.x >> 5],
-                                                             rows[threadIdx.x >> 5]);
-  if (!live) return;
+  }
+};
+
+template <int SET, bool PC, bool WARP>
+__global__ void __launch_bounds__(kTailThreads, WARP ? 1 : PC ? kTailBlocksPerSM - 2 : kTailBlocksPerSM)
+    dec_tail_kernel(const uint32_t *__restrict__ E, int lde, const int *__restrict__ okin,
+                    const uint8_t *__restrict__ Cin, const DecKeys keys, uint8_t *__restrict__ K,
+                    int *__restrict__ rc, const Segs segs) {
+  using p = P<SET>;
+  constexpr int SB = p::synd_bytes, CB = SB + (PC ? 32 : 0);  // C0 bytes, ciphertext bytes
+  constexpr int RPW = WARP ? 1 : 16;                          // requests per warp
+  const int lane = threadIdx.x & 31, half = lane & 1;
+  const long long op0 = ((long long)blockIdx.x * (kTailThreads / 32) + (threadIdx.x >> 5)) * RPW;
+  const int r = WARP ? 0 : lane >> 1;
+  int seg;
+  const bool live = seg_live(segs, op0 + r, &seg);
+  const uint32_t livemask = __ballot_sync(0xffffffffu, live);
+  if (!livemask) return;
+  // lanes of rows that are not live hash the warp's first live row and store nothing
+  const int src_lane = live ? lane : __ffs(livemask) - 1;
+  const long long op = op0 + (WARP ? 0 : src_lane >> 1);
+  seg = __shfl_sync(0xffffffffu, seg, src_lane);
+  bool ok = okin[op] != 0;
+  const uint8_t *c = Cin + op * CB;
+  const uint32_t *erow = E + op * lde;
+  if constexpr (PC) {
+    // plaintext confirmation (mc:crypto_kem/348864pc/vec/kem_dec.c:43-48): SHAKE256(2 || e, 32) of the
+    // decoded e must equal C1 (its value when decoding failed does not change the outcome)
+    const EncOnlySrc esrc{erow};
+    uint32_t diff = 0;
+    auto c1word = [&](int j) -> uint32_t {
+      uint32_t v = 0;
+#pragma unroll
+      for (int k = 0; k < 4; k++) v |= (uint32_t)c[SB + 4 * j + k] << (8 * k);
+      return v;
+    };
+    if constexpr (WARP) {
+      const uint64_t h = kem_hash_warp<p::e_bytes, 1 + p::e_bytes>(2u, esrc, lane);
+      if (lane < 4) diff = ((uint32_t)h ^ c1word(2 * lane)) | ((uint32_t)(h >> 32) ^ c1word(2 * lane + 1));
+      diff = __reduce_or_sync(0xffffffffu, diff);
+    } else {
+      uint32_t cf[4];
+      kem_hash_pair<p::e_bytes, 1 + p::e_bytes>(cf, 2u, esrc, half);
+#pragma unroll
+      for (int i = 0; i < 4; i++) diff |= cf[i] ^ c1word(2 * i + half);
+      diff |= __shfl_xor_sync(0xffffffffu, diff, 1);
+    }
+    ok = ok && diff == 0;
+  }
+  const DecHashSrc<SET, PC> src{erow, reinterpret_cast<const uint32_t *>(keys.k[seg].s), c, ok ? 0xFFFFFFFFu : 0u,
+                                (CB % 4 == 0) && ((reinterpret_cast<uintptr_t>(Cin) & 3) == 0)};
+  uint32_t h[4];
+  if constexpr (WARP) {
+    const uint64_t hw = kem_hash_warp<p::e_bytes, p::pre_bytes + (PC ? 32 : 0)>(ok ? 1u : 0u, src, lane);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint64_t v = __shfl_sync(0xffffffffu, hw, i);
+      h[i] = half ? (uint32_t)(v >> 32) : (uint32_t)v;
+    }
+  } else {
+    kem_hash_pair<p::e_bytes, p::pre_bytes + (PC ? 32 : 0)>(h, ok ? 1u : 0u, src, half);
+  }
+  if (!live || (WARP && lane >= 2)) return;
   bool pad_bad = false;
   if (p::mt % 8) pad_bad = (c[SB - 1] >> (p::mt % 8)) != 0;
-  uint8_t *k = K + op * 32;
+  if (pad_bad) {
 #pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int bb = 0; bb < 8; bb++) k[8 * i + bb] = pad_bad ? 0xFF : (uint8_t)(h[i] >> (8 * bb));
-  if (rc) rc[op] = pad_bad ? -1 : 0;
+    for (int i = 0; i < 4; i++) h[i] = 0xFFFFFFFFu;
+  }
+  store_hash_words(K + op * 32, h, half);
+  if (rc && half == 0) rc[op] = pad_bad ? -1 : 0;
 }
 
 // ---------------------------------------------------------------- launchers
@@ -1544,11 +1571,17 @@ cudaError_t launch_dec_tail(const uint32_t *E, int lde, const int *ok, const uin
                             uint8_t *K, int *rc, const Segs &segs, bool pc, cudaStream_t st) {
   const long long N = seg_rows(segs);
   if (N <= 0) return cudaSuccess;
-  const unsigned blocks = (unsigned)((N + kTailThreads - 1) / kTailThreads);
-  if (pc)
-    dec_tail_kernel<SET, true><<<blocks, kTailThreads, 0, st>>>(E, lde, ok, C, keys, K, rc, segs);
-  else
-    dec_tail_kernel<SET, false><<<blocks, kTailThreads, 0, st>>>(E, lde, ok, C, keys, K, rc, segs);
+  auto launch = [&](auto kern, int rows_per_block) {
+    kern<<<(unsigned)((N + rows_per_block - 1) / rows_per_block), kTailThreads, 0, st>>>(E, lde, ok, C, keys, K, rc,
+                                                                                       segs);
+  };
+  if (hash_warp_form(segs)) {
+    if (pc) launch(dec_tail_kernel<SET, true, true>, kTailThreads / 32);
+    else launch(dec_tail_kernel<SET, false, true>, kTailThreads / 32);
+  } else {
+    if (pc) launch(dec_tail_kernel<SET, true, false>, kTailThreads / 2);
+    else launch(dec_tail_kernel<SET, false, false>, kTailThreads / 2);
+  }
   return cudaGetLastError();
 }
 

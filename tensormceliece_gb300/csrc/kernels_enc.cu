@@ -461,66 +461,136 @@ __global__ void __launch_bounds__(kSampleThreadsMax)
 // c = e[0:mt] xor (T e[mt:n]); K = SHAKE256(1 || e || c). When the public
 // key's padding bits are set (6960119 only), c and K are zeroed
 // (mc:crypto_kem/6960119/vec/kem_enc.c:21-66).
+// Bound by the integer ALU (10 Keccak-f per request for 8192128). WARP: a warp
+// per request, for launches that leave most of the GPU idle (hash_warp_form);
+// else two lanes per request, 16 requests per warp: 8192128, 65536 requests
+// 206 us against 271 us with one lane per request, where a scheduler held 4 or
+// 3 warps of whole permutations (7 or 6 of half ones now) and the ciphertext
+// was stored a byte at a time by the lane that hashed it (whole rows by the
+// warp now).
+// the ciphertext words of one request, C0 || C1 (C1: plaintext confirmation)
 template <int SET, bool PC>
-__global__ void __launch_bounds__(kTailThreads) finalize_kernel(const uint32_t *__restrict__ E, int lde,
-                                                                const uint32_t *__restrict__ S, int lds,
-                                                                uint8_t *__restrict__ C, uint8_t *__restrict__ K,
-                                                                const Segs segs, uint32_t pk_bad_mask) {
+struct EncHashSrc {
   using p = P<SET>;
-  constexpr int SB = p::synd_bytes, CB = SB + (PC ? 32 : 0);  // C0 bytes, ciphertext bytes
-  __shared__ uint32_t stage[kTailThreads / 32][32 * kStageStride];
-  __shared__ const uint32_t *rows[kTailThreads / 32][32];
-  const long long N = seg_rows(segs);
-  const long long op = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long opc = op < N ? op : N - 1;  // every lane of a warp takes part in the staged hash
-  int seg;
-  const bool live = seg_live(segs, op, &seg);
-  const uint32_t *e = E + opc * lde;
-  const uint32_t *sy = S + opc * lds;
-  // C0 word w: e[0:mt] xor the syndrome, bits from mt on cleared (zero past C0)
-  auto c0word = [&](int w) -> uint32_t {
+  const uint32_t *er, *sr;  // e and T e[mt:n]
+  const uint32_t *c1;       // 8 words of C1 (registers)
+  __device__ uint32_t e(int w) const { return er[w]; }
+  __device__ uint32_t c0(int w) const {
     if (w >= p::mw) return 0u;
-    uint32_t v = e[w] ^ sy[w];
+    uint32_t v = er[w] ^ sr[w];
     if (w == p::mt / 32 && (p::mt % 32)) v &= (1u << (p::mt % 32)) - 1u;
     return v;
-  };
-  // plaintext confirmation: C1 = SHAKE256(2 || e, 32) (mc:crypto_kem/348864pc/vec/kem_enc.c:32)
-  uint64_t h2[4] = {0, 0, 0, 0};
-  if constexpr (PC) {
-    auto none = [](int) -> uint32_t { return 0u; };
-    kem_hash_staged<p::e_bytes, 1 + p::e_bytes>(h2, 2u, e, none, stage[threadIdx.x >> 5], rows[threadIdx.x >> 5]);
   }
-  auto c1byte = [&](int j) -> uint32_t {
-    const uint64_t v = j < 8 ? h2[0] : j < 16 ? h2[1] : j < 24 ? h2[2] : h2[3];
-    return (uint32_t)(v >> (8 * (j & 7))) & 0xFFu;
-  };
-  auto cbyte = [&](int x) -> uint32_t {
-    if (x < SB) return (c0word(x >> 2) >> (8 * (x & 3))) & 0xFFu;
-    return x < CB ? c1byte(x - SB) : 0u;
-  };
-  // word w of the ciphertext C0 || C1 (zero past it)
-  auto cword = [&](int w) -> uint32_t {
-    if (!PC || 4 * w + 4 <= SB) return c0word(w);
-    if (4 * w >= CB) return 0u;
-    if (SB % 4 == 0) {
-      const int j4 = w - SB / 4;
-      const uint64_t v = j4 < 2 ? h2[0] : j4 < 4 ? h2[1] : j4 < 6 ? h2[2] : h2[3];
-      return (uint32_t)(v >> (32 * (j4 & 1)));
+  __device__ uint32_t c1w(int w) const {
+    uint32_t v = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) v = w == i ? c1[i] : v;
+    return v;
+  }
+  __device__ uint32_t c(int w) const {
+    constexpr int W0 = p::synd_bytes / 4;
+    if (!PC) return c0(w);
+    if (w < W0) return c0(w);
+    if (p::synd_bytes % 4 == 0) return c1w(w - W0);
+    if (w == W0) return c0(w) | (c1[0] << 16);
+    return (c1w(w - W0 - 1) >> 16) | (c1w(w - W0) << 16);
+  }
+};
+
+template <int SET, bool PC, bool WARP>
+__global__ void __launch_bounds__(kTailThreads, WARP ? 1 : PC ? kTailBlocksPerSM - 2 : kTailBlocksPerSM)
+    finalize_kernel(const uint32_t *__restrict__ E, int lde, const uint32_t *__restrict__ S, int lds,
+                    uint8_t *__restrict__ C, uint8_t *__restrict__ K, const Segs segs, uint32_t pk_bad_mask) {
+  using p = P<SET>;
+  constexpr int SB = p::synd_bytes, CB = SB + (PC ? 32 : 0);  // C0 bytes, ciphertext bytes
+  constexpr int RPW = WARP ? 1 : 16;                          // requests per warp
+  const int lane = threadIdx.x & 31, half = lane & 1;
+  const long long op0 = ((long long)blockIdx.x * (kTailThreads / 32) + (threadIdx.x >> 5)) * RPW;
+  const int r = WARP ? 0 : lane >> 1;
+  int seg;
+  const bool live = seg_live(segs, op0 + r, &seg);
+  const uint32_t livemask = __ballot_sync(0xffffffffu, live);
+  if (!livemask) return;
+  const uint32_t badmask = __ballot_sync(0xffffffffu, (pk_bad_mask >> seg) & 1u);
+  // lanes of rows that are not live hash the warp's first live row and store nothing
+  const long long op = live ? op0 + r : op0 + (WARP ? 0 : (__ffs(livemask) - 1) >> 1);
+  uint32_t c1[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  const EncHashSrc<SET, PC> src{E + op * lde, S + op * lds, c1};
+  uint32_t own[4];
+  // plaintext confirmation: C1 = SHAKE256(2 || e, 32) (mc:crypto_kem/348864pc/vec/kem_enc.c:32)
+  if constexpr (PC) {
+    const EncOnlySrc esrc{src.er};
+    if constexpr (WARP) {
+      const uint64_t h = kem_hash_warp<p::e_bytes, 1 + p::e_bytes>(2u, esrc, lane);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const uint64_t v = __shfl_sync(0xffffffffu, h, i);
+        c1[2 * i] = (uint32_t)v;
+        c1[2 * i + 1] = (uint32_t)(v >> 32);
+      }
+    } else {
+      kem_hash_pair<p::e_bytes, 1 + p::e_bytes>(own, 2u, esrc, half);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const uint32_t o = __shfl_xor_sync(0xffffffffu, own[i], 1);
+        c1[2 * i] = half ? o : own[i];
+        c1[2 * i + 1] = half ? own[i] : o;
+      }
     }
-    return cbyte(4 * w) | (cbyte(4 * w + 1) << 8) | (cbyte(4 * w + 2) << 16) | (cbyte(4 * w + 3) << 24);
+  }
+  if constexpr (WARP) {
+    const uint64_t h = kem_hash_warp<p::e_bytes, p::pre_bytes + (PC ? 32 : 0)>(1u, src, lane);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint64_t v = __shfl_sync(0xffffffffu, h, i);
+      own[i] = half ? (uint32_t)(v >> 32) : (uint32_t)v;
+    }
+  } else {
+    kem_hash_pair<p::e_bytes, p::pre_bytes + (PC ? 32 : 0)>(own, 1u, src, half);
+  }
+  const bool bad = (badmask >> lane) & 1u;
+  if (live && (!WARP || lane < 2)) {
+    if (bad) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) own[i] = 0;
+    }
+    store_hash_words(K + op * 32, own, half);
+    if constexpr (PC) {
+      uint32_t v[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) v[i] = bad ? 0u : half ? c1[2 * i + 1] : c1[2 * i];
+      store_hash_words(C + op * CB + SB, v, half);
+    }
+  }
+  // C0 of the warp's rows, in the widest units that divide a row at this buffer's alignment
+  const uint32_t *Eb = E + op0 * lde, *Sb = S + op0 * lds;
+  uint8_t *cb = C + op0 * CB;
+  auto c0_of = [&](int row, int w) -> uint32_t {
+    uint32_t v = Eb[(long long)row * lde + w] ^ Sb[(long long)row * lds + w];
+    if (w == p::mt / 32 && (p::mt % 32)) v &= (1u << (p::mt % 32)) - 1u;
+    return ((badmask >> (WARP ? 0 : 2 * row)) & 1u) ? 0u : v;
   };
-  uint64_t h[4];
-  kem_hash_staged<p::e_bytes, p::pre_bytes + (PC ? 32 : 0)>(h, 1u, e, cword, stage[threadIdx.x >> 5],
-                                                             rows[threadIdx.x >> 5]);
-  if (!live) return;
-  const bool pk_bad = (pk_bad_mask >> seg) & 1u;
-  uint8_t *c = C + op * CB;
-  uint8_t *k = K + op * 32;
-  for (int x = 0; x < CB; x++) c[x] = pk_bad ? 0 : (uint8_t)cbyte(x);
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int b = 0; b < 8; b++) k[8 * i + b] = pk_bad ? 0 : (uint8_t)(h[i] >> (8 * b));
+  auto row_live = [&](int row) { return ((livemask >> (WARP ? 0 : 2 * row)) & 1u) != 0; };
+  const uintptr_t align = reinterpret_cast<uintptr_t>(C);
+  if (SB % 4 == 0 && CB % 4 == 0 && (align & 3) == 0) {
+    constexpr int U = SB / 4;
+    for (int x = lane; x < RPW * U; x += 32) {
+      const int row = x / U, w = x - row * U;
+      if (row_live(row)) *reinterpret_cast<uint32_t *>(cb + row * CB + 4 * w) = c0_of(row, w);
+    }
+  } else if (SB % 2 == 0 && CB % 2 == 0 && (align & 1) == 0) {
+    constexpr int U = SB / 2;
+    for (int x = lane; x < RPW * U; x += 32) {
+      const int row = x / U, w = x - row * U;
+      if (row_live(row))
+        *reinterpret_cast<uint16_t *>(cb + row * CB + 2 * w) = (uint16_t)(c0_of(row, w >> 1) >> (16 * (w & 1)));
+    }
+  } else {
+    for (int x = lane; x < RPW * SB; x += 32) {
+      const int row = x / SB, w = x - row * SB;
+      if (row_live(row)) cb[row * CB + w] = (uint8_t)(c0_of(row, w >> 2) >> (8 * (w & 3)));
+    }
+  }
 }
 
 // ---------------------------------------------------------------- column image of T
@@ -552,6 +622,19 @@ cudaError_t launch_transpose_pk(const uint32_t *T, int lda, int mt, int k, uint3
 }
 
 // ---------------------------------------------------------------- launchers
+// A warp per request while every SM scheduler has at most one such warp (see
+// KeccakWarp): beyond that its six-fold instruction count outweighs its
+// latency. Rows that are not live exit at once and do not count.
+constexpr int kHashWarpsPerSM = 4;
+bool hash_warp_form(const Segs &segs) {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  long long live = 0;
+  for (int i = 0; i < segs.nseg; i++) live += segs.nreq[i];
+  return live <= (long long)kHashWarpsPerSM * sms;
+}
+
 // GMC_SAMPLE_PIPELINE=0 in the environment (read once per process) puts
 // every batch on the lane-per-request sampler instead of the pipelined one.
 static bool sample_pipelined() {
@@ -654,11 +737,17 @@ cudaError_t launch_finalize(const uint32_t *E, int lde, const uint32_t *S, int l
                             const Segs &segs, uint32_t pk_bad_mask, bool pc, cudaStream_t st) {
   const long long N = seg_rows(segs);
   if (N <= 0) return cudaSuccess;
-  long long blocks = (N + kTailThreads - 1) / kTailThreads;
-  if (pc)
-    finalize_kernel<SET, true><<<(unsigned)blocks, kTailThreads, 0, st>>>(E, lde, S, lds, C, K, segs, pk_bad_mask);
-  else
-    finalize_kernel<SET, false><<<(unsigned)blocks, kTailThreads, 0, st>>>(E, lde, S, lds, C, K, segs, pk_bad_mask);
+  auto launch = [&](auto kern, int rows_per_block) {
+    kern<<<(unsigned)((N + rows_per_block - 1) / rows_per_block), kTailThreads, 0, st>>>(E, lde, S, lds, C, K, segs,
+                                                                                       pk_bad_mask);
+  };
+  if (hash_warp_form(segs)) {
+    if (pc) launch(finalize_kernel<SET, true, true>, kTailThreads / 32);
+    else launch(finalize_kernel<SET, false, true>, kTailThreads / 32);
+  } else {
+    if (pc) launch(finalize_kernel<SET, true, false>, kTailThreads / 2);
+    else launch(finalize_kernel<SET, false, false>, kTailThreads / 2);
+  }
   return cudaGetLastError();
 }
 

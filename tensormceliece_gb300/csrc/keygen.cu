@@ -13,8 +13,8 @@
 // control bits of the support permutation, and sk = seed | pivots | g |
 // control bits | r[0:n/8].
 //
-// Seed chains (stream 0): kg_expand, one thread per key and chain link,
-// expands 16 links of every key ahead of the rounds into an expansion store
+// Seed chains (stream 0): kg_expand, a warp (or two lanes) per key and chain
+// link, expands 16 links of every key ahead of the rounds into an expansion store
 // (more for the rare key that needs them); a chain link costs 251 sequential
 // Keccak-f permutations for 8192128, so expanding ahead keeps the chain
 // latency off the rounds.
@@ -97,48 +97,68 @@ __device__ __forceinline__ void kg_cluster_sync() {
 constexpr uint8_t kKgMinpoly = 1, kKgDistinct = 2, kKgRank = 4, kKgAll = 7;
 
 // ---------------------------------------------------------------- expansion
-// One link of every listed key's seed chain: thread i takes key = keys[i]
-// (or i), expands r = SHAKE256({64} || seed) into slot (a, i) of a block of
-// nb keys, stores the seed after r's blocks, and advances the key's chain
-// to seed' = r[rlen-32 : rlen].
-template <int SET>
+// One link of every listed key's seed chain: key i of the launch is keys[i]
+// (or i); r = SHAKE256({64} || seed) goes into slot (a, i) of a block of nb
+// keys with the seed after r's blocks, and the key's chain advances to
+// seed' = r[rlen-32 : rlen]. A link is rblocks permutations in a row (251 for
+// 8192128), all latency. WARP: a warp per key (207 cycles a Keccak round
+// alone on its scheduler), else two lanes per key (277); one lane per key took
+// 403 (1.20 ms a link for 8192128, 0.61 ms with a warp). The warp form's instructions per key are 6 times the
+// pair form's, so it is taken while every scheduler has at most two such warps.
+constexpr int kExpandWarpKeysPerSM = 8;
+template <int SET, bool WARP>
 __global__ void __launch_bounds__(32) kg_expand_kernel(uint8_t *__restrict__ seedc, const int *__restrict__ keys,
                                                        int nb, int a, uint8_t *__restrict__ out) {
   using C = KG<SET>;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nb) return;
+  const int lane = threadIdx.x, half = lane & 1;
+  const int i0 = WARP ? blockIdx.x : 16 * blockIdx.x + (lane >> 1);
+  const int i = i0 < nb ? i0 : nb - 1;  // every lane permutes; lanes past the list write nothing
+  const bool live = i0 < nb;
   const int key = keys ? keys[i] : i;
   uint8_t *r = out + ((long long)a * nb + i) * C::rstride;
-  uint8_t in[40];
-  in[0] = 64;
-#pragma unroll
-  for (int j = 0; j < 32; j++) in[1 + j] = seedc[32 * key + j];
-  in[33] = 0x1F;
-#pragma unroll
-  for (int j = 34; j < 40; j++) in[j] = 0;
-  uint64_t s[25];
-#pragma unroll
-  for (int j = 0; j < 25; j++) s[j] = 0;
-  // absorb {64} || seed || 0x1F, final bit of the 136-byte block
-#pragma unroll
-  for (int l = 0; l < 5; l++) {
-    uint64_t w = 0;
-#pragma unroll
-    for (int b = 0; b < 8; b++) w |= (uint64_t)in[8 * l + b] << (8 * b);
-    s[l] = w;
-  }
-  s[16] ^= 0x8000000000000000ull;
-  uint64_t *o = reinterpret_cast<uint64_t *>(r);
+  uint32_t *seed = reinterpret_cast<uint32_t *>(seedc + 32 * (long long)key);
+  // word j of {64} || seed || 0x1F (zero from word 9 on)
+  auto msg = [&](int j) -> uint32_t {
+    if (j > 8) return 0u;
+    const uint32_t prev = j ? seed[j - 1] : 64u << 24, cur = j < 8 ? seed[j] : 0x1Fu;
+    return __funnelshift_l(prev, cur, 8);
+  };
+  if constexpr (WARP) {
+    const KeccakWarp kw(lane);
+    uint64_t s = lane < 17 ? (uint64_t)msg(2 * lane) | ((uint64_t)msg(2 * lane + 1) << 32) : 0ull;
+    if (lane == 16) s ^= 0x8000000000000000ull;
+    uint64_t *o = reinterpret_cast<uint64_t *>(r);
 #pragma unroll 1
-  for (int b = 0; b < C::rblocks; b++) {
-    keccak_f1600(s);
+    for (int b = 0; b < C::rblocks; b++) {
+      kw.permute(s);
+      if (lane < 17) o[17 * b + lane] = s;
+    }
+    if (lane < 8) reinterpret_cast<uint32_t *>(r + C::dofs)[lane] = seed[lane];
+    __syncwarp();
+    seedc[32 * (long long)key + lane] = r[C::rlen - 32 + lane];
+  } else {
+    uint32_t s[25];
 #pragma unroll
-    for (int j = 0; j < 17; j++) o[17 * b + j] = s[j];
-  }
+    for (int j = 0; j < 25; j++) s[j] = j < 17 ? msg(2 * j + half) : 0u;
+    if (half) s[16] ^= 0x80000000u;
+    uint32_t *o = reinterpret_cast<uint32_t *>(r);
+#pragma unroll 1
+    for (int b = 0; b < C::rblocks; b++) {
+      keccak_f1600_pair(s, half);
+      if (live) {
 #pragma unroll
-  for (int j = 0; j < 32; j++) {
-    r[C::dofs + j] = in[1 + j];
-    seedc[32 * key + j] = r[C::rlen - 32 + j];
+        for (int j = 0; j < 17; j++) o[34 * b + 2 * j + half] = s[j];
+      }
+    }
+    if (live) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) reinterpret_cast<uint32_t *>(r + C::dofs)[2 * j + half] = seed[2 * j + half];
+    }
+    __syncwarp();  // the key's other lane's blocks and seed copy are done
+    if (live) {
+#pragma unroll
+      for (int j = 0; j < 16; j++) seedc[32 * (long long)key + 16 * half + j] = r[C::rlen - 32 + 16 * half + j];
+    }
   }
 }
 
@@ -1094,7 +1114,10 @@ int keypair_batch(uint8_t *pk, uint8_t *sk, const uint8_t *seeds, long long nkey
       }
       blk.seq0 = (int)links.size();
       for (int a = 0; a < nlinks; a++) {
-        kg_expand_kernel<SET><<<(blk.nb + 31) / 32, 32, 0, s0>>>(d_seedc, blk.keys, blk.nb, a, blk.base);
+        if (blk.nb <= kExpandWarpKeysPerSM * sms)
+          kg_expand_kernel<SET, true><<<blk.nb, 32, 0, s0>>>(d_seedc, blk.keys, blk.nb, a, blk.base);
+        else
+          kg_expand_kernel<SET, false><<<(blk.nb + 15) / 16, 32, 0, s0>>>(d_seedc, blk.keys, blk.nb, a, blk.base);
         cudaEvent_t ev;
         if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return e;
         links.push_back(ev);
