@@ -160,11 +160,11 @@ static int get_field(int set, FieldDev *out) {
   const HostField &F = host_field(S.m);
   FftTables ft = build_fft_tables(S.m, S.fft_d);
   std::vector<uint16_t> all;
-  // u16 tables, then the bit-sliced u32 tables at even (4-byte aligned) offsets
+  auto pad = [&] { all.resize((all.size() + kFieldAlign - 1) / kFieldAlign * kFieldAlign, 0); };
   auto put = [&](const std::vector<uint16_t> &v) {
-    if (all.size() & 1) all.push_back(0);
     const size_t at = all.size();
     all.insert(all.end(), v.begin(), v.end());
+    pad();
     return at;
   };
   const size_t o_exp = put(F.exp), o_log = put(F.log), o_twist = put(ft.twist_log), o_frlo = put(ft.frob_lo),

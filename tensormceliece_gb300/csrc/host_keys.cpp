@@ -171,7 +171,8 @@ FftTables build_fft_tables(int m, int d) {
     v[2 * w] = (uint16_t)(x & 0xFFFFu);
     v[2 * w + 1] = (uint16_t)(x >> 16);
   };
-  t.alpha_bs.assign((size_t)2 * ((1 << d) - 1) * H * m, 0);
+  const int row = alpha_bs_stride(H * m);
+  t.alpha_bs.assign((size_t)2 * ((1 << d) - 1) * row, 0);
   for (int l = 0, aoff = 0; l < d; aoff += 1 << (m - l - 1), l++)
     for (int xh = 0; xh < (1 << (d - 1 - l)); xh++)
       for (int h = 0; h < H; h++)
@@ -182,7 +183,7 @@ FftTables build_fft_tables(int m, int d) {
             const uint16_t a = F.exp[t.alpha_log[aoff + (c << (d - 1 - l)) + xh]];
             w |= (uint32_t)((a >> b) & 1) << k;
           }
-          put_word(t.alpha_bs, ((size_t)((1 << d) - (1 << (d - l)) + xh) * H + h) * m + b, w);
+          put_word(t.alpha_bs, (size_t)((1 << d) - (1 << (d - l)) + xh) * row + h * m + b, w);
         }
   t.frob_hi_bs.assign((size_t)2 * H * m, 0);
   for (int h = 0; h < H; h++)

@@ -36,7 +36,7 @@ struct FftTables {
   // word belongs to chunk c = 32 h + k (h < 2^(m-d) / 32) and plane b holds
   // bit b of the field element. Stored as u32 words split into (low, high)
   // u16 halves so they travel in the u16 table buffers.
-  //   alpha_bs[((2^d - 2^(d-l) + xh) * H + h) * m + b]: alpha_{l, (c << (d-1-l)) + xh}, xh < 2^(d-1-l)
+  //   alpha_bs[(2^d - 2^(d-l) + xh) * alpha_bs_stride(H m) + h m + b]: alpha_{l, (c << (d-1-l)) + xh}, xh < 2^(d-1-l)
   //   frob_hi_bs[h * m + b]: frob_hi[c]
   std::vector<uint16_t> alpha_bs;
   std::vector<uint16_t> frob_hi_bs;

@@ -15,7 +15,8 @@ constexpr int kTailThreads = 64;
 constexpr int kTailBlocksPerSM = 14;
 constexpr int kBMWarps = 14;    // Berlekamp-Massey kernel: default and largest warps per block (32 requests per warp)
 constexpr int kBMCtWarps = 8;   // its constant-time form: largest warps per block
-constexpr int kBMLatWarps = 28;  // Berlekamp-Massey latency form: largest warps per block (one request per warp)
+constexpr int kBMLatWarps = 24;  // Berlekamp-Massey latency form: largest warps per block (one request per warp)
+constexpr int kBMLatCopyWarps = 8;  // its smallest block: warps without a request help to copy the tables
 constexpr long long kBMBitslicedMinRows = 24576;  // smaller batches take the latency form
 constexpr int kRootWarps = 8;  // root-finding kernel: default and largest warps per block
 
@@ -145,14 +146,17 @@ struct DecKeyDev {
   const uint32_t *cond;  // the sk's Benes control bits ((2m - 1) 2^(m-1) bits, as 32-bit words)
 };
 
-// Per-field / per-set device tables (shared by all keys of a set).
+// Per-field / per-set device tables (shared by all keys of a set). Every table
+// starts on a 16-byte boundary and is followed by readable memory up to the
+// next one (the kernels copy whole 16-byte units).
+constexpr int kFieldAlign = 8;  // u16 entries
 struct FieldDev {
   const uint16_t *gexp;   // [2q-1]
   const uint16_t *glog;   // [q]
   const uint16_t *fft_twist_log;  // concatenated per level l = 0..d-1: [2^(d-l)]
   const uint16_t *frob_lo;        // x^(2^d) for x < 2^d
   // bit-sliced over 32 chunks per word (bit k: chunk 32 h + k), plane b = bit b
-  const uint32_t *fft_alpha_bs;   // [(2^d - 2^(d-l) + xh) * H + h][m]: alpha_{l, (c << (d-1-l)) + xh}
+  const uint32_t *fft_alpha_bs;   // [2^d - 2^(d-l) + xh][alpha_bs_stride(H m)], entry h m + b: alpha_{l, (c << (d-1-l)) + xh}
   const uint32_t *frob_hi_bs;     // [h][m]: (c 2^d)^(2^d)
   const uint16_t *zech;           // [q]: log(1 + g^k), zech[0] = 3q (zero)
   // [2^(d+1)][m]: for the twist constant c of each fft_twist_log entry, c x^i (i < m), so a product

@@ -16,6 +16,8 @@
 // decoder yields the same session key. The BM update rule follows the
 // library's (mc:crypto_kem/348864/vec/bm.c:156), so locators agree with the
 // oracle's stage output as well.
+#include <type_traits>
+
 #include "kernels.h"
 #include "device_common.cuh"
 
@@ -25,6 +27,18 @@ __device__ __forceinline__ uint32_t warp_xor(uint32_t v) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) v ^= __shfl_xor_sync(0xffffffffu, v, o);
   return v;
+}
+
+// Copies a field table of n 16-bit entries to shared memory by the whole block,
+// 16 bytes a thread (both sides 16-byte aligned; n is rounded up to whole
+// units). A block of few warps spends most of a small launch here if it copies
+// entry by entry: one 8192128 request, Berlekamp-Massey 125 -> 92 us, roots
+// 29 -> 25 us.
+__device__ __forceinline__ void copy_table(void *dst, const void *src, int n) {
+  const int units = (2 * n + 15) / 16;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < units; i += blockDim.x)
+    reinterpret_cast<uint4 *>(dst)[i] = reinterpret_cast<const uint4 *>(src)[i];
 }
 
 // ---------------------------------------------------------------- pack_ct
@@ -125,8 +139,8 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
   extern __shared__ __align__(16) uint32_t bsm[];
   uint16_t *gexp = reinterpret_cast<uint16_t *>(bsm) + LY::exp_off;
   uint16_t *glog = reinterpret_cast<uint16_t *>(bsm) + LY::log_off;
-  for (int i = threadIdx.x; i < Q - 1; i += blockDim.x) gexp[i] = fd.gexp[i];
-  for (int i = threadIdx.x; i < Q; i += blockDim.x) glog[i] = fd.glog[i];
+  copy_table(gexp, fd.gexp, Q);
+  copy_table(glog, fd.glog, Q);
   for (int i = threadIdx.x; i < LY::zero_len; i += blockDim.x) bsm[LY::zero_off + i] = 0u;
   __syncthreads();
   const uint32_t *ZP = bsm + LY::zero_off;
@@ -581,42 +595,49 @@ __global__ void __launch_bounds__(kBMCtWarps * 32, 1) dec_bm_ct_kernel(const uin
 }
 
 // ---------------------------------------------------------------- BM, latency form
-// Used for small batches (fewer requests than the bit-sliced form needs to
-// fill the GPU): per-request latency is one warp walking 2t iterations of
-// ~100 instructions instead of a group of 32 walking ~1500.
-// One warp per request (persistent grid). Coefficient i of C (connection
-// polynomial) lives in lane i%32, slot i/32, as its log only: the update
-// C_i += f B_i is done in the log domain with Zech logarithms,
-// log(a + b) = log a + zech(log b - log a), one table lookup instead of an
-// antilog and a log. Any log at or above the zero sentinel 2q-2 means 0.
-// B = x^s B' is kept unshifted: B' (the connection polynomial before the last
-// length change, as logs) sits in a per-warp shared array behind a guard of
-// 2t zero logs, so B_i is the entry at i - s and the per-iteration shift is
-// s += 1. The syndrome logs sit behind a 32-entry zero guard, so the
-// discrepancy reads s_{n-i} for every lane of an active slot without a
-// per-lane test (C_i = 0 above deg C). Coefficients above t are never
+// Used for small batches (fewer requests than the bit-sliced forms need to
+// fill the GPU): one warp per request (persistent grid), coefficient i =
+// 1 + 32 k + lane of C (connection polynomial) in slot k of a lane as its log
+// only; C_0 = 1 is implicit. The update C_i += f B_i is done in the log domain
+// with Zech logarithms, log(a + b) = log a + zech(log b - log a), one table
+// lookup instead of an antilog and a log. Any log at or above the zero
+// sentinel 2q-2 means 0. B = x^s B' is kept unshifted: B' (the connection
+// polynomial before the last length change, as logs) sits in a per-warp shared
+// array behind a guard of 2t zero logs, so B_i is the entry at i - s and the
+// per-iteration shift is s += 1. The syndrome logs sit behind a 32-entry zero
+// guard, so the discrepancy reads s_{n-i} for every lane of an active slot
+// without a per-lane test (C_i = 0 above deg C). Coefficients above t are never
 // updated, as in the library's fixed-size arrays.
 // Degree bounds used to skip empty slots (exact, also for undecodable input):
-// before iteration n, deg C <= L and deg B <= n+1-L, so the discrepancy needs
-// coefficients i <= min(L, t) and the update i <= min(max(L, n+1-L), t).
+// before iteration n, deg C <= L and deg B <= n+1-L, so both loops need
+// coefficients i <= min(max(L, n+1-L), t), a bound that never falls. The
+// iterations therefore run in ceil(t / 32) loops, one per number of active
+// slots, each with straight-line slot code: the slots' table lookups overlap.
+// With a test per slot their latencies added up: 8192128, 1 / 2048 / 8192 /
+// 20000 (6688128) requests 92 / 114 / 258 / 625 us, against 58 / 74 / 199 /
+// 459 us now. Four warps per request with a barrier an iteration were slower
+// (66 us for one request, 338 against 105 us for 4096).
+// Bound: the chain of one iteration up to about 2000 requests, above that the
+// bank conflicts of the table lookups (about 9 shared-memory wavefronts a slot).
 template <int SET>
 struct BMLatLayout {
   using p = P<SET>;
   static constexpr int Q = p::q, T = p::t;
-  static constexpr int NS = (T + 1 + 31) / 32;
+  static constexpr int NS = (T + 31) / 32;
   static constexpr int exp_off = 0, log_off = 2 * Q, zech_off = 3 * Q;
   static constexpr int shared_u16 = 4 * Q;
   static constexpr int sguard = 32, bguard = 2 * T;
   static constexpr int s_off = 0, s_len = sguard + 2 * T;          // per warp, u16
-  static constexpr int b_off = s_len, b_len = bguard + 32 * NS;
-  static constexpr int warp_u16 = (s_len + b_len + 1) & ~1;
+  static constexpr int raw_off = s_len, raw_len = 2 * T;
+  static constexpr int b_off = raw_off + raw_len, b_len = bguard + 1 + 32 * NS;
+  static constexpr int warp_u16 = (b_off + b_len + 1) & ~1;
   static constexpr int bytes(int warps) { return shared_u16 * 2 + warps * warp_u16 * 2; }
 };
 
 template <int SET>
 __global__ void __launch_bounds__(kBMLatWarps * 32, 2) dec_bm_lat_kernel(const uint32_t *__restrict__ S2, int lds2,
                                                                   FieldDev fd, const Segs segs,
-                                                                  uint16_t *__restrict__ Sig) {
+                                                                  uint16_t *__restrict__ Sig, int nwb) {
   using p = P<SET>;
   using LY = BMLatLayout<SET>;
   constexpr int M = p::m, Q = p::q, T = p::t, D = p::fft_d;
@@ -628,20 +649,21 @@ __global__ void __launch_bounds__(kBMLatWarps * 32, 2) dec_bm_lat_kernel(const u
   uint16_t *gexp = lsm + LY::exp_off;
   uint16_t *glog = lsm + LY::log_off;
   uint16_t *zech = lsm + LY::zech_off;
-  for (int i = threadIdx.x; i < 2 * Q - 1; i += blockDim.x) gexp[i] = fd.gexp[i];
-  for (int i = threadIdx.x; i < Q; i += blockDim.x) {
-    glog[i] = fd.glog[i];
-    zech[i] = fd.zech[i];
-  }
+  copy_table(gexp, fd.gexp, 2 * Q);
+  copy_table(glog, fd.glog, Q);
+  copy_table(zech, fd.zech, Q);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint16_t *wsm = lsm + LY::shared_u16 + warp * LY::warp_u16;
   uint16_t *slog = wsm + LY::s_off + LY::sguard;  // slog[-32 .. -1] = zero logs
+  uint16_t *sraw = wsm + LY::raw_off;
   uint16_t *blog = wsm + LY::b_off + LY::bguard;  // blog[-2t .. -1] = zero logs
-  for (int i = lane; i < LY::sguard; i += 32) wsm[LY::s_off + i] = (uint16_t)ZL;
-  for (int i = lane; i < LY::bguard; i += 32) wsm[LY::b_off + i] = (uint16_t)ZL;
+  if (warp < nwb) {
+    for (int i = lane; i < LY::sguard; i += 32) wsm[LY::s_off + i] = (uint16_t)ZL;
+    for (int i = lane; i < LY::bguard; i += 32) wsm[LY::b_off + i] = (uint16_t)ZL;
+  }
   __syncthreads();
+  if (warp >= nwb) return;  // warps that only help to copy the tables
   const long long N = seg_rows(segs);
-  const int nwb = blockDim.x >> 5;  // warps per block (a launch parameter up to kBMLatWarps)
   const long long nwarps = (long long)gridDim.x * nwb;
   for (long long op = (long long)blockIdx.x * nwb + warp; op < N; op += nwarps) {
     int seg;
@@ -654,44 +676,45 @@ __global__ void __launch_bounds__(kBMLatWarps * 32, 2) dec_bm_lat_kernel(const u
         const int b = j * M, w = b >> 5, sh = b & 31;
         uint32_t v = srow[w] >> sh;
         if (sh + M > 32) v |= srow[w + 1] << (32 - sh);
-        slog[j] = glog[v & (Q - 1)];
+        v &= Q - 1;
+        sraw[j] = (uint16_t)v;
+        slog[j] = glog[v];
       }
     }
     // B' = 1, s = 1 (B = x)
-#pragma unroll
-    for (int k = 0; k < NS; k++) blog[lane + 32 * k] = (lane + 32 * k == 0) ? 0 : (uint16_t)ZL;
+    for (int j = lane; j <= 32 * NS; j += 32) blog[j] = j == 0 ? 0 : (uint16_t)ZL;
     __syncwarp();
     uint32_t lC[NS];
 #pragma unroll
-    for (int k = 0; k < NS; k++) lC[k] = (lane + 32 * k == 0) ? 0 : ZL;
-    int L = 0, sft = 1;
+    for (int k = 0; k < NS; k++) lC[k] = ZL;
+    int L = 0, sft = 1, n = 0;
     uint32_t lb = 0;  // log b, b = 1
+    // the iterations that need K slots
+    auto iterate = [&](auto slots) {
+      constexpr int K = decltype(slots)::value;
 #pragma unroll 1
-    for (int n = 0; n < 2 * T; n++) {
-      const int bd = L < T ? L : T;                       // discrepancy: i <= min(L, t) (L <= n)
-      int bu = (L > n + 1 - L) ? L : n + 1 - L;           // update: i <= min(max(L, n+1-L), t)
-      bu = bu < T ? bu : T;
-      uint32_t dp = 0;
-      const uint16_t *sn = slog + n - lane;
+      for (; n < 2 * T; n++) {
+        if (K < NS && (L > 32 * K || n + 1 - L > 32 * K)) return;
+        const uint16_t *sn = slog + n - 1 - lane, *bs = blog + 1 + lane - sft;
+        uint32_t dp = 0, lbi[K];
 #pragma unroll
-      for (int k = 0; k < NS; k++)
-        if (32 * k <= bd) dp ^= gf_mul_log<M>(gexp, lC[k], sn[-32 * k]);
-      const uint32_t d = __reduce_xor_sync(0xffffffffu, dp);
-      if (d) {
-        const bool upd = (n >= 2 * L);
-        const int ld = glog[d];
-        int lf = ld - (int)lb;
-        if (lf < 0) lf += Q - 1;
-        const uint16_t *bs = blog + lane - sft;
-        uint32_t lco[NS];
+        for (int k = 0; k < K; k++) dp ^= gf_mul_log<M>(gexp, lC[k], sn[-32 * k]);
 #pragma unroll
-        for (int k = 0; k < NS; k++) {
-          lco[k] = lC[k];
-          if (32 * k <= bu) {
-            // log(C_i + f B_i): p = log(f B_i); zero B_i keeps C_i, zero C_i takes p
+        for (int k = 0; k < K; k++) lbi[k] = bs[32 * k];
+        const uint32_t d = __reduce_xor_sync(0xffffffffu, dp) ^ sraw[n];
+        if (d) {
+          const bool upd = (n >= 2 * L);
+          const int ld = glog[d];
+          int lf = ld - (int)lb;
+          if (lf < 0) lf += Q - 1;
+          uint32_t lco[K];
+#pragma unroll
+          for (int k = 0; k < K; k++) {
+            // log(C_i + f B_i): pl = log(f B_i); zero B_i keeps C_i, zero C_i takes pl
             constexpr uint32_t Q1 = Q - 1;
-            const uint32_t lbi = bs[32 * k], lc = lC[k];
-            uint32_t pl = (uint32_t)lf + lbi;
+            const uint32_t lc = lC[k];
+            lco[k] = lc;
+            uint32_t pl = (uint32_t)lf + lbi[k];
             pl = min(pl, pl - Q1);                      // < q-1 when B_i != 0
             uint32_t kk = pl - lc;                      // log(f B_i / C_i) mod q-1
             kk = min(kk + Q1, kk);
@@ -699,36 +722,37 @@ __global__ void __launch_bounds__(kBMLatWarps * 32, 2) dec_bm_lat_kernel(const u
             uint32_t nl = lc + z;
             nl = min(nl, nl - Q1);                      // >= 2q-2 when the sum is 0
             nl = (lc >= (uint32_t)ZL) ? pl : nl;
-            nl = (lbi >= (uint32_t)ZL) ? lc : nl;
-            const bool in = (k < NS - 1) || (lane + 32 * k <= T);  // coefficients above t stay zero
-            if (in) lC[k] = nl;
+            nl = (lbi[k] >= (uint32_t)ZL) ? lc : nl;
+            if (32 * (k + 1) <= T || 1 + lane + 32 * k <= T) lC[k] = nl;  // coefficients above t stay zero
+          }
+          if (upd) {
+            __syncwarp();  // every lane has read B' before it is replaced
+#pragma unroll
+            for (int k = 0; k < K; k++) blog[1 + lane + 32 * k] = (uint16_t)lco[k];
+            __syncwarp();
+            L = n + 1 - L;
+            lb = ld;
+            sft = 0;
           }
         }
-        if (upd) {
-          __syncwarp();  // every lane has read B' before it is replaced
-#pragma unroll
-          for (int k = 0; k < NS; k++)
-            if (32 * k <= bu) blog[lane + 32 * k] = (uint16_t)lco[k];
-          __syncwarp();
-          L = n + 1 - L;
-          lb = ld;
-          sft = 0;
-        }
+        sft++;
       }
-      sft++;
-    }
+    };
+    iterate(std::integral_constant<int, 1>{});
+    iterate(std::integral_constant<int, 2>{});
+    if constexpr (NS > 2) iterate(std::integral_constant<int, 3>{});
+    if constexpr (NS > 3) iterate(std::integral_constant<int, 4>{});
+    static_assert(NS >= 2 && NS <= 4, "one loop per number of active slots");
     // sigma(x) = sum_deg C[t-deg] x^deg -> FFT coefficient slots (deg < 2^d);
-    // coefficients are < 2^m <= 2^13, so bit 15 is free for the length flag
+    // coefficients are < 2^m <= 2^13, so bit 15 of the constant coefficient
+    // is free for the flag of a final length L > t
     uint16_t *sig = Sig + op * SIG;
-    for (int x = lane; x < SIG; x += 32)
-      if (x > T) sig[x] = 0;
+    for (int x = T + lane; x < SIG; x += 32) sig[x] = x == T ? 1 : 0;
 #pragma unroll
     for (int k = 0; k < NS; k++) {
-      const int i = lane + 32 * k;
-      const int deg = T - i;
-      // bit 15 of the constant coefficient flags a final length L > t
+      const int i = 1 + lane + 32 * k;
       const uint32_t c = gexp[min(lC[k], (uint32_t)ZL)];
-      if (i <= T && deg < SIG) sig[deg] = (uint16_t)(c | ((deg == 0 && L > T) ? 0x8000u : 0u));
+      if (i <= T) sig[T - i] = (uint16_t)(c | ((i == T && L > T) ? 0x8000u : 0u));
     }
     __syncwarp();
   }
@@ -763,13 +787,13 @@ struct RootLayout {
   static constexpr int log_off = exp_off + exp_len, log_len = CT ? 0 : Q;
   static constexpr int twist_off = log_off + log_len, twist_len = CT ? (2 << D) * M : 2 << D;
   static constexpr int frlo_off = twist_off + twist_len, frlo_len = SIG;
-  static constexpr int shared_u16 = (frlo_off + frlo_len + 1) & ~1;
-  // u32 region: bit-sliced alpha, bit-sliced frob_hi
-  // bit-sliced butterfly constants, one row of NH * M planes per (level, block): rows padded to an odd
-  // stride so that 32 lanes reading 32 different rows hit 32 different banks
-  static constexpr int abs_row = NH * M, abs_stride = abs_row | 1;
-  static constexpr int abs_off = shared_u16 / 2, abs_len = (SIG - 1) * abs_stride;
-  static constexpr int fhbs_off = abs_off + abs_len, fhbs_len = NH * M;
+  static constexpr int shared_u16 = frlo_off + frlo_len;
+  static_assert(log_off % 8 == 0 && twist_off % 8 == 0 && frlo_off % 8 == 0 && shared_u16 % 8 == 0,
+                "tables are copied in 16-byte units");
+  // u32 region: bit-sliced butterfly constants (one row of NH * M planes per level and block), bit-sliced frob_hi
+  static constexpr int abs_stride = alpha_bs_stride(NH * M);
+  static constexpr int abs_off = shared_u16 / 2, abs_len = ((SIG - 1) * abs_stride + 3) & ~3;
+  static constexpr int fhbs_off = abs_off + abs_len, fhbs_len = (NH * M + 3) & ~3;
   static constexpr int shared_u32 = fhbs_off + fhbs_len;
   static constexpr int ewp = (p::ew + 1) & ~1;
   // per warp (u32): e words | roots [t] (element, then pos << 16 | element)
@@ -928,16 +952,15 @@ __global__ void __launch_bounds__(kRootWarps * 32, 2) dec_root_kernel(const uint
   uint32_t *abs_ = rsm + LY::abs_off;
   uint32_t *fhbs = rsm + LY::fhbs_off;
   if constexpr (CT) {
-    for (int i = threadIdx.x; i < LY::twist_len; i += blockDim.x) tlog[i] = fd.fft_twist_cols[i];
+    copy_table(tlog, fd.fft_twist_cols, LY::twist_len);
   } else {
-    for (int i = threadIdx.x; i < 2 * Q - 1; i += blockDim.x) gexp[i] = fd.gexp[i];
-    for (int i = threadIdx.x; i < Q; i += blockDim.x) glog[i] = fd.glog[i];
-    for (int i = threadIdx.x; i < (2 << D); i += blockDim.x) tlog[i] = fd.fft_twist_log[i];
+    copy_table(gexp, fd.gexp, 2 * Q);
+    copy_table(glog, fd.glog, Q);
+    copy_table(tlog, fd.fft_twist_log, 2 << D);
   }
-  for (int i = threadIdx.x; i < SIG; i += blockDim.x) frlo[i] = fd.frob_lo[i];
-  for (int i = threadIdx.x; i < (SIG - 1) * LY::abs_row; i += blockDim.x)
-    abs_[(i / LY::abs_row) * LY::abs_stride + i % LY::abs_row] = fd.fft_alpha_bs[i];
-  for (int i = threadIdx.x; i < LY::fhbs_len; i += blockDim.x) fhbs[i] = fd.frob_hi_bs[i];
+  copy_table(frlo, fd.frob_lo, SIG);
+  copy_table(abs_, fd.fft_alpha_bs, 2 * (SIG - 1) * LY::abs_stride);
+  copy_table(fhbs, fd.frob_hi_bs, 2 * NH * M);
   __syncthreads();
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1353,20 +1376,21 @@ cudaError_t launch_dec_bm(const uint32_t *S2, int lds2, FieldDev fd, const Segs 
     return cudaGetLastError();
   }
   if (N < kBMBitslicedMinRows) {  // small batch: warp per request (lower latency per request)
-    // warps per block: the requests in one round over two blocks per SM when
-    // they fit (8192 requests: 27 warps on 304 blocks, where fixed 24-warp
-    // blocks left 896 requests for a second round), else kBMLatWarps
+    // warps per block: as few rounds over two blocks per SM as kBMLatWarps
+    // allows, all of them full
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long per_block = sms > 0 ? (N + 2LL * sms - 1) / (2LL * sms) : kBMLatWarps;
-    const int lw = per_block < kBMLatWarps ? (per_block > 0 ? (int)per_block : 1) : kBMLatWarps;
+    const long long blocks = 2LL * (sms > 0 ? sms : 1);
+    const long long rounds = (N + blocks * kBMLatWarps - 1) / (blocks * kBMLatWarps);
+    const int lw = (int)((N + blocks * rounds - 1) / (blocks * rounds));
     const int smem_l = BMLatLayout<SET>::bytes(lw);
+    const int threads = 32 * (lw < kBMLatCopyWarps ? kBMLatCopyWarps : lw);
     cudaError_t err = cudaFuncSetAttribute(dec_bm_lat_kernel<SET>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            BMLatLayout<SET>::bytes(kBMLatWarps));
     if (err != cudaSuccess) return err;
-    const int gl = persistent_blocks(dec_bm_lat_kernel<SET>, lw * 32, smem_l, N, lw);
-    dec_bm_lat_kernel<SET><<<gl, lw * 32, smem_l, st>>>(S2, lds2, fd, segs, Sig);
+    const int gl = persistent_blocks(dec_bm_lat_kernel<SET>, threads, smem_l, N, lw);
+    dec_bm_lat_kernel<SET><<<gl, threads, smem_l, st>>>(S2, lds2, fd, segs, Sig, lw);
     return cudaGetLastError();
   }
   warps = bm_block_warps(N, warps);

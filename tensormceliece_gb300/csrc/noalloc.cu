@@ -71,14 +71,15 @@ constexpr size_t kScratchBytes =
          DecScratch<4>::total(kMaxRequests));
 
 // per-set field/FFT tables (u16 entries): exp (2q-1) | log (q) | twist (2^(d+1)) | frob_lo (2^d) |
-// bit-sliced alpha (2 (2^d - 1) 2 m) | bit-sliced frob_hi (2 * 2 m) | zech (q), u32 tables at even offsets
-constexpr int kFieldSlot = 2 * 8192 + 8192 + 256 + 128 + 2 * 127 * 2 * 13 + 2 * 2 * 13 + 8192 + 16;
-static_assert(kFieldSlot % 2 == 0, "per-set slots must keep the u32 tables 4-byte aligned");
+// bit-sliced alpha (2 (2^d - 1) rows) | bit-sliced frob_hi (2 * 2 m) | zech (q), each 16-byte aligned
+constexpr int kFieldSlot =
+    2 * 8192 + 8192 + 256 + 128 + 2 * 127 * alpha_bs_stride(2 * 13) + 2 * 2 * 13 + 8192 + 7 * kFieldAlign;
+constexpr int kFieldSlotPadded = (kFieldSlot + kFieldAlign - 1) / kFieldAlign * kFieldAlign;
 
 }  // namespace
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
-static __device__ __align__(256) uint16_t g_noalloc_fields[GMC_NSETS][kFieldSlot];
+static __device__ __align__(256) uint16_t g_noalloc_fields[GMC_NSETS][kFieldSlotPadded];
 
 namespace {
 
@@ -123,11 +124,11 @@ int device_setup(int dev, const DeviceSetup **out) {
     const gmc_setinfo &S = set_info(set);
     const HostField &F = host_field(S.m);
     FftTables ft = build_fft_tables(S.m, S.fft_d);
-    std::vector<uint16_t> all(kFieldSlot, 0);
+    std::vector<uint16_t> all(kFieldSlotPadded, 0);
     size_t o = 0;
     bool fits = true;
     auto put = [&](const std::vector<uint16_t> &v) {
-      o += o & 1;  // u32 tables start 4-byte aligned
+      o = (o + kFieldAlign - 1) / kFieldAlign * kFieldAlign;
       const size_t at = o;
       if (o + v.size() > all.size()) {
         fits = false;
@@ -140,7 +141,7 @@ int device_setup(int dev, const DeviceSetup **out) {
     const size_t o_exp = put(F.exp), o_log = put(F.log), o_twist = put(ft.twist_log), o_flo = put(ft.frob_lo),
                  o_abs = put(ft.alpha_bs), o_fhbs = put(ft.frob_hi_bs), o_zech = put(ft.zech);
     if (!fits) return set_error(GMC_ECUDA, "gmc_dec_batch_noalloc: field table slot too small");
-    uint16_t *base = su.fields + (size_t)set * kFieldSlot;
+    uint16_t *base = su.fields + (size_t)set * kFieldSlotPadded;
     if (cudaMemcpy(base, all.data(), all.size() * 2, cudaMemcpyHostToDevice) != cudaSuccess)
       return set_error(GMC_ECUDA, "gmc_dec_batch_noalloc: field table copy failed");
     su.fd[set].gexp = base + o_exp;

@@ -31,6 +31,12 @@ struct gmc_setinfo {
 #define GMC_HD
 #endif
 
+// Words between the rows of the bit-sliced butterfly constants (one row of
+// planes per level and block): odd, so that 32 lanes reading 32 different rows
+// of the shared-memory copy hit 32 different banks. The device table has the
+// same stride, so that the kernels copy it 16 bytes at a time.
+constexpr int alpha_bs_stride(int row_words) { return row_words | 1; }
+
 // Compile-time parameters for templated kernels.
 template <int SET> struct Set;
 template <> struct Set<0> { static constexpr int m = 12, n = 3488, t = 64; };
