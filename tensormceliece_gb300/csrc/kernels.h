@@ -14,7 +14,7 @@ constexpr int kSampleThreadsMax = 128;  // sampler block size is a launch parame
 constexpr int kTailThreads = 64;
 constexpr int kTailBlocksPerSM = 14;
 constexpr int kBMWarps = 14;    // Berlekamp-Massey kernel: default and largest warps per block (32 requests per warp)
-constexpr int kBMCtWarps = 8;   // its constant-time form: largest warps per block
+constexpr int kBMCtBlocksPerSM = 3;  // its constant-time form: blocks (groups of 32 requests) resident per SM
 constexpr int kBMLatWarps = 24;  // Berlekamp-Massey latency form: largest warps per block (one request per warp)
 constexpr int kBMLatCopyWarps = 8;  // its smallest block: warps without a request help to copy the tables
 constexpr long long kBMBitslicedMinRows = 24576;  // smaller batches take the latency form
@@ -177,8 +177,7 @@ cudaError_t launch_pack_ct(const uint8_t *C, const Segs &segs, uint32_t *X, int 
 // Berlekamp-Massey: S2 (2t packed syndromes) -> Sig [N][2^fft_d] u16, the
 // error locator's coefficients by degree (the leading x^t term is implicit
 // when t = 2^fft_d).
-// warps: warps per block of the bit-sliced form (1..kBMWarps; 0 = kBMWarps;
-// the constant-time form takes at most kBMCtWarps).
+// warps: warps per block of the bit-sliced form (1..kBMWarps; 0 = kBMWarps).
 // ct: the constant-time form (inversion-free, no tables, slot bounds from the
 // iteration alone; the same locators).
 template <int SET>

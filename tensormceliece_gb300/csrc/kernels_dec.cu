@@ -107,23 +107,30 @@ struct BMLayout {
   static_assert(2 * T <= 2 * R, "ring index j - R for j < 2t");
 };
 
-// acc (2M-1 planes, unreduced) -> r (M planes) mod the field polynomial
+// acc (2M-1 planes, unreduced) -> r (M planes) mod the field polynomial, in
+// three-input XORs: with h_j the plane of x^(M+j), x^13 = x^4 + x^3 + x + 1
+// (x^12 = x^3 + 1); h_0 .. h_2 first take what falls back above x^(M-1)
 template <int M>
-__device__ __forceinline__ void bs_reduce(uint32_t (&r)[M], uint32_t (&acc)[2 * M - 1]) {
+__device__ __forceinline__ void bs_reduce(uint32_t (&r)[M], const uint32_t (&acc)[2 * M - 1]) {
+  uint32_t h[M];
 #pragma unroll
-  for (int k = 2 * M - 2; k >= M; k--) {
-    if (M == 13) {
-      acc[k - 13] ^= acc[k];
-      acc[k - 12] ^= acc[k];
-      acc[k - 10] ^= acc[k];
-      acc[k - 9] ^= acc[k];
-    } else {
-      acc[k - 12] ^= acc[k];
-      acc[k - 9] ^= acc[k];
-    }
+  for (int j = 0; j < M - 1; j++) h[j] = acc[M + j];
+  h[M - 1] = 0;
+  if constexpr (M == 13) {
+    h[0] ^= acc[22] ^ acc[23];
+    h[1] ^= acc[23] ^ acc[24];
+    h[2] ^= acc[24];
+    uint32_t pr[M];  // h_k + h_(k-1)
+#pragma unroll
+    for (int k = 0; k < M; k++) pr[k] = k ? h[k] ^ h[k - 1] : h[0];
+#pragma unroll
+    for (int k = 0; k < M; k++) r[k] = k >= 3 ? acc[k] ^ pr[k] ^ pr[k - 3] : acc[k] ^ pr[k];
+  } else {
+    h[0] ^= acc[21];
+    h[1] ^= acc[22];
+#pragma unroll
+    for (int k = 0; k < M; k++) r[k] = k >= 3 ? acc[k] ^ h[k] ^ h[k - 3] : acc[k] ^ h[k];
   }
-#pragma unroll
-  for (int k = 0; k < M; k++) r[k] = acc[k];
 }
 
 template <int SET>
@@ -397,200 +404,259 @@ __device__ __forceinline__ void bs_inv(uint32_t (&r)[M], const uint32_t (&a)[M])
   }
 }
 
-// The bit-sliced layout of dec_bm_kernel with nothing that depends on the
+// The bit-sliced arithmetic of dec_bm_kernel with nothing that depends on the
 // syndromes in an address, a branch or a trip count:
 //  - inversion-free update, no division d / b and no log tables: with b the
 //    discrepancy of the last length change, C <- b C + d B (B carrying its x
-//    shift as in dec_bm_kernel). By induction C = lambda C_lib for a nonzero
-//    scalar lambda per request (a product of b's), with the same length L and
-//    the same update decisions as the library's rule (d != 0 exactly when the
-//    library's d is), also under the truncation to t + 1 coefficients;
+//    shift). By induction C = lambda C_lib for a nonzero scalar lambda per
+//    request (a product of b's), with the same length L and the same update
+//    decisions as the library's rule (d != 0 exactly when the library's d is),
+//    also under the truncation to t + 1 coefficients;
 //  - slot bounds from n alone: deg C <= L <= n and deg B <= n + 1;
 //  - at the end every coefficient is multiplied by lambda^-1 (C_0 = lambda;
 //    one bit-sliced inversion per group), which gives the library's locator
 //    (C_0 = 1) exactly.
 // The update decisions stay per-request masks (ballots), L is selected, never
 // branched on.
-// Shared memory: M zero planes, then per warp all 2t syndromes as planes and
-// B over the 32 NS + 1 coefficient positions the slot loops address (the
-// form needs about twice the registers of the table form, so it runs at
-// kBMCtWarps warps per SM, where this layout fits).
+// A block holds one group of 32 requests, a warp per slot of 32 coefficients
+// (lane l of warp k holds C_i, i = 1 + 32 k + l): the two products of an
+// iteration take one slot's time, and a slot's planes (C, B, b, d) fit in
+// registers. Every warp adds up its slot's part of the discrepancy; the parts
+// meet in shared memory behind the iteration's one barrier, and every warp sums
+// them and keeps b and L itself. C_0 = lambda is held by one more warp as planes
+// in shared memory: its two products an iteration (lambda s_n and the next
+// lambda, b lambda) have one coefficient, so they are spread over the lanes by
+// output plane instead (a 33rd coefficient would cost a slot of its own).
+// B_i of iteration n sits at ring entry (i - n) mod (t + 2), so the new
+// B_{i+1} = (U ? C_i : B_i) replaces B_i in place.
+// Bound by the integer ALU: three plane products per coefficient and iteration.
+// 8192128, 8192 / 65536 requests: 425 / 2540 us, against 1095 / 3260 us with a
+// warp per group holding all its slots (250 registers, 8 warps per SM, and at
+// 8192 requests one or two warps on each SM).
 template <int SET>
 struct BMCtLayout {
   using p = P<SET>;
   static constexpr int T = p::t, M = p::m;
-  static constexpr int NS = (T + 1 + 31) / 32;
-  static constexpr int zero_len = 16;                 // u32: zero planes first, then the warps' areas
-  static constexpr int s_words = 2 * T * M;           // syndrome planes [j][b]
-  static constexpr int b_words = (32 * NS + 1) * M;   // B planes [i][b]
-  static constexpr int warp_u32 = s_words + b_words;
-  static constexpr int bytes(int warps) { return zero_len * 4 + warps * warp_u32 * 4; }
-  static_assert(32 * NS * M <= s_words, "C planes are staged in the syndrome area");
+  static constexpr int NS = (T + 31) / 32;             // coefficient warps per block; warp NS holds lambda
+  static constexpr int R = T + 2;                      // ring entries of B
+  static constexpr int zero_len = 16;                  // u32: zero planes (s_j, j < 0)
+  static constexpr int part_off = zero_len;            // discrepancy parts, 16 words per warp, two buffers
+  static constexpr int part_len = 2 * (NS + 1) * 16;
+  static constexpr int lam_off = part_off + part_len;  // lambda's planes at 16 .. 16 + M - 1, zeros around them
+  static constexpr int lam_len = 64;
+  static constexpr int prod_off = lam_off + lam_len;     // the unreduced planes of the lambda warp's two products
+  static constexpr int prod_len = 96;
+  static constexpr int s_off = prod_off + prod_len;    // syndrome planes [j][b], then C planes
+  static constexpr int s_len = (2 * T * M + 31) / 32 * 32;
+  static constexpr int b_off = s_off + s_len;          // B planes [ring entry][b]
+  static constexpr int b_len = R * M;
+  static constexpr int bytes = (b_off + b_len) * 4;
+  static_assert((32 * NS + 1) * M <= s_len, "C planes are staged in the syndrome area");
 };
 
+// bit j of lane l -> bit l of lane j
+__device__ __forceinline__ uint32_t transpose32(uint32_t v, int lane) {
+  uint32_t m = 0x0000FFFFu;
+#pragma unroll
+  for (int s = 16; s; s >>= 1) {
+    const uint32_t o = __shfl_xor_sync(0xffffffffu, v, s);
+    v = (lane & s) ? ((o >> s) & m) | (v & ~m) : (v & m) | ((o & m) << s);
+    m ^= m << (s >> 1);
+  }
+  return v;
+}
+
+// the first M (at most 16) words of shared memory to d, four at a time
+template <int M>
+__device__ __forceinline__ void load_planes(uint32_t (&d)[M], const uint32_t *src) {
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    const uint4 v = reinterpret_cast<const uint4 *>(src)[q];
+    d[4 * q] = v.x;
+    d[4 * q + 1] = v.y;
+    d[4 * q + 2] = v.z;
+    d[4 * q + 3] = v.w;
+  }
+  if constexpr (M == 13) d[12] = src[12];
+}
+template <int M>
+__device__ __forceinline__ void store_planes(uint32_t *dst, const uint32_t (&d)[M]) {
+#pragma unroll
+  for (int q = 0; q < 3; q++)
+    reinterpret_cast<uint4 *>(dst)[q] = make_uint4(d[4 * q], d[4 * q + 1], d[4 * q + 2], d[4 * q + 3]);
+  if constexpr (M == 13) dst[12] = d[12];
+}
+
 template <int SET>
-__global__ void __launch_bounds__(kBMCtWarps * 32, 1) dec_bm_ct_kernel(const uint32_t *__restrict__ S2, int lds2,
-                                                                       const Segs segs, uint16_t *__restrict__ Sig) {
+__global__ void __launch_bounds__((BMCtLayout<SET>::NS + 1) * 32, kBMCtBlocksPerSM)
+    dec_bm_ct_kernel(const uint32_t *__restrict__ S2, int lds2, const Segs segs, uint16_t *__restrict__ Sig) {
   using p = P<SET>;
   using LY = BMCtLayout<SET>;
   constexpr int M = p::m, T = p::t, D = p::fft_d;
-  constexpr int NS = LY::NS;
+  constexpr int NS = LY::NS, R = LY::R, THREADS = 32 * (NS + 1);
   constexpr int SIG = 1 << D;
   static_assert(M == 12 || M == 13, "field polynomial");
   extern __shared__ __align__(16) uint32_t csm[];
-  for (int i = threadIdx.x; i < LY::zero_len; i += blockDim.x) csm[i] = 0u;
-  __syncthreads();
-  const uint32_t *ZP = csm;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t *SP = csm + LY::zero_len + warp * LY::warp_u32;
-  uint32_t *BP = SP + LY::s_words;
-  const long long N = seg_rows(segs);
-  const long long ngroups = (N + 31) / 32;
-  const int nwb = blockDim.x >> 5;
-  const long long g_lo = ngroups * blockIdx.x / gridDim.x, g_hi = ngroups * (blockIdx.x + 1) / gridDim.x;
-  for (long long g = g_lo + warp; g < g_hi; g += nwb) {
-    const long long op = g * 32 + lane;
-    int seg;
-    const bool live = op < N && seg_live(segs, op, &seg);
-    const uint32_t *srow = S2 + op * lds2;
-#pragma unroll 1
-    for (int j = 0; j < 2 * T; j++) {
-      uint32_t v = 0;
-      if (live) {
-        const int bb = j * M, w = bb >> 5, sh = bb & 31;
-        v = srow[w] >> sh;
-        if (sh + M > 32) v |= srow[w + 1] << (32 - sh);
-      }
-      uint32_t mine = 0;
+  const uint32_t *ZP = csm;
+  uint32_t *SP = csm + LY::s_off, *BP = csm + LY::b_off, *LAM = csm + LY::lam_off + 16,
+           *PROD = csm + LY::prod_off;
+  const long long op = (long long)blockIdx.x * 32 + lane;
+  int seg;
+  const bool live = seg_live(segs, op, &seg);
+  if (!__any_sync(0xffffffffu, live)) return;  // the same for every warp
+  const uint32_t *srow = S2 + op * lds2;
+  for (int x = threadIdx.x; x < LY::s_off; x += THREADS) csm[x] = 0u;
+  for (int w = warp; w < LY::s_len / 32; w += NS + 1) SP[32 * w + lane] = transpose32(live ? srow[w] : 0u, lane);
+  for (int x = threadIdx.x; x < LY::b_len; x += THREADS) BP[x] = x == M ? 0xFFFFFFFFu : 0u;  // B = x
+  __syncthreads();
+  if (threadIdx.x == 0) LAM[0] = 0xFFFFFFFFu;  // C = 1
+  uint32_t C[M], bq[M];  // C_i of this lane; b of every request (warp-uniform planes)
 #pragma unroll
-      for (int b = 0; b < M; b++) {
-        const uint32_t pl = __ballot_sync(0xffffffffu, (v >> b) & 1u);
-        mine = (lane == b) ? pl : mine;
-      }
-      if (lane < M) SP[j * M + lane] = mine;
+  for (int b = 0; b < M; b++) {
+    C[b] = 0u;
+    bq[b] = b == 0 ? 0xFFFFFFFFu : 0u;
+  }
+  const int i = 1 + threadIdx.x;  // this lane's coefficient (warps below NS)
+  const bool in = i <= T;
+  int idx = i, idx0 = 0;  // ring entries of B_i and of B_0 (never read: B_0 = 0; replaced by the new B_1)
+  int L = 0;              // this lane's request
+  // the lambda warp: bit j of rmask = coefficient of x^lane in x^(M + j) mod the field polynomial
+  uint32_t rmask = 0;
+  {
+    uint32_t v = M == 13 ? 0x1Bu : 0x9u;
+    for (int j = 0; j < M - 1; j++) {
+      rmask |= ((v >> lane) & 1u) << j;
+      v = (v << 1) ^ ((v >> (M - 1)) & 1u ? (1u << M) | (M == 13 ? 0x1Bu : 0x9u) : 0u);
     }
-    uint32_t C[NS][M];
-#pragma unroll
-    for (int k = 0; k < NS; k++)
-#pragma unroll
-      for (int b = 0; b < M; b++) C[k][b] = (k == 0 && lane == 0 && b == 0) ? 0xFFFFFFFFu : 0u;
-    for (int w = lane; w < LY::b_words; w += 32) BP[w] = (w == M) ? 0xFFFFFFFFu : 0u;
-    uint32_t bq[M];  // b of every request (warp-uniform planes); b = 1
-#pragma unroll
-    for (int b = 0; b < M; b++) bq[b] = b == 0 ? 0xFFFFFFFFu : 0u;
-    __syncwarp();
-    int L = 0;  // this lane's request
+  }
+  __syncthreads();
 #pragma unroll 1
-    for (int n = 0; n < 2 * T; n++) {
-      const int bd = n < T ? n : T;          // deg C <= L <= n
-      const int bu = n + 1 < T ? n + 1 : T;  // deg B <= n + 1
-      uint32_t d[M];
-      {
-        uint32_t acc[2 * M - 1];
+  for (int n = 0; n < 2 * T; n++) {
+    const int bu = n + 1 < T ? n + 1 : T;  // deg C <= L <= n, deg B <= n + 1
+    uint32_t *part = csm + LY::part_off + (n & 1) * ((NS + 1) * 16);
+    uint32_t lam = 0;         // lambda warp: plane `lane` of lambda
+    uint32_t acc[2 * M - 1];  // b C_i, then b C_i + d B_i, unreduced
+    if (warp == NS) {
+      // output plane k = lane of lambda s_n and of b lambda
+      uint32_t c = 0, e = 0;
 #pragma unroll
-        for (int k = 0; k < 2 * M - 1; k++) acc[k] = 0;
-#pragma unroll
-        for (int k = 0; k < NS; k++) {
-          if (32 * k <= bd) {
-            const int j = n - lane - 32 * k;  // s_j, j < 0 reads the zero planes
-            const uint32_t *sp = j >= 0 ? SP + j * M : ZP;
-#pragma unroll
-            for (int b2 = 0; b2 < M; b2++) {
-              const uint32_t sv = sp[b2];
-#pragma unroll
-              for (int b1 = 0; b1 < M; b1++) acc[b1 + b2] ^= C[k][b1] & sv;
-            }
-          }
-        }
-        bs_reduce<M>(d, acc);
-#pragma unroll
-        for (int b = 0; b < M; b++) d[b] = __reduce_xor_sync(0xffffffffu, d[b]);
+      for (int j = 0; j < M; j++) {
+        const uint32_t lv = LAM[lane - j];  // zero outside lambda's planes (16 below, 19 above)
+        c ^= lv & SP[n * M + j];
+        e ^= lv & bq[j];
       }
-      uint32_t nz = 0;
-#pragma unroll
-      for (int b = 0; b < M; b++) nz |= d[b];
-      const uint32_t U = nz & __ballot_sync(0xffffffffu, 2 * L <= n);
-      L = ((U >> lane) & 1u) ? n + 1 - L : L;
-      // C_i <- b C_i + d B_i; B_{i+1} <- (U ? C_i(old) : B_i); slots in
-      // descending order (slot k's write of B_{32(k+1)} follows slot k+1's read)
-#pragma unroll
-      for (int k = NS - 1; k >= 0; k--) {
-        if (32 * k <= bu) {
-          const int i = lane + 32 * k;
-          const uint32_t *bp = BP + i * M;
-          uint32_t bi[M];
-#pragma unroll
-          for (int b = 0; b < M; b++) bi[b] = bp[b];
-          __syncwarp();
-          const bool in = (k < NS - 1) || (i <= T);
-          uint32_t r[M];
-#pragma unroll
-          for (int b = 0; b < M; b++) r[b] = (C[k][b] & bq[M - 1]) ^ (bi[b] & d[M - 1]);
-#pragma unroll
-          for (int jj = M - 2; jj >= 0; jj--) {
-            const uint32_t top = r[M - 1];
-#pragma unroll
-            for (int b = M - 1; b > 0; b--) r[b] = r[b - 1];
-            r[0] = top;
-            if (M == 13) {
-              r[1] ^= top;
-              r[3] ^= top;
-              r[4] ^= top;
-            } else {
-              r[3] ^= top;
-            }
-#pragma unroll
-            for (int b = 0; b < M; b++) r[b] ^= (C[k][b] & bq[jj]) ^ (bi[b] & d[jj]);
-          }
-          uint32_t *bn = BP + (i + 1) * M;
-#pragma unroll
-          for (int b = 0; b < M; b++) {
-            const uint32_t cold = C[k][b];
-            if (in) C[k][b] = r[b];
-            if (i + 1 <= T) bn[b] = (U & cold) | (~U & bi[b]);
-          }
-          __syncwarp();
-        }
-      }
-#pragma unroll
-      for (int b = 0; b < M; b++) bq[b] = (U & d[b]) | (~U & bq[b]);
-      if (lane < M) BP[lane] = 0;
+      lam = LAM[lane];
+      // plane M lands on a 16-byte boundary
+      PROD[16 - M + lane] = c;
+      PROD[48 + 16 - M + lane] = e;
       __syncwarp();
-    }
-    // C <- C / C_0 (C_0 = lambda != 0)
-    {
-      uint32_t c0[M], inv[M];
 #pragma unroll
-      for (int b = 0; b < M; b++) c0[b] = __shfl_sync(0xffffffffu, C[0][b], 0);
-      bs_inv<M>(inv, c0);
+      for (int q = 0; q < 3; q++) {
+        const uint4 hc = reinterpret_cast<const uint4 *>(PROD + 16)[q], he = reinterpret_cast<const uint4 *>(PROD + 64)[q];
+        const uint32_t vc[4] = {hc.x, hc.y, hc.z, hc.w}, ve[4] = {he.x, he.y, he.z, he.w};
 #pragma unroll
-      for (int k = 0; k < NS; k++) {
-        uint32_t r[M];
-        bs_mul_reg<M>(r, inv, C[k]);
-#pragma unroll
-        for (int b = 0; b < M; b++) C[k][b] = r[b];
+        for (int k = 0; k < 4; k++) {
+          const uint32_t m = 0u - ((rmask >> (4 * q + k)) & 1u);
+          c ^= vc[k] & m;
+          e ^= ve[k] & m;
+        }
       }
+      if (lane < M) {
+        part[16 * NS + lane] = c;
+        LAM[lane] = e;
+      }
+    } else if (32 * warp < bu) {
+      uint32_t d[M];
+#pragma unroll
+      for (int k = 0; k < 2 * M - 1; k++) acc[k] = 0;
+      const int j = n - i;  // s_j, j < 0 reads the zero planes
+      const uint32_t *sp = j >= 0 ? SP + j * M : ZP;
+#pragma unroll
+      for (int b2 = 0; b2 < M; b2++) {
+        const uint32_t sv = sp[b2];
+#pragma unroll
+        for (int b1 = 0; b1 < M; b1++) acc[b1 + b2] ^= C[b1] & sv;
+      }
+      bs_reduce<M>(d, acc);
+#pragma unroll
+      for (int b = 0; b < M; b++) d[b] = __reduce_xor_sync(0xffffffffu, d[b]);
+      // b C_i under the latency of the reductions
+#pragma unroll
+      for (int k = 0; k < 2 * M - 1; k++) acc[k] = 0;
+#pragma unroll
+      for (int b2 = 0; b2 < M; b2++)
+#pragma unroll
+        for (int b1 = 0; b1 < M; b1++) acc[b1 + b2] ^= bq[b1] & C[b2];
+      if (lane == 0) store_planes<M>(part + 16 * warp, d);
     }
+    __syncthreads();
+    // the parts of warps that hold no coefficient yet are zero
+    uint32_t d[M];
+    load_planes<M>(d, part + 16 * NS);
 #pragma unroll
-    for (int k = 0; k < NS; k++)
+    for (int k = 0; k < NS; k++) {
+      uint32_t v[M];
+      load_planes<M>(v, part + 16 * k);
 #pragma unroll
-      for (int b = 0; b < M; b++) SP[(lane + 32 * k) * M + b] = C[k][b];
-    __syncwarp();
-    if (live) {
-      uint16_t *sig = Sig + op * SIG;
+      for (int b = 0; b < M; b++) d[b] ^= v[b];
+    }
+    uint32_t nz = 0;
+#pragma unroll
+    for (int b = 0; b < M; b++) nz |= d[b];
+    const uint32_t U = nz & __ballot_sync(0xffffffffu, 2 * L <= n);
+    L = ((U >> lane) & 1u) ? n + 1 - L : L;
+    if (warp == NS) {
+      if (lane < M) BP[idx0 * M + lane] = U & lam;  // B_1 <- (U ? C_0(old) : B_0 = 0)
+    } else if (32 * warp < bu) {
+      // C_i <- b C_i + d B_i; B_{i+1} <- (U ? C_i(old) : B_i)
+      uint32_t *bp = BP + idx * M;
+#pragma unroll
+      for (int b2 = 0; b2 < M; b2++) {
+        const uint32_t bi = in ? bp[b2] : 0u;
+#pragma unroll
+        for (int b1 = 0; b1 < M; b1++) acc[b1 + b2] ^= d[b1] & bi;
+        if (i < T) bp[b2] = (U & C[b2]) | (~U & bi);
+      }
+      bs_reduce<M>(C, acc);  // stays zero above t
+    }
+    idx = idx == 0 ? R - 1 : idx - 1;
+    idx0 = idx0 == 0 ? R - 1 : idx0 - 1;
+#pragma unroll
+    for (int b = 0; b < M; b++) bq[b] = (U & d[b]) | (~U & bq[b]);
+  }
+  __syncthreads();  // the syndromes are read no more
+  // C <- C / C_0 (C_0 = lambda != 0)
+  if (warp < NS) {
+    uint32_t c0[M], inv[M], r[M];
+    load_planes<M>(c0, LAM);
+    bs_inv<M>(inv, c0);
+    bs_mul_reg<M>(r, inv, C);
+#pragma unroll
+    for (int b = 0; b < M; b++) SP[i * M + b] = r[b];
+  } else if (lane < M) {
+    SP[lane] = lane == 0 ? 0xFFFFFFFFu : 0u;
+  }
+  __syncthreads();
+  // the locator by degree, 8 coefficients (16 bytes of the request's row) at a time
+  if (live) {
+    uint4 *sig = reinterpret_cast<uint4 *>(Sig + op * SIG);
 #pragma unroll 1
-      for (int deg = 0; deg < SIG; deg++) {
-        const int i = T - deg;
-        uint32_t v = 0;
-        if (i >= 0) {
+    for (int u = warp; u < SIG / 8; u += NS + 1) {
+      uint32_t wd[4] = {0, 0, 0, 0};
 #pragma unroll
-          for (int b = 0; b < M; b++) v |= ((SP[i * M + b] >> lane) & 1u) << b;
+      for (int e = 0; e < 8; e++) {
+        const int deg = 8 * u + e, ci = T - deg;
+        uint32_t v = 0;
+        if (ci >= 0) {
+#pragma unroll
+          for (int b = 0; b < M; b++) v |= ((SP[ci * M + b] >> lane) & 1u) << b;
         }
         v |= (deg == 0 && L > T) ? 0x8000u : 0u;
-        sig[deg] = (uint16_t)v;
+        wd[e >> 1] |= v << (16 * (e & 1));
       }
+      sig[u] = make_uint4(wd[0], wd[1], wd[2], wd[3]);
     }
-    __syncwarp();
   }
 }
 
@@ -1366,13 +1432,11 @@ cudaError_t launch_dec_bm(const uint32_t *S2, int lds2, FieldDev fd, const Segs 
   if (warps < 0 || warps > kBMWarps) return cudaErrorInvalidValue;
   if (warps == 0) warps = kBMWarps;
   if (ct) {  // constant-time form, every batch size
-    warps = bm_block_warps(N, warps < kBMCtWarps ? warps : kBMCtWarps);
-    const int smem_ct = BMCtLayout<SET>::bytes(warps);
-    cudaError_t err = cudaFuncSetAttribute(dec_bm_ct_kernel<SET>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           BMCtLayout<SET>::bytes(kBMCtWarps));
+    using LY = BMCtLayout<SET>;
+    cudaError_t err =
+        cudaFuncSetAttribute(dec_bm_ct_kernel<SET>, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::bytes);
     if (err != cudaSuccess) return err;
-    const int gb = persistent_blocks(dec_bm_ct_kernel<SET>, warps * 32, smem_ct, (N + 31) / 32, warps);
-    dec_bm_ct_kernel<SET><<<gb, warps * 32, smem_ct, st>>>(S2, lds2, segs, Sig);
+    dec_bm_ct_kernel<SET><<<(unsigned)((N + 31) / 32), (LY::NS + 1) * 32, LY::bytes, st>>>(S2, lds2, segs, Sig);
     return cudaGetLastError();
   }
   if (N < kBMBitslicedMinRows) {  // small batch: warp per request (lower latency per request)
