@@ -14,12 +14,12 @@
 // control bits | r[0:n/8].
 //
 // Seed chains (stream 0): kg_expand, a warp (or two lanes) per key and chain
-// link, expands 16 links of every key ahead of the rounds into an expansion store
-// (more for the rare key that needs them); a chain link costs 251 sequential
-// Keccak-f permutations for 8192128, so expanding ahead keeps the chain
-// latency off the rounds.
-// Device pipeline of one round (each pending key gets k <= 8 attempts, k
-// filling 4 x SMs attempts; stream 1):
+// link, expands links of every key ahead of the rounds into an expansion store;
+// a chain link costs 251 sequential Keccak-f permutations for 8192128, so
+// expanding ahead keeps the chain latency off the rounds. A key that has its
+// winner ends its links in flight.
+// Device pipeline of one round of systematic keys (each pending key gets k <= 8
+// attempts, k filling 4 x SMs attempts; stream 1):
 //   kg_minpoly   one CTA per attempt  powers of f in GF((2^m)^t), Gauss-Jordan
 //   kg_support   one CTA per attempt  bitonic sort of (value, index) pairs
 //   kg_build     CTAs per attempt     columns of A_L (the rank test's matrix)
@@ -32,6 +32,9 @@
 //   kg_assemble  pk and sk bytes
 // Only the rank test runs on the ~70% of attempts whose A_L is singular; the
 // full elimination (4-5x the rank test's work for 8192128) runs once per key.
+// Semi-systematic attempts succeed but for ~1%, so their rounds skip the rank
+// test; calls of a few systematic keys, which leave the GPU empty, skip it too
+// and overlap the attempts of a key instead (keypair_few).
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
@@ -43,6 +46,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/gmc.h"
@@ -105,10 +109,14 @@ constexpr uint8_t kKgMinpoly = 1, kKgDistinct = 2, kKgRank = 4, kKgAll = 7;
 // alone on its scheduler), else two lanes per key (277); one lane per key took
 // 403 (1.20 ms a link for 8192128, 0.61 ms with a warp). The warp form's instructions per key are 6 times the
 // pair form's, so it is taken while every scheduler has at most two such warps.
+// done[key] (mapped host memory, set while launches are in flight) ends the
+// links of a key that has its winner: the host issues links ahead of the
+// rounds, and a link that is not needed any more returns within 8 permutations.
 constexpr int kExpandWarpKeysPerSM = 8;
 template <int SET, bool WARP>
 __global__ void __launch_bounds__(32) kg_expand_kernel(uint8_t *__restrict__ seedc, const int *__restrict__ keys,
-                                                       int nb, int a, uint8_t *__restrict__ out) {
+                                                       int nb, int a, uint8_t *__restrict__ out,
+                                                       const volatile uint8_t *done) {
   using C = KG<SET>;
   const int lane = threadIdx.x, half = lane & 1;
   const int i0 = WARP ? blockIdx.x : 16 * blockIdx.x + (lane >> 1);
@@ -130,6 +138,7 @@ __global__ void __launch_bounds__(32) kg_expand_kernel(uint8_t *__restrict__ see
     uint64_t *o = reinterpret_cast<uint64_t *>(r);
 #pragma unroll 1
     for (int b = 0; b < C::rblocks; b++) {
+      if ((b & 7) == 0 && __any_sync(0xffffffffu, done[key] != 0)) return;
       kw.permute(s);
       if (lane < 17) o[17 * b + lane] = s;
     }
@@ -144,6 +153,7 @@ __global__ void __launch_bounds__(32) kg_expand_kernel(uint8_t *__restrict__ see
     uint32_t *o = reinterpret_cast<uint32_t *>(r);
 #pragma unroll 1
     for (int b = 0; b < C::rblocks; b++) {
+      if ((b & 7) == 0 && __all_sync(0xffffffffu, done[key] != 0)) return;
       keccak_f1600_pair(s, half);
       if (live) {
 #pragma unroll
@@ -187,7 +197,9 @@ __global__ void __launch_bounds__(kMinpolyThreads) kg_minpoly_kernel(const uint8
                                                                      const uint16_t *__restrict__ gexp,
                                                                      const uint16_t *__restrict__ glog,
                                                                      uint16_t *__restrict__ gout,
-                                                                     uint8_t *__restrict__ status) {
+                                                                     uint8_t *__restrict__ status,
+                                                                 const int *__restrict__ key_of,
+                                                                 const volatile uint8_t *done) {
   using C = KG<SET>;
   using L = MinpolySmem<SET>;
   using X = ExtPoly<SET>;
@@ -215,6 +227,8 @@ __global__ void __launch_bounds__(kMinpolyThreads) kg_minpoly_kernel(const uint8
   auto mulz = [&](uint16_t x) -> uint16_t { return ex[min((int)lg[x] + log2, ZL)]; };
   // powers f^c = f^(c-1) * f
   for (int c = 2; c <= T; c++) {
+    // an attempt in flight whose key has its winner (key_of: given where attempts overlap)
+    if (key_of && (c & 15) == 0 && __syncthreads_or(tid == 0 && done[key_of[att]])) return;
     const uint16_t *prev = col + (c - 1) * T;
     if (tid < T) la[tid] = lg[prev[tid]];
     __syncthreads();
@@ -439,7 +453,10 @@ __global__ void __launch_bounds__(ElimCfg<TB>::nt, ElimCfg<TB>::minb) kg_elim_ke
                                                                   uint8_t *__restrict__ status, int need, int set_bit,
                                                                   int forward, int cl, uint16_t *__restrict__ rowid_out,
                                                                   int semi, uint8_t *__restrict__ clist_out,
-                                                                  uint16_t *__restrict__ pi_all) {
+                                                                  uint16_t *__restrict__ pi_all,
+                                                                  const int *__restrict__ key_of,
+                                                                  const volatile uint8_t *done,
+                                                                  int *__restrict__ stop) {
   using C = KG<SET>;
   using L = ElimSmem<SET, TB>;
   constexpr int MT = C::mt, NT = ElimCfg<TB>::nt;
@@ -464,6 +481,9 @@ __global__ void __launch_bounds__(ElimCfg<TB>::nt, ElimCfg<TB>::minb) kg_elim_ke
   const int R = semi ? MT - 32 : MT;
   int *clist = misc + 4;  // the window's pivot columns (offsets from R)
   for (int base = 0; base < MT;) {
+    // an attempt in flight whose key has its winner stops at a panel: one thread of the cluster reads the flag, every
+    // CTA acts on the copy in stop[slot], which is written before this panel's barrier and read after it
+    if (key_of && crank == 0 && tid == NT - 1) stop[slot] = done[key_of[slot]];
     const bool fpanel = semi && base == R;
     const int np = fpanel ? 32 : min(32, (base < R ? R : MT) - base);
     const uint32_t npmask = np == 32 ? 0xffffffffu : ((1u << np) - 1);
@@ -626,6 +646,7 @@ __global__ void __launch_bounds__(ElimCfg<TB>::nt, ElimCfg<TB>::minb) kg_elim_ke
     // every CTA of the cluster has read the panel words before any updates them
     if (cl > 1) kg_cluster_sync();
     else __syncthreads();
+    if (key_of && *(volatile int *)(stop + slot)) return;
     for (int g = (pw0 >> 5) + ((crank - (pw0 >> 5)) % cl + cl) % cl; g < ngroups; g += cl) {
       const int w0 = 32 * g;
       for (int i = tid; i < 1024; i += NT) {
@@ -761,6 +782,7 @@ template <int SET>
 __global__ void __launch_bounds__(kCbitsThreads) kg_cbits_kernel(const uint16_t *__restrict__ piall,
                                                                  const int *__restrict__ att_of,
                                                                  const int *__restrict__ out_of, int nwin,
+                                                                 const uint8_t *__restrict__ status, int need,
                                                                  uint8_t *__restrict__ cond_out,
                                                                  uint8_t *__restrict__ cb_ok) {
   using C = KG<SET>;
@@ -770,7 +792,7 @@ __global__ void __launch_bounds__(kCbitsThreads) kg_cbits_kernel(const uint16_t 
   uint32_t *A = kgsm_cb + L::a, *B = kgsm_cb + L::b, *T = kgsm_cb + L::t, *CB = kgsm_cb + L::cb;
   uint16_t *PI = reinterpret_cast<uint16_t *>(kgsm_cb + L::pi_u32);
   const int w = blockIdx.x;
-  if (w >= nwin) return;
+  if (w >= nwin || (status[att_of[w]] & need) != need) return;
   const int tid = threadIdx.x;
   const uint16_t *pi0 = piall + (long long)att_of[w] * q;
   for (int i = tid; i < q; i += kCbitsThreads) PI[i] = pi0[i];
@@ -894,7 +916,7 @@ __global__ void __launch_bounds__(kCbitsThreads) kg_cbits_kernel(const uint16_t 
 // ff ff ff ff 00 00 00 00 | g_0..g_{t-1} (LE u16) | control bits | r[0:n/8].
 template <int SET>
 __global__ void kg_assemble_kernel(const int *__restrict__ att_of, const int *__restrict__ out_of, int nwin,
-                                   const uint8_t *const *__restrict__ rptr, const uint16_t *__restrict__ gall,
+                                   const uint8_t *__restrict__ status, const uint8_t *const *__restrict__ rptr, const uint16_t *__restrict__ gall,
                                    const uint8_t *__restrict__ cond, const uint32_t *__restrict__ matF,
                                    const uint16_t *__restrict__ rowid, const uint8_t *__restrict__ clist,
                                    uint8_t *__restrict__ pk_out, uint8_t *__restrict__ sk_out) {
@@ -905,6 +927,7 @@ __global__ void kg_assemble_kernel(const int *__restrict__ att_of, const int *__
   const int w = blockIdx.y;
   if (w >= nwin) return;
   const int att = att_of[w];
+  if (status[att] != kKgAll) return;
   if (threadIdx.x == 0) {
     pivots = 0xFFFFFFFFull;
     if (clist) {
@@ -983,7 +1006,6 @@ cudaError_t kg_attrs() {
     if (e == cudaSuccess) e = smem_attr(kg_support_kernel<SET>, KG<SET>::q * 8);
     if (e == cudaSuccess) e = smem_attr(kg_build_kernel<SET>, BuildSmem<SET>::bytes);
     if (e == cudaSuccess) e = smem_attr(kg_elim_kernel<SET, kg_table_bits<SET>()>, ElimSmem<SET, kg_table_bits<SET>()>::bytes);
-    if (e == cudaSuccess) e = smem_attr(kg_elim_kernel<SET, kg_table_bits<SET>()>, ElimSmem<SET, kg_table_bits<SET>()>::bytes);
     if (e == cudaSuccess) e = smem_attr(kg_cbits_kernel<SET>, CbitsSmem<SET>::bytes);
     return e;
   }();
@@ -999,34 +1021,392 @@ constexpr long long kMaxAttemptsPerKey = 100000;
 constexpr int kMaxSpeculation = 8;        // attempts per key and round
 constexpr int kExpandBlock = 16;          // twice the minimum chain links per key of an extension block
 constexpr long long kChunkBytes = 2ll << 30;  // device-side pk + sk staging per chunk of keys
+// Calls of at most this many keys run overlapping attempts (keypair_few): their
+// full eliminations, kFewWaves per key in flight, fit the GPU side by side.
+constexpr int kFewKeys = 8;
+constexpr int kFewWaves = 4;
+constexpr int kFewCluster = 8;  // CTAs per matrix while at most half of kFewKeys share the GPU
 
-// Round state, double-buffered: the winners of round r (stream 2) read round
-// r's buffers while round r+1 (stream 1) fills the others.
+// Buffers of one round (or wave) of attempts.
 struct KgRound {
   uint8_t *status = nullptr;
   uint16_t *g = nullptr, *pi = nullptr;
-  uint32_t *matL = nullptr;
+  uint32_t *matL = nullptr;                             // the rank test's matrices
   const uint8_t **rptr = nullptr;                       // per attempt: its r in the expansion store
   int *win = nullptr;                                   // [2][wcap]: attempt, output slot
   const uint8_t **h_rptr = nullptr;                     // pinned
   uint8_t *h_status = nullptr;
   int *h_win = nullptr;
   cudaEvent_t ranked = nullptr, done = nullptr;
+  // the full eliminations' matrices and what the winners' assembly reads
+  uint32_t *matF = nullptr;
+  uint16_t *rowid = nullptr;
+  uint8_t *cond = nullptr, *clist = nullptr;
+  // keypair_few only, per attempt
+  uint8_t *cbok = nullptr;
+  int *stop = nullptr;
+
+  cudaError_t alloc_attempts(int cap, int wcap, size_t gstride, size_t q, cudaStream_t st) {
+    cudaError_t e;
+    if ((e = dalloc(&status, (size_t)cap, st)) != cudaSuccess) return e;
+    if ((e = dalloc(&g, (size_t)cap * gstride, st)) != cudaSuccess) return e;
+    if ((e = dalloc(&pi, (size_t)cap * q, st)) != cudaSuccess) return e;
+    if ((e = dalloc(&rptr, (size_t)cap, st)) != cudaSuccess) return e;
+    if ((e = dalloc(&win, (size_t)2 * wcap, st)) != cudaSuccess) return e;
+    if ((e = cudaMallocHost(&h_rptr, (size_t)cap * sizeof(void *))) != cudaSuccess) return e;
+    if ((e = cudaMallocHost(&h_status, (size_t)cap)) != cudaSuccess) return e;
+    if ((e = cudaMallocHost(&h_win, (size_t)2 * wcap * sizeof(int))) != cudaSuccess) return e;
+    if ((e = cudaEventCreateWithFlags(&ranked, cudaEventDisableTiming)) != cudaSuccess) return e;
+    return cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+  }
+  cudaError_t alloc_full(int n, size_t words, size_t mt, size_t cond_bytes, cudaStream_t st) {
+    cudaError_t e;
+    if ((e = dalloc(&matF, (size_t)n * words, st)) != cudaSuccess) return e;
+    if ((e = dalloc(&rowid, (size_t)n * mt, st)) != cudaSuccess) return e;
+    if ((e = dalloc(&cond, (size_t)n * cond_bytes, st)) != cudaSuccess) return e;
+    return dalloc(&clist, (size_t)n * 32, st);
+  }
+  // the buffers of n attempts with their full matrices, carved from a device and a pinned slab (null slabs: only
+  // advances the offsets)
+  void carve(size_t n, size_t gstride, size_t q, size_t words, size_t mt, size_t cond_bytes, uint8_t *dev,
+             size_t *dev_at, uint8_t *pinned, size_t *pinned_at) {
+    auto take = [](auto *&p, uint8_t *slab, size_t *at, size_t count) {
+      if (slab) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(slab + *at);
+      *at += (count * sizeof(*p) + 255) / 256 * 256;
+    };
+    take(status, dev, dev_at, n);
+    take(g, dev, dev_at, n * gstride);
+    take(pi, dev, dev_at, n * q);
+    take(rptr, dev, dev_at, n);
+    take(win, dev, dev_at, 2 * n);
+    take(matF, dev, dev_at, n * words);
+    take(rowid, dev, dev_at, n * mt);
+    take(cond, dev, dev_at, n * cond_bytes);
+    take(cbok, dev, dev_at, n);
+    take(stop, dev, dev_at, n);
+    take(h_rptr, pinned, pinned_at, n);
+    take(h_status, pinned, pinned_at, n);
+    take(h_win, pinned, pinned_at, 2 * n);
+  }
+  void release(cudaStream_t st) {
+    for (void *p : {(void *)status, (void *)g, (void *)pi, (void *)matL, (void *)rptr, (void *)win, (void *)matF,
+                    (void *)rowid, (void *)cond, (void *)clist})
+      if (p) cudaFreeAsync(p, st);
+    if (h_rptr) cudaFreeHost(h_rptr);
+    if (h_status) cudaFreeHost(h_status);
+    if (h_win) cudaFreeHost(h_win);
+    if (ranked) cudaEventDestroy(ranked);
+    if (done) cudaEventDestroy(done);
+  }
 };
 
-// Expansion store block: kExpandBlock chained attempts for each of nb keys,
-// expanded on stream 0 ahead of the rounds; attempt a of the block's i-th key
-// at base + (a * nb + i) * rstride.
-struct KgBlock {
-  uint8_t *base = nullptr;
-  int *keys = nullptr;    // device list (null: keys 0..nb-1)
-  int *h_keys = nullptr;  // pinned source of the list
-  int nb = 0;
-  int seq0 = 0;         // launch sequence number of the block's first link
-  int a0 = 0, nlinks = 0;  // attempts a0 .. a0 + nlinks - 1 of each of its keys
-  std::vector<int> slot;  // key -> index in the block, -1 if absent
+// The seed chains of a chunk of keys: blocks of links (consecutive attempts of
+// each of a block's keys) expanded on stream 0 ahead of their use; attempt a of
+// a block's i-th key at base + ((a - a0) * nb + i) * rstride.
+template <int SET>
+struct KgChains {
+  using C = KG<SET>;
+  struct Block {
+    uint8_t *base = nullptr;
+    int *keys = nullptr;    // device list (null: keys 0..nb-1)
+    int *h_keys = nullptr;  // pinned source of the list
+    int nb = 0;
+    int seq0 = 0;            // launch sequence number of the block's first link
+    int a0 = 0, nlinks = 0;  // attempts a0 .. a0 + nlinks - 1 of each of its keys
+    std::vector<int> slot;   // key -> index in the block, -1 if absent
+  };
+  cudaStream_t s0 = nullptr;
+  int sms = 0;
+  long long nk = 0;
+  uint8_t *seedc = nullptr;        // chain heads
+  volatile uint8_t *done = nullptr;  // mapped host memory: key has its winner
+  std::vector<Block> blocks;
+  std::vector<cudaEvent_t> links;  // one per expansion launch, in stream-0 order
+  std::vector<std::vector<int>> kblocks;  // per key: its store blocks, in chain order
+
+  cudaError_t begin(const uint8_t *seeds, long long n) {
+    nk = n;
+    kblocks.assign(n, {});
+    for (long long i = 0; i < n; i++) done[i] = 0;
+    return cudaMemcpyAsync(seedc, seeds, (size_t)n * 32, cudaMemcpyHostToDevice, s0);
+  }
+  // nlinks more links, from attempt a0, of the listed keys (null: all)
+  cudaError_t add(const std::vector<long long> *keys, int a0, int nlinks) {
+    blocks.emplace_back();  // owned by the list from here on (freed with it on any exit)
+    const int bid = (int)blocks.size() - 1;
+    Block &blk = blocks.back();
+    blk.nb = keys ? (int)keys->size() : (int)nk;
+    blk.a0 = a0;
+    blk.nlinks = nlinks;
+    blk.slot.assign(nk, -1);
+    cudaError_t e = dalloc(&blk.base, (size_t)blk.nb * nlinks * C::rstride, s0);
+    if (e != cudaSuccess) return e;
+    if (keys) {
+      if ((e = cudaMallocHost(&blk.h_keys, (size_t)blk.nb * sizeof(int))) != cudaSuccess) return e;
+      for (int i = 0; i < blk.nb; i++) blk.h_keys[i] = (int)(*keys)[i];
+      if ((e = dalloc(&blk.keys, (size_t)blk.nb, s0)) != cudaSuccess) return e;
+      if ((e = cudaMemcpyAsync(blk.keys, blk.h_keys, (size_t)blk.nb * sizeof(int), cudaMemcpyHostToDevice, s0)) !=
+          cudaSuccess)
+        return e;
+    }
+    for (int i = 0; i < blk.nb; i++) {
+      const int key = keys ? (int)(*keys)[i] : i;
+      blk.slot[key] = i;
+      kblocks[key].push_back(bid);
+    }
+    blk.seq0 = (int)links.size();
+    for (int a = 0; a < nlinks; a++) {
+      if (blk.nb <= kExpandWarpKeysPerSM * sms)
+        kg_expand_kernel<SET, true><<<blk.nb, 32, 0, s0>>>(seedc, blk.keys, blk.nb, a, blk.base, done);
+      else
+        kg_expand_kernel<SET, false><<<(blk.nb + 15) / 16, 32, 0, s0>>>(seedc, blk.keys, blk.nb, a, blk.base, done);
+      cudaEvent_t ev;
+      if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return e;
+      links.push_back(ev);
+      if ((e = cudaEventRecord(ev, s0)) != cudaSuccess) return e;
+    }
+    return cudaGetLastError();
+  }
+  // every pending key has been in every block so far (the same attempts): extend them up to `need` attempts
+  cudaError_t ensure(const std::vector<long long> &pending, int need, int at_least) {
+    const Block &last = blocks[kblocks[pending[0]].back()];
+    const int end = last.a0 + last.nlinks;
+    return need > end ? add(&pending, end, std::max(need - end, at_least)) : cudaSuccess;
+  }
+  // attempt A of a key: its r, and the launch it comes from
+  const uint8_t *attempt(long long key, int A, int *seq) const {
+    int bi = 0;
+    while (A >= blocks[kblocks[key][bi]].a0 + blocks[kblocks[key][bi]].nlinks) bi++;
+    const Block &blk = blocks[kblocks[key][bi]];
+    *seq = blk.seq0 + (A - blk.a0);
+    return blk.base + ((long long)(A - blk.a0) * blk.nb + blk.slot[key]) * C::rstride;
+  }
+  void clear(cudaStream_t st) {
+    for (Block &blk : blocks) {
+      if (blk.base) cudaFreeAsync(blk.base, st);
+      if (blk.keys) cudaFreeAsync(blk.keys, st);
+      if (blk.h_keys) cudaFreeHost(blk.h_keys);
+    }
+    blocks.clear();
+    for (cudaEvent_t ev : links) cudaEventDestroy(ev);
+    links.clear();
+  }
 };
 
+// the kernels of an attempt up to its support
+template <int SET>
+void launch_attempts(const KgRound &b, int natt, const FieldDev &fd, const int *key_of, const volatile uint8_t *done,
+                     cudaStream_t st) {
+  using C = KG<SET>;
+  kg_minpoly_kernel<SET><<<natt, kMinpolyThreads, MinpolySmem<SET>::bytes, st>>>(b.rptr, natt, fd.gexp, fd.glog, b.g,
+                                                                               b.status, key_of, done);
+  kg_support_kernel<SET><<<natt, kSupportThreads, C::q * 8, st>>>(b.rptr, natt, b.pi, b.status);
+}
+
+// full eliminations of n matrices (attempts att_of, or slot = attempt), cl CTAs each
+template <int SET>
+cudaError_t launch_full_elim(const KgRound &b, int n, const int *att_of, int need, int set_bit, int cl, bool semi,
+                             const FieldDev &fd, const int *key_of, const volatile uint8_t *done, cudaStream_t st) {
+  using C = KG<SET>;
+  kg_build_kernel<SET><<<dim3(C::rw / 8, n), kBuildThreads, BuildSmem<SET>::bytes, st>>>(
+      b.g, b.pi, att_of, b.status, b.matF, C::rw, C::rw, fd.gexp, fd.glog);
+  cudaLaunchConfig_t lc = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cl;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  lc.gridDim = dim3(n * cl);
+  lc.blockDim = dim3(ElimCfg<kg_table_bits<SET>()>::nt);
+  lc.dynamicSmemBytes = ElimSmem<SET, kg_table_bits<SET>()>::bytes;
+  lc.stream = st;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  return cudaLaunchKernelEx(&lc, kg_elim_kernel<SET, kg_table_bits<SET>()>, b.matF, (int)C::rw, (int)C::rw, att_of,
+                            b.status, need, set_bit, 0, cl, b.rowid, semi ? 1 : 0,
+                            semi ? b.clist : (uint8_t *)nullptr, semi ? b.pi : (uint16_t *)nullptr, key_of, done,
+                            b.stop);
+}
+
+// GMC_KG_TRACE=1: one stderr line per round (host clock, ms since the call)
+struct KgTrace {
+  bool on;
+  std::chrono::steady_clock::time_point t0 = std::chrono::steady_clock::now();
+  KgTrace() {
+    static const bool env = getenv("GMC_KG_TRACE") && getenv("GMC_KG_TRACE")[0] == '1';
+    on = env;
+  }
+  double ms() const {
+    return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+  }
+};
+
+// Few keys: the call is the latency of the seed chains and of one attempt's
+// kernels, and the GPU is nearly empty. Wave a runs attempt a of every key that
+// is still open, straight to the full elimination (no rank test first: its time
+// would be added to every winner), as soon as link a of the chain is there;
+// kFewWaves waves overlap, each on its own stream, the control bits beside the
+// elimination. The host takes the waves' results in order, so the first
+// successful attempt wins as in the library; done[] then ends the links,
+// minimal polynomials and eliminations still in flight for that key.
+// 8192128, one key: 4.4 ms (the key of a fourth attempt 5.2 ms), against 16.2 ms with a round of 8 attempts (8 links
+// before the first rank test) and the winner's full elimination after it.
+template <int SET>
+int keypair_few(uint8_t *pk, uint8_t *sk, const uint8_t *seeds, int nk, cudaStream_t s0, cudaStream_t s1) {
+  using C = KG<SET>;
+  int rc = GMC_OK, dev = 0;
+  const KgTrace trace;
+  FieldDev fd{};
+  KgRound W[kFewWaves];
+  cudaStream_t st[kFewWaves] = {};
+  KgChains<SET> ch;
+  uint8_t *slab = nullptr, *pinned = nullptr, *d_pk = nullptr, *d_sk = nullptr, *h_done = nullptr, *h_cbok = nullptr;
+  size_t dev_bytes = 0, pinned_bytes = 0;
+  std::vector<long long> open;
+  std::vector<long long> wave_keys[kFewWaves];
+  const int cl = 2 * nk <= kFewKeys ? kFewCluster : kElimCluster;
+  int launched = 0;
+  if (field_tables(SET, &fd) != GMC_OK) return GMC_ECUDA;
+  KG_CUDA(cudaGetDevice(&dev));
+  KG_CUDA(cudaDeviceGetAttribute(&ch.sms, cudaDevAttrMultiProcessorCount, dev));
+  KG_CUDA(kg_attrs<SET>());
+  ch.s0 = s0;
+  for (int pass = 0; pass < 2; pass++) {  // sizes, then pointers
+    size_t dev_at = 0, pinned_at = 0;
+    for (KgRound &b : W)
+      b.carve(nk, C::gstride, C::q, (size_t)C::mt * C::rw, C::mt, C::cond_bytes, slab, &dev_at, pinned, &pinned_at);
+    if (pass == 0) {
+      dev_bytes = dev_at + 256 + nk * (C::pk_bytes + C::sk_bytes);
+      pinned_bytes = pinned_at + 512;
+      KG_CUDA(dalloc(&slab, dev_bytes, s0));
+      KG_CUDA(cudaMallocHost(&pinned, pinned_bytes));
+    } else {
+      ch.seedc = slab + dev_at;
+      d_pk = ch.seedc + 256;
+      d_sk = d_pk + nk * C::pk_bytes;
+      h_done = pinned + pinned_at;
+      h_cbok = h_done + 256;
+    }
+  }
+  static_assert(kFewKeys * 32 <= 256, "seed chain heads");
+  ch.done = h_done;
+  KG_CUDA(ch.begin(seeds, nk));
+  KG_CUDA(ch.add(nullptr, 0, kFewWaves + 2));
+  for (int w = 0; w < kFewWaves; w++) {
+    KG_CUDA(cudaEventCreateWithFlags(&W[w].ranked, cudaEventDisableTiming));
+    KG_CUDA(cudaEventCreateWithFlags(&W[w].done, cudaEventDisableTiming));
+    KG_CUDA(cudaStreamCreateWithFlags(&st[w], cudaStreamNonBlocking));
+  }
+  if (trace.on) fprintf(stderr, "[keygen] set up at %.2f ms\n", trace.ms());
+  for (int i = 0; i < nk; i++) open.push_back(i);
+  for (int wave = 0; !open.empty(); wave++) {
+    // waves in flight: wave .. wave + kFewWaves - 1 (buffer = wave mod kFewWaves, free since its results were read)
+    for (; launched < wave + kFewWaves; launched++) {
+      const int bi = launched % kFewWaves;
+      KgRound &b = W[bi];
+      KG_CUDA(ch.ensure(open, launched + 2, 2));
+      const int n = (int)open.size();
+      int seq = 0;
+      wave_keys[bi] = open;
+      for (int j = 0; j < n; j++) {
+        b.h_rptr[j] = ch.attempt(open[j], launched, &seq);
+        b.h_win[j] = j;
+        b.h_win[nk + j] = (int)open[j];
+      }
+      KG_CUDA(cudaStreamWaitEvent(st[bi], ch.links[seq], 0));
+      KG_CUDA(cudaMemcpyAsync(b.rptr, b.h_rptr, (size_t)n * sizeof(void *), cudaMemcpyHostToDevice, st[bi]));
+      KG_CUDA(cudaMemcpyAsync(b.win, b.h_win, (size_t)2 * nk * sizeof(int), cudaMemcpyHostToDevice, st[bi]));
+      KG_CUDA(cudaMemsetAsync(b.status, 0, (size_t)n, st[bi]));
+      launch_attempts<SET>(b, n, fd, b.win + nk, ch.done, st[bi]);
+      KG_CUDA(cudaEventRecord(b.ranked, st[bi]));
+      KG_CUDA(cudaStreamWaitEvent(s1, b.ranked, 0));
+      kg_cbits_kernel<SET><<<n, kCbitsThreads, CbitsSmem<SET>::bytes, s1>>>(
+          b.pi, b.win, b.win, n, b.status, kKgMinpoly | kKgDistinct, b.cond, b.cbok);
+      KG_CUDA(cudaEventRecord(b.done, s1));
+      KG_CUDA(launch_full_elim<SET>(b, n, nullptr, kKgMinpoly | kKgDistinct, kKgRank, cl, false, fd, b.win + nk,
+                                    ch.done, st[bi]));
+      KG_CUDA(cudaMemcpyAsync(b.h_status, b.status, n, cudaMemcpyDeviceToHost, st[bi]));
+      KG_CUDA(cudaStreamWaitEvent(st[bi], b.done, 0));
+      KG_CUDA(cudaEventRecord(b.ranked, st[bi]));
+    }
+    const int bi = wave % kFewWaves;
+    KgRound &b = W[bi];
+    KG_CUDA(cudaEventSynchronize(b.ranked));
+    int nw = 0;
+    for (size_t j = 0; j < wave_keys[bi].size(); j++) {
+      const long long key = wave_keys[bi][j];
+      if (ch.done[key] || b.h_status[j] != kKgAll) continue;  // (a done key's later attempts may have run on)
+      ch.done[key] = 1;
+      open.erase(std::find(open.begin(), open.end(), key));
+      b.h_win[nw] = (int)j;
+      b.h_win[nk + nw] = (int)key;
+      nw++;
+    }
+    if (trace.on)
+      fprintf(stderr, "[keygen] set %d wave %d: %zu attempts, %d winners at %.2f ms\n", SET, wave,
+              wave_keys[bi].size(), nw, trace.ms());
+    if (nw) {
+      // the assembly's lists index matF, rowid and cond by attempt: one launch per winner
+      KG_CUDA(cudaMemcpyAsync(b.win, b.h_win, (size_t)2 * nk * sizeof(int), cudaMemcpyHostToDevice, st[bi]));
+      KG_CUDA(cudaMemcpyAsync(h_cbok, b.cbok, (size_t)nk, cudaMemcpyDeviceToHost, st[bi]));
+      for (int w = 0; w < nw; w++) {
+        const int j = b.h_win[w];
+        kg_assemble_kernel<SET><<<dim3(256, 1), 256, 0, st[bi]>>>(
+            b.win + w, b.win + nk + w, 1, b.status, (const uint8_t *const *)b.rptr, b.g,
+            b.cond + (size_t)j * C::cond_bytes, b.matF + (size_t)j * C::mt * C::rw, b.rowid + (size_t)j * C::mt, nullptr,
+            d_pk, d_sk);
+      }
+      KG_CUDA(cudaGetLastError());
+      KG_CUDA(cudaStreamSynchronize(st[bi]));
+      for (int w = 0; w < nw; w++)
+        if (!h_cbok[b.h_win[w]]) {
+          rc = kg_fail(GMC_EKEY, "gmc_keypair_batch: control bits do not encode the support permutation");
+          goto done;
+        }
+    }
+    if (wave >= kMaxAttemptsPerKey) {
+      rc = kg_fail(GMC_EKEY, "gmc_keypair_batch: no systematic key within the attempt limit");
+      goto done;
+    }
+  }
+  KG_CUDA(cudaMemcpyAsync(pk, d_pk, (size_t)nk * C::pk_bytes, cudaMemcpyDeviceToHost, s0));
+  KG_CUDA(cudaMemcpyAsync(sk, d_sk, (size_t)nk * C::sk_bytes, cudaMemcpyDeviceToHost, s0));
+  if (trace.on) fprintf(stderr, "[keygen] copied at %.2f ms\n", trace.ms());
+done:
+  if (h_done)
+    for (int i = 0; i < nk; i++) h_done[i] = 1;  // whatever is still in flight stops
+  cudaStreamSynchronize(s0);
+  cudaStreamSynchronize(s1);
+  for (int w = 0; w < kFewWaves; w++)
+    if (st[w]) {
+      cudaStreamSynchronize(st[w]);
+      cudaStreamDestroy(st[w]);
+    }
+  if (trace.on) fprintf(stderr, "[keygen] idle at %.2f ms\n", trace.ms());
+  ch.clear(s1);
+  for (KgRound &b : W) {
+    if (b.ranked) cudaEventDestroy(b.ranked);
+    if (b.done) cudaEventDestroy(b.done);
+  }
+  if (slab) cudaFreeAsync(slab, s1);
+  {
+    cudaError_t e = cudaStreamSynchronize(s1);
+    if (rc == GMC_OK && e != cudaSuccess) rc = kg_fail(GMC_ECUDA, std::string("gmc_keypair_batch: ") + cudaGetErrorString(e));
+  }
+  if (pinned) cudaFreeHost(pinned);
+  if (trace.on) fprintf(stderr, "[keygen] returned at %.2f ms\n", trace.ms());
+  return rc;
+}
+
+// Many keys, or the semi-systematic form.
+// Systematic keys: rounds of rank tests, double-buffered: the winners of round
+// r (stream 2) read round r's buffers while round r+1 (stream 1) fills the
+// others.
+// Semi-systematic keys: almost every attempt succeeds (the last 32 pivots come
+// from 64 columns), so a round gives every key one attempt and takes it
+// straight to the full elimination, control bits and assembly, and one link is
+// expanded ahead. 460896f, 200 keys: 17.2 ms, against 37.8 ms with 3 speculative
+// attempts per key, rank tests and 24 links expanded and waited for.
 template <int SET>
 int keypair_batch(uint8_t *pk, uint8_t *sk, const uint8_t *seeds, long long nkeys, bool semi, cudaStream_t s0,
                   cudaStream_t s1, cudaStream_t s2) {
@@ -1036,20 +1416,12 @@ int keypair_batch(uint8_t *pk, uint8_t *sk, const uint8_t *seeds, long long nkey
   int dev = 0, sms = 0, cap = 0, wcap = 0;
   long long kc = 0;
   KgRound R[2];
-  std::vector<KgBlock> blocks;
-  std::vector<cudaEvent_t> links;  // one per expansion launch, in stream-0 order
-  std::vector<std::vector<int>> kblocks;  // per key: its store blocks, in chain order
-  uint8_t *d_seedc = nullptr;
-  uint32_t *d_matF = nullptr;
-  uint16_t *d_rowid = nullptr;
-  uint8_t *d_cond = nullptr, *d_cbok = nullptr, *d_pk = nullptr, *d_sk = nullptr, *d_clist = nullptr;
+  KgChains<SET> ch;
+  uint8_t *d_cbok = nullptr, *d_pk = nullptr, *d_sk = nullptr, *h_done = nullptr;
   std::vector<long long> pending, next;
   std::vector<int> na;
   std::vector<uint8_t> h_cbok;
-  // GMC_KG_TRACE=1: one stderr line per round (host clock, ms since the call)
-  static const bool trace = getenv("GMC_KG_TRACE") && getenv("GMC_KG_TRACE")[0] == '1';
-  const auto t_start = std::chrono::steady_clock::now();
-  auto ms_now = [&] { return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count(); };
+  const KgTrace trace;
   if (field_tables(SET, &fd) != GMC_OK) return GMC_ECUDA;
   KG_CUDA(cudaGetDevice(&dev));
   KG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -1060,23 +1432,16 @@ int keypair_batch(uint8_t *pk, uint8_t *sk, const uint8_t *seeds, long long nkey
   if (const char *v = getenv("GMC_KG_CHUNK_KEYS")) kc = std::max(1ll, std::min(kc, atoll(v)));
   wcap = (int)std::min<long long>(kc, cap);
   for (KgRound &b : R) {
-    KG_CUDA(dalloc(&b.status, (size_t)cap, s1));
-    KG_CUDA(dalloc(&b.g, (size_t)cap * C::gstride, s1));
-    KG_CUDA(dalloc(&b.pi, (size_t)cap * C::q, s1));
-    KG_CUDA(dalloc(&b.matL, (size_t)cap * C::mt * C::rwl, s1));
-    KG_CUDA(dalloc(&b.rptr, (size_t)cap, s1));
-    KG_CUDA(dalloc(&b.win, (size_t)2 * wcap, s1));
-    KG_CUDA(cudaMallocHost(&b.h_rptr, (size_t)cap * sizeof(void *)));
-    KG_CUDA(cudaMallocHost(&b.h_status, (size_t)cap));
-    KG_CUDA(cudaMallocHost(&b.h_win, (size_t)2 * wcap * sizeof(int)));
-    KG_CUDA(cudaEventCreateWithFlags(&b.ranked, cudaEventDisableTiming));
-    KG_CUDA(cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming));
+    KG_CUDA(b.alloc_attempts(cap, wcap, C::gstride, C::q, s1));
+    if (!semi) KG_CUDA(dalloc(&b.matL, (size_t)cap * C::mt * C::rwl, s1));
   }
-  KG_CUDA(dalloc(&d_seedc, (size_t)kc * 32, s1));
-  KG_CUDA(dalloc(&d_matF, (size_t)wcap * C::mt * C::rw, s1));
-  KG_CUDA(dalloc(&d_rowid, (size_t)wcap * C::mt, s1));
-  KG_CUDA(dalloc(&d_cond, (size_t)wcap * C::cond_bytes, s1));
-  KG_CUDA(dalloc(&d_clist, (size_t)wcap * 32, s1));
+  // one set of full matrices: the semi-systematic rounds do not overlap, and the winners' stages run on one stream
+  KG_CUDA(R[0].alloc_full(wcap, (size_t)C::mt * C::rw, C::mt, C::cond_bytes, s1));
+  ch.s0 = s0;
+  ch.sms = sms;
+  KG_CUDA(cudaMallocHost(&h_done, (size_t)kc));
+  ch.done = h_done;
+  KG_CUDA(dalloc(&ch.seedc, (size_t)kc * 32, s1));
   KG_CUDA(dalloc(&d_cbok, (size_t)kc, s1));
   KG_CUDA(dalloc(&d_pk, (size_t)kc * C::pk_bytes, s1));
   KG_CUDA(dalloc(&d_sk, (size_t)kc * C::sk_bytes, s1));
@@ -1084,95 +1449,71 @@ int keypair_batch(uint8_t *pk, uint8_t *sk, const uint8_t *seeds, long long nkey
   for (long long k0 = 0; k0 < nkeys; k0 += kc) {
     const long long nk = std::min(kc, nkeys - k0);
     // chain heads, then the first store block for every key (stream 0 runs ahead of the rounds)
-    KG_CUDA(cudaMemcpyAsync(d_seedc, seeds + 32 * k0, (size_t)nk * 32, cudaMemcpyHostToDevice, s0));
-    kblocks.assign(nk, {});
+    KG_CUDA(ch.begin(seeds + 32 * k0, nk));
     na.assign(nk, 0);
     pending.clear();
     for (long long i = 0; i < nk; i++) pending.push_back(i);
-    auto add_block = [&](const std::vector<long long> *keys, int a0, int nlinks) -> cudaError_t {
-      blocks.emplace_back();  // owned by the list from here on (freed with it on any exit)
-      const int bid = (int)blocks.size() - 1;
-      KgBlock &blk = blocks.back();
-      blk.nb = keys ? (int)keys->size() : (int)nk;
-      blk.a0 = a0;
-      blk.nlinks = nlinks;
-      blk.slot.assign(nk, -1);
-      cudaError_t e = dalloc(&blk.base, (size_t)blk.nb * nlinks * C::rstride, s0);
-      if (e != cudaSuccess) return e;
-      if (keys) {
-        if ((e = cudaMallocHost(&blk.h_keys, (size_t)blk.nb * sizeof(int))) != cudaSuccess) return e;
-        for (int i = 0; i < blk.nb; i++) blk.h_keys[i] = (int)(*keys)[i];
-        if ((e = dalloc(&blk.keys, (size_t)blk.nb, s0)) != cudaSuccess) return e;
-        if ((e = cudaMemcpyAsync(blk.keys, blk.h_keys, (size_t)blk.nb * sizeof(int), cudaMemcpyHostToDevice,
-                                 s0)) != cudaSuccess)
-          return e;
-      }
-      for (int i = 0; i < blk.nb; i++) {
-        const int key = keys ? (int)(*keys)[i] : i;
-        blk.slot[key] = i;
-        kblocks[key].push_back(bid);
-      }
-      blk.seq0 = (int)links.size();
-      for (int a = 0; a < nlinks; a++) {
-        if (blk.nb <= kExpandWarpKeysPerSM * sms)
-          kg_expand_kernel<SET, true><<<blk.nb, 32, 0, s0>>>(d_seedc, blk.keys, blk.nb, a, blk.base);
-        else
-          kg_expand_kernel<SET, false><<<(blk.nb + 15) / 16, 32, 0, s0>>>(d_seedc, blk.keys, blk.nb, a, blk.base);
-        cudaEvent_t ev;
-        if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return e;
-        links.push_back(ev);
-        if ((e = cudaEventRecord(ev, s0)) != cudaSuccess) return e;
-      }
-      return cudaGetLastError();
-    };
     // links ahead: a key needs more than L attempts with probability ~0.71^L
     // (29% of attempts succeed for every set), so ln(nk)/0.34 + 8 links cover
-    // the whole chunk but in ~6% of calls
-    int ahead = std::min(64, std::max(12, (int)std::ceil(std::log((double)nk) / 0.3425) + 8));
+    // the whole chunk but in ~6% of calls; links of keys that are done return
+    // at once
+    int ahead = semi ? 1 : std::min(64, std::max(12, (int)std::ceil(std::log((double)nk) / 0.3425) + 8));
     // GMC_KG_AHEAD_LINKS: links expanded ahead (1..64); fewer make the extension blocks carry the chains
     if (const char *v = getenv("GMC_KG_AHEAD_LINKS")) ahead = std::max(1, std::min(64, atoi(v)));
-    KG_CUDA(add_block(nullptr, 0, ahead));
+    KG_CUDA(ch.add(nullptr, 0, ahead));
     KG_CUDA(cudaMemsetAsync(d_cbok, 0, (size_t)nk, s2));
+    KG_CUDA(cudaStreamSynchronize(s2));  // (semi-systematic rounds write it on stream 1)
     for (int round = 0; !pending.empty(); round++) {
       KgRound &b = R[round & 1];
-      if (round >= 2) KG_CUDA(cudaEventSynchronize(b.done));  // round-2's winners released these buffers
-      const int nr = (int)std::min<long long>((long long)pending.size(), cap);
-      const int k = std::max(1, std::min(kMaxSpeculation, cap / nr));
+      if (!semi && round >= 2) KG_CUDA(cudaEventSynchronize(b.done));  // round-2's winners released these buffers
+      const int nr = (int)std::min<long long>((long long)pending.size(), semi ? wcap : cap);
+      const int k = semi ? 1 : std::max(1, std::min(kMaxSpeculation, cap / nr));
       const int natt = nr * k;
-      // chains that run past their store: one more block for every pending key
-      // (every pending key has been in every block so far: the same attempts)
+      // chains that run past their store: as many more links for every pending key as this round needs, and at
+      // least an extension block's worth
       {
-        const KgBlock &last = blocks[kblocks[pending[0]].back()];
-        const int end = last.a0 + last.nlinks;
-        int need = end;
+        int need = 0;
         for (int j = 0; j < nr; j++) need = std::max(need, na[pending[j]] + k);
-        // as many links as this round needs, at least one extension block's worth
-        if (need > end) KG_CUDA(add_block(&pending, end, std::max(need - end, kExpandBlock / 2)));
+        KG_CUDA(ch.ensure(pending, need, semi ? 1 : kExpandBlock / 2));
       }
       int wait_seq = 0;
       for (int j = 0; j < nr; j++) {
         const long long key = pending[j];
         for (int a = 0; a < k; a++) {
-          const int A = na[key] + a;
-          int bi = 0;
-          while (A >= blocks[kblocks[key][bi]].a0 + blocks[kblocks[key][bi]].nlinks) bi++;
-          const KgBlock &blk = blocks[kblocks[key][bi]];
-          const int al = A - blk.a0;
-          b.h_rptr[j * k + a] = blk.base + ((long long)al * blk.nb + blk.slot[key]) * C::rstride;
-          wait_seq = std::max(wait_seq, blk.seq0 + al);
+          int seq = 0;
+          b.h_rptr[j * k + a] = ch.attempt(key, na[key] + a, &seq);
+          wait_seq = std::max(wait_seq, seq);
         }
       }
-      KG_CUDA(cudaStreamWaitEvent(s1, links[wait_seq], 0));
+      KG_CUDA(cudaStreamWaitEvent(s1, ch.links[wait_seq], 0));
       KG_CUDA(cudaMemcpyAsync(b.rptr, b.h_rptr, (size_t)natt * sizeof(void *), cudaMemcpyHostToDevice, s1));
       KG_CUDA(cudaMemsetAsync(b.status, 0, (size_t)natt, s1));
-      kg_minpoly_kernel<SET><<<natt, kMinpolyThreads, MinpolySmem<SET>::bytes, s1>>>(b.rptr, natt, fd.gexp,
-                                                                                   fd.glog, b.g, b.status);
-      kg_support_kernel<SET><<<natt, kSupportThreads, C::q * 8, s1>>>(b.rptr, natt, b.pi, b.status);
-      kg_build_kernel<SET><<<dim3(C::rwl / 8, natt), kBuildThreads, BuildSmem<SET>::bytes, s1>>>(
-          b.g, b.pi, nullptr, b.status, b.matL, C::rwl, C::rwl, fd.gexp, fd.glog);
-      kg_elim_kernel<SET, kg_table_bits<SET>()><<<natt, ElimCfg<kg_table_bits<SET>()>::nt, ElimSmem<SET, kg_table_bits<SET>()>::bytes, s1>>>(
-          b.matL, C::rwl, C::rwl, nullptr, b.status, kKgMinpoly | kKgDistinct, kKgRank, 1, 1, nullptr, semi ? 1 : 0,
-          nullptr, nullptr);
+      launch_attempts<SET>(b, natt, fd, nullptr, nullptr, s1);
+      if (semi) {
+        KgRound full = b;  // this round's attempts with the one set of full matrices
+        full.matF = R[0].matF;
+        full.rowid = R[0].rowid;
+        full.cond = R[0].cond;
+        full.clist = R[0].clist;
+        for (int j = 0; j < nr; j++) {
+          b.h_win[j] = j;
+          b.h_win[wcap + j] = (int)pending[j];
+        }
+        KG_CUDA(cudaMemcpyAsync(b.win, b.h_win, (size_t)2 * wcap * sizeof(int), cudaMemcpyHostToDevice, s1));
+        KG_CUDA(launch_full_elim<SET>(full, nr, nullptr, kKgMinpoly | kKgDistinct, kKgRank, kElimCluster, true, fd,
+                                      nullptr, nullptr, s1));
+        kg_cbits_kernel<SET><<<nr, kCbitsThreads, CbitsSmem<SET>::bytes, s1>>>(b.pi, b.win, b.win + wcap, nr, b.status,
+                                                                             kKgAll, full.cond, d_cbok);
+        kg_assemble_kernel<SET><<<dim3(256, nr), 256, 0, s1>>>(b.win, b.win + wcap, nr, b.status,
+                                                                (const uint8_t *const *)b.rptr, b.g, full.cond,
+                                                                full.matF, full.rowid, full.clist, d_pk, d_sk);
+      } else {
+        kg_build_kernel<SET><<<dim3(C::rwl / 8, natt), kBuildThreads, BuildSmem<SET>::bytes, s1>>>(
+            b.g, b.pi, nullptr, b.status, b.matL, C::rwl, C::rwl, fd.gexp, fd.glog);
+        kg_elim_kernel<SET, kg_table_bits<SET>()><<<natt, ElimCfg<kg_table_bits<SET>()>::nt, ElimSmem<SET, kg_table_bits<SET>()>::bytes, s1>>>(
+            b.matL, C::rwl, C::rwl, nullptr, b.status, kKgMinpoly | kKgDistinct, kKgRank, 1, 1, nullptr, 0, nullptr,
+            nullptr, nullptr, nullptr, nullptr);
+      }
       KG_CUDA(cudaGetLastError());
       KG_CUDA(cudaMemcpyAsync(b.h_status, b.status, natt, cudaMemcpyDeviceToHost, s1));
       KG_CUDA(cudaEventRecord(b.ranked, s1));
@@ -1184,8 +1525,11 @@ int keypair_batch(uint8_t *pk, uint8_t *sk, const uint8_t *seeds, long long nkey
         int a = 0;
         while (a < k && b.h_status[(size_t)j * k + a] != kKgAll) a++;
         if (a < k) {
-          b.h_win[nw] = j * k + a;
-          b.h_win[wcap + nw] = (int)key;
+          h_done[key] = 1;
+          if (!semi) {
+            b.h_win[nw] = j * k + a;
+            b.h_win[wcap + nw] = (int)key;
+          }
           nw++;
         } else {
           na[key] += k;
@@ -1197,46 +1541,33 @@ int keypair_batch(uint8_t *pk, uint8_t *sk, const uint8_t *seeds, long long nkey
         }
       }
       for (size_t j = nr; j < pending.size(); j++) next.push_back(pending[j]);
-      if (nw) {
-        int *watt = b.win, *wout = b.win + wcap;
+      if (nw && !semi) {
+        KgRound full = b;
+        full.matF = R[0].matF;
+        full.rowid = R[0].rowid;
+        full.cond = R[0].cond;
+        const int *watt = b.win, *wout = b.win + wcap;
         KG_CUDA(cudaStreamWaitEvent(s2, b.ranked, 0));
         KG_CUDA(cudaMemcpyAsync(b.win, b.h_win, (size_t)2 * wcap * sizeof(int), cudaMemcpyHostToDevice, s2));
-        kg_build_kernel<SET><<<dim3(C::rw / 8, nw), kBuildThreads, BuildSmem<SET>::bytes, s2>>>(
-            b.g, b.pi, watt, b.status, d_matF, C::rw, C::rw, fd.gexp, fd.glog);
-        {
-          // the winners' status has every bit: the full elimination re-derives the same pivots
-          cudaLaunchConfig_t lc = {};
-          cudaLaunchAttribute at[1];
-          at[0].id = cudaLaunchAttributeClusterDimension;
-          at[0].val.clusterDim.x = kElimCluster;
-          at[0].val.clusterDim.y = 1;
-          at[0].val.clusterDim.z = 1;
-          lc.gridDim = dim3(nw * kElimCluster);
-          lc.blockDim = dim3(ElimCfg<kg_table_bits<SET>()>::nt);
-          lc.dynamicSmemBytes = ElimSmem<SET, kg_table_bits<SET>()>::bytes;
-          lc.stream = s2;
-          lc.attrs = at;
-          lc.numAttrs = 1;
-          KG_CUDA(cudaLaunchKernelEx(&lc, kg_elim_kernel<SET, kg_table_bits<SET>()>, d_matF, (int)C::rw, (int)C::rw, (const int *)watt,
-                                     b.status, (int)kKgAll, (int)kKgAll, 0, kElimCluster, d_rowid, semi ? 1 : 0,
-                                     semi ? d_clist : (uint8_t *)nullptr, semi ? b.pi : (uint16_t *)nullptr));
-        }
-        kg_cbits_kernel<SET><<<nw, kCbitsThreads, CbitsSmem<SET>::bytes, s2>>>(b.pi, watt, wout, nw, d_cond, d_cbok);
-        kg_assemble_kernel<SET><<<dim3(256, nw), 256, 0, s2>>>(watt, wout, nw, (const uint8_t *const *)b.rptr, b.g,
-                                                                d_cond, d_matF, d_rowid, semi ? d_clist : nullptr,
-                                                                d_pk, d_sk);
+        // the winners' status has every bit: the full elimination re-derives the same pivots
+        KG_CUDA(launch_full_elim<SET>(full, nw, watt, kKgAll, kKgAll, kElimCluster, false, fd, nullptr, nullptr, s2));
+        kg_cbits_kernel<SET><<<nw, kCbitsThreads, CbitsSmem<SET>::bytes, s2>>>(b.pi, watt, wout, nw, b.status, kKgAll,
+                                                                             full.cond, d_cbok);
+        kg_assemble_kernel<SET><<<dim3(256, nw), 256, 0, s2>>>(watt, wout, nw, b.status,
+                                                                (const uint8_t *const *)b.rptr, b.g, full.cond,
+                                                                full.matF, full.rowid, nullptr, d_pk, d_sk);
         KG_CUDA(cudaGetLastError());
       }
       KG_CUDA(cudaEventRecord(b.done, s2));
-      if (trace)
+      if (trace.on)
         fprintf(stderr, "[keygen] set %d round %d: %d keys x %d attempts (link <= %d, %zu blocks), %d winners, "
-                        "ranked at %.2f ms\n", SET, round, nr, k, wait_seq, blocks.size(), nw, ms_now());
+                        "ranked at %.2f ms\n", SET, round, nr, k, wait_seq, ch.blocks.size(), nw, trace.ms());
       pending.swap(next);
     }
     KG_CUDA(cudaStreamSynchronize(s2));
-    if (trace) fprintf(stderr, "[keygen] winners done at %.2f ms\n", ms_now());
+    if (trace.on) fprintf(stderr, "[keygen] winners done at %.2f ms\n", trace.ms());
     KG_CUDA(cudaStreamSynchronize(s0));
-    if (trace) fprintf(stderr, "[keygen] expansion done at %.2f ms\n", ms_now());
+    if (trace.on) fprintf(stderr, "[keygen] expansion done at %.2f ms\n", trace.ms());
     h_cbok.resize(nk);
     KG_CUDA(cudaMemcpy(h_cbok.data(), d_cbok, (size_t)nk, cudaMemcpyDeviceToHost));
     for (long long i = 0; i < nk; i++)
@@ -1246,41 +1577,24 @@ int keypair_batch(uint8_t *pk, uint8_t *sk, const uint8_t *seeds, long long nkey
       }
     KG_CUDA(cudaMemcpy(pk + k0 * C::pk_bytes, d_pk, (size_t)nk * C::pk_bytes, cudaMemcpyDeviceToHost));
     KG_CUDA(cudaMemcpy(sk + k0 * C::sk_bytes, d_sk, (size_t)nk * C::sk_bytes, cudaMemcpyDeviceToHost));
-    for (KgBlock &blk : blocks) {
-      cudaFreeAsync(blk.base, s1);
-      if (blk.keys) cudaFreeAsync(blk.keys, s1);
-      if (blk.h_keys) cudaFreeHost(blk.h_keys);
-    }
-    blocks.clear();
-    for (cudaEvent_t ev : links) cudaEventDestroy(ev);
-    links.clear();
+    ch.clear(s1);
   }
 done:
+  if (h_done)
+    for (long long i = 0; i < kc; i++) h_done[i] = 1;  // links still in flight return
   cudaStreamSynchronize(s0);
   cudaStreamSynchronize(s1);
   cudaStreamSynchronize(s2);
-  for (KgBlock &blk : blocks) {
-    if (blk.base) cudaFreeAsync(blk.base, s1);
-    if (blk.keys) cudaFreeAsync(blk.keys, s1);
-    if (blk.h_keys) cudaFreeHost(blk.h_keys);
-  }
-  for (cudaEvent_t ev : links) cudaEventDestroy(ev);
-  for (KgRound &b : R) {
-    for (void *p : {(void *)b.status, (void *)b.g, (void *)b.pi, (void *)b.matL, (void *)b.rptr, (void *)b.win})
-      if (p) cudaFreeAsync(p, s1);
-    if (b.h_rptr) cudaFreeHost(b.h_rptr);
-    if (b.h_status) cudaFreeHost(b.h_status);
-    if (b.h_win) cudaFreeHost(b.h_win);
-    if (b.ranked) cudaEventDestroy(b.ranked);
-    if (b.done) cudaEventDestroy(b.done);
-  }
-  for (void *p : {(void *)d_seedc, (void *)d_matF, (void *)d_rowid, (void *)d_cond, (void *)d_cbok, (void *)d_pk,
-                  (void *)d_sk, (void *)d_clist})
+  ch.clear(s1);
+  for (KgRound &b : R) b.release(s1);
+  for (void *p : {(void *)ch.seedc, (void *)d_cbok, (void *)d_pk, (void *)d_sk})
     if (p) cudaFreeAsync(p, s1);
   {
     cudaError_t e = cudaStreamSynchronize(s1);
     if (rc == GMC_OK && e != cudaSuccess) rc = kg_fail(GMC_ECUDA, std::string("gmc_keypair_batch: ") + cudaGetErrorString(e));
   }
+  if (h_done) cudaFreeHost(h_done);
+  if (trace.on) fprintf(stderr, "[keygen] returned at %.2f ms\n", trace.ms());
   return rc;
 }
 #undef KG_CUDA
@@ -1312,12 +1626,18 @@ extern "C" int gmc_keypair_batch(int set, unsigned char *pk, unsigned char *sk, 
   if (e != cudaSuccess) {
     rc = kg_fail(GMC_ECUDA, std::string("gmc_keypair_batch: ") + cudaGetErrorString(e));
   } else {
+    const bool few = !semi && nkeys <= kFewKeys;
     switch (set) {
-      case 0: rc = keypair_batch<0>(pk, sk, seeds, nkeys, semi, s0, s1, s2); break;
-      case 1: rc = keypair_batch<1>(pk, sk, seeds, nkeys, semi, s0, s1, s2); break;
-      case 2: rc = keypair_batch<2>(pk, sk, seeds, nkeys, semi, s0, s1, s2); break;
-      case 3: rc = keypair_batch<3>(pk, sk, seeds, nkeys, semi, s0, s1, s2); break;
-      case 4: rc = keypair_batch<4>(pk, sk, seeds, nkeys, semi, s0, s1, s2); break;
+#define GMC_KG_RUN(S)                                                                                          \
+  case S:                                                                                                      \
+    rc = few ? keypair_few<S>(pk, sk, seeds, (int)nkeys, s0, s1) : keypair_batch<S>(pk, sk, seeds, nkeys, semi, s0, s1, s2); \
+    break;
+      GMC_KG_RUN(0)
+      GMC_KG_RUN(1)
+      GMC_KG_RUN(2)
+      GMC_KG_RUN(3)
+      GMC_KG_RUN(4)
+#undef GMC_KG_RUN
     }
   }
   if (s0) cudaStreamDestroy(s0);
