@@ -302,8 +302,8 @@ int gmc_get_dec_constant_time(void);
  * of the decoding kernels (bm_warps: Berlekamp-Massey warps of 32 requests,
  * 1..14, default 14, not used by the constant-time form; root_warps:
  * root-finding warps of one request, 1..8, default 8) and the
- * pipelined sampler's resident warps per SM (sample_sm_warps, 0 = as many as
- * fit, the default); gmc_tune_set_launch / gmc_tune_get_launch set and read
+ * pipelined sampler's resident warps per SM (sample_sm_warps, 0 = the
+ * default, 16); gmc_tune_set_launch / gmc_tune_get_launch set and read
  * them by hand. */
 int gmc_autotune(int set, long long n, const char *cache_path);
 int gmc_autotune_load(const char *cache_path);

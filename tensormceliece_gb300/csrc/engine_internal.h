@@ -48,7 +48,7 @@ struct SetTune {
   int gemm_stages = 4;        // tcgen05 GEMM pipeline depth (2, 3 or 4 A/X buffers per CTA)
   int bm_warps = kBMWarps;    // Berlekamp-Massey (bit-sliced form) warps per block: 32 requests each
   int root_warps = 8;         // root-finding warps per block: one request each
-  int sample_sm_warps = 0;    // pipelined sampler: resident warps per SM (0 = as many as fit)
+  int sample_sm_warps = 0;    // pipelined sampler: resident warps per SM (0 = the default, kSamplePipeWarps)
   int tuned = 0;              // 1 when measured on this device
   double enc_ms = 0, dec_ms = 0;
   long long n = 0;

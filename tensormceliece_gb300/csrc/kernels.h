@@ -7,6 +7,8 @@
 namespace gmc {
 
 constexpr int kSampleWarpsPerSM = 8;     // sampler: resident warps per SM (lanes fetch requests)
+constexpr int kSamplePipeWarps = 16;     // pipelined sampler: resident warps per SM unless tuned
+constexpr int kSampleGroupWarps = 2;     // its groups: warps per scheduler before a warp gets a further group
 constexpr int kSampleThreadsMax = 128;  // sampler block size is a launch parameter (32, 64 or 128)
 // hash kernels: 64-thread blocks, 32 requests each (two lanes per request), 14
 // of them resident per SM, so that 65536 requests run in one wave of 13-14
@@ -122,7 +124,7 @@ cudaError_t launch_transpose_pk(const uint32_t *T, int lda, int mt, int k, uint3
 // counter: 4 bytes of device scratch (zeroed here, on st) that nothing else
 // touches until the sampler ends; the pipelines lend the first word of the
 // buffer the sampler does not write (S in dense mode, Ens in sparse mode).
-// sm_warps: resident warps per SM of the pipelined sampler (0 = as many as fit).
+// sm_warps: resident warps per SM of the pipelined sampler (0 = the default, kSamplePipeWarps).
 // mark (optional): called after each kernel with its stage name (profiling).
 template <int SET>
 cudaError_t launch_sample(const uint8_t *seeds, const Segs &segs, uint32_t *E, int lde, uint32_t *Ens, int ldx,

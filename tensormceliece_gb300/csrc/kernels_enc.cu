@@ -239,41 +239,49 @@ __global__ void __launch_bounds__(kSampleThreadsMax) sample_kernel(const uint8_t
 }
 
 // ---------------------------------------------------------------- pipelined sampling
-// The seed chain's next state is the first 32 bytes of an attempt's first
-// Keccak-f block, so only that block is on the chain's critical path; the
-// attempt's further squeeze blocks (P - 1 of them: P = 2 for 348864 and
-// 8192128, 3 for 460896, 4 for 6688128 and 6960119) are not. A request is
-// held by a group of G >= P lanes: at every step lane 0 of the group starts
-// the next attempt (absorb 64 || state, permute) while lane r < P permutes the
-// state lane r - 1 left in shared memory a step earlier (block r of an older
-// attempt; the state is not held in registers through the check below); all
-// lanes permute in lockstep, so a step costs one permutation and an attempt
-// completes every step once the pipeline is full. Each block's 17 output
-// words go to the attempt's slot of a per-group ring in shared memory; when
-// block P - 1 lands, the warp checks the attempt (candidate filter, first t
-// kept, repeats) exactly as the lane-per-request form does, and a success
-// drops the group's younger attempts. Groups take further requests from the
-// launch-wide counter like the lanes of sample_kernel. Per request this costs
-// P - 1 speculative first blocks and P - 1 steps of pipeline fill, but the
-// chain's critical path is one permutation per attempt instead of P, which
-// matters most for the slowest chains of a batch (about 24 attempts for the
-// slowest of 65536 requests).
+// A Keccak state is held by two lanes (keccak_f1600_pair), a warp holds 16, and
+// all permute in lockstep: a step is one permutation. The warp then checks
+// every attempt whose last block landed (candidate filter, first t kept,
+// repeats) and finishes the successful ones, one at a time. An attempt needs P
+// blocks (P = 2 for 348864 and 8192128, 3 for 460896, 4 for 6688128 and
+// 6960119). Two ways to fill the 16 pairs:
+//  - pair per request, while the launch has more requests than pairs: a pair
+//    runs its request's blocks in turn, P steps an attempt, and takes the next
+//    request from the launch-wide counter after a success. No permutation is
+//    wasted;
+//  - group of P pairs per request, for the few requests left to a warp once the
+//    counter has run out, and for batches that do not fill the pairs: the seed
+//    chain's next state is the first 32 bytes of an attempt's first block, so
+//    pair 0 of the group starts the next attempt (absorb 64 || state, permute) at
+//    every step while pair r permutes the state that pair r - 1 left in shared
+//    memory a step earlier (block r of an older attempt). An attempt completes
+//    every step, P times as fast for the chain, at P - 1 speculative attempts
+//    per request; the slowest of 65536 requests needs about 24 attempts.
+// 65536 requests, sampler with the sparse syndrome, against one lane per state in
+// speculative groups of 2 or 4 lanes throughout: 348864 212 / 273 us, 460896
+// 416 / 586, 6688128 677 / 817, 6960119 559 / 698, 8192128 377 / 428; 3001
+// requests: 72 / 104, 105 / 184, 175 / 243, 128 / 173, 124 / 173 us.
+// Bound: the Keccak instructions and the per-attempt checks while the counter
+// lasts, then the longest chains (a step of one warp is about 7100 cycles of
+// Keccak and 3500 around it).
 template <int SET>
 struct PipeLayout {
   using p = P<SET>;
   static constexpr int perms = (p::cand_bytes + 135) / 136;  // Keccak-f blocks per attempt
-  static constexpr int G = perms <= 2 ? 2 : 4;                // lanes per group
-  static constexpr int NG = 32 / G;                          // groups per warp at most
+  static constexpr int NP = 16;                              // pairs per warp
+  static constexpr int NG = NP / perms;                      // groups per warp
   static constexpr int raw_words = (p::cand_bytes + 7) / 8;  // u64 words of one attempt's draw
+  static constexpr int slot_words = raw_words | 1;           // odd u64 stride: slots on distinct banks
   static constexpr int bm_words = (p::ew + 1) & ~1;
-  static constexpr int group_words = perms * raw_words + 1;  // odd u64 stride: groups on distinct banks
   static constexpr int cand_off = bm_words * 4;
-  static constexpr int state_off = cand_off + (p::t * 2 + 7) / 8 * 8;  // [25][32] u64 block states
-  static constexpr int ring_off = state_off + 25 * 32 * 8;
-  static constexpr int warp_bytes = ring_off + NG * group_words * 8;
-  static_assert(perms <= G && raw_words <= 17 * perms, "pipeline geometry");
+  static constexpr int state_off = cand_off + (p::t * 2 + 7) / 8 * 8;  // [25][32] u32 block states
+  static constexpr int ring_off = state_off + 25 * 32 * 4;
+  static constexpr int warp_bytes = ring_off + NP * slot_words * 8;
+  static_assert(raw_words <= 17 * perms && raw_words > 17 * (perms - 1) && raw_words > 4, "pipeline geometry");
 };
 
+// groups = 0: pair per request first, then the warp's last requests as groups; else only groups, at most `groups`
+// per warp
 template <int SET, bool SPARSE>
 __global__ void __launch_bounds__(kSampleThreadsMax)
     sample_pipe_kernel(const uint8_t *__restrict__ seeds, const Segs segs, uint32_t *__restrict__ E, int lde,
@@ -281,113 +289,91 @@ __global__ void __launch_bounds__(kSampleThreadsMax)
                        unsigned int *__restrict__ counter, int groups) {
   using p = P<SET>;
   using LY = PipeLayout<SET>;
-  constexpr int PP = LY::perms, G = LY::G, RW = LY::raw_words, NCW = (p::t + 31) / 32;
+  constexpr int PP = LY::perms, NG = LY::NG, RW = LY::raw_words, NCW = (p::t + 31) / 32;
   constexpr int ncand = p::cand_bytes / 2;
   constexpr uint32_t mask = p::q - 1;
   constexpr int sh = p::mt % 32, w0 = p::mt / 32;
   extern __shared__ __align__(16) uint32_t sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int half = lane & 1, pair = lane >> 1;
   uint8_t *wb = reinterpret_cast<uint8_t *>(sm) + (size_t)warp * LY::warp_bytes;
   uint32_t *bm = reinterpret_cast<uint32_t *>(wb);
   uint16_t *cand = reinterpret_cast<uint16_t *>(wb + LY::cand_off);
-  uint64_t *sts = reinterpret_cast<uint64_t *>(wb + LY::state_off);
-  uint64_t *ring = reinterpret_cast<uint64_t *>(wb + LY::ring_off);
+  uint32_t *sts = reinterpret_cast<uint32_t *>(wb + LY::state_off);
+  uint32_t *ring = reinterpret_cast<uint32_t *>(wb + LY::ring_off);
   for (int w = lane; w < LY::bm_words; w += 32) bm[w] = 0;
   __syncwarp();
-  const int g = lane / G, r = lane % G;
-  const bool chain = r == 0 && g < groups;  // the lane that owns the group's request and seed chain
   const long long N = seg_rows(segs);
-  bool has = false, exhausted = !chain;
+  const bool seed_words = (reinterpret_cast<uintptr_t>(seeds) & 3) == 0;
+  // the request of this pair (its group's, in lanes of pair 0): words 2i + half of the current attempt's state
+  bool has = false;
   long long op = 0;
-  int myseg = 0, attempt = 0;
-  uint64_t st[4] = {0, 0, 0, 0};
-  bool valid = false;  // this lane holds block r of attempt att of the group's request
-  int att = 0;
-#pragma unroll 1
-  while (true) {
-    // chain lanes without a request take the next ones (segment gaps are skipped)
-    const uint32_t need = __ballot_sync(0xffffffffu, !has && !exhausted);
+  int myseg = 0;
+  uint32_t st[4] = {0, 0, 0, 0};
+
+  // pairs that want a request take the next ones (segment gaps are skipped); false when the counter has run out
+  auto fetch = [&](bool want) -> bool {
+    const uint32_t need = __ballot_sync(0xffffffffu, want && half == 0);
+    bool more = true;
     if (need) {
       const int leader = __ffs(need) - 1;
       unsigned int base = 0;
       if (lane == leader) base = atomicAdd(counter, (unsigned int)__popc(need));
       base = __shfl_sync(0xffffffffu, base, leader);
-      if ((need >> lane) & 1) {
-        const long long idx = (long long)base + __popc(need & ((1u << lane) - 1));
+      if (want) {
+        const long long idx = (long long)base + __popc(need & ((1u << (lane & ~1)) - 1));
         if (idx >= N) {
-          exhausted = true;
+          more = false;
         } else {
           op = idx;
           has = seg_live(segs, idx, &myseg);
-          attempt = 0;
           if (has) {
-            const uint8_t *sd = seeds + 32 * idx;
+            const uint8_t *sd = seeds + 32 * idx + 4 * half;
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-              uint64_t v = 0;
+              uint32_t v = 0;
+              if (seed_words) {
+                v = *reinterpret_cast<const uint32_t *>(sd + 8 * i);
+              } else {
 #pragma unroll
-              for (int b = 0; b < 8; b++) v |= (uint64_t)sd[8 * i + b] << (8 * b);
+                for (int b = 0; b < 4; b++) v |= (uint32_t)sd[8 * i + b] << (8 * b);
+              }
               st[i] = v;
             }
           }
         }
       }
     }
-    if (!__any_sync(0xffffffffu, has || valid)) {
-      if (__all_sync(0xffffffffu, exhausted)) break;
-      continue;
-    }
-    // lane 0 of a group starts its request's next attempt (SHAKE256 absorb of
-    // {64} || state); lane r > 0 continues the block state lane r - 1 left in
-    // shared memory a step earlier
-    if (r == 0) {
-      valid = has;
-      att = attempt;
-    }
-    uint64_t s[25];
-    if (r == 0) {
+    return more;
+  };
+  // SHAKE256 absorb of {64} || state
+  auto absorb = [&](uint32_t (&A)[25]) {
+    uint32_t prev = 64u << 24;
 #pragma unroll
-      for (int i = 0; i < 25; i++) s[i] = 0;
-      s[0] = 64ull | (st[0] << 8);
-      s[1] = (st[0] >> 56) | (st[1] << 8);
-      s[2] = (st[1] >> 56) | (st[2] << 8);
-      s[3] = (st[2] >> 56) | (st[3] << 8);
-      s[4] = (st[3] >> 56) | (0x1Full << 8);
-      s[16] = 0x8000000000000000ull;
-    } else {
-#pragma unroll
-      for (int i = 0; i < 25; i++) s[i] = sts[i * 32 + lane - 1];
+    for (int i = 0; i < 4; i++) {
+      const uint32_t o = __shfl_xor_sync(0xffffffffu, st[i], 1);
+      A[i] = __funnelshift_l(half ? o : prev, st[i], 8);
+      prev = o;
     }
-    __syncwarp();  // every predecessor state read before this step's states overwrite them
-    keccak_f1600(s);
+    A[4] = half ? 0u : __funnelshift_l(prev, 0x1Fu, 8);
 #pragma unroll
-    for (int i = 0; i < 25; i++) sts[i * 32 + lane] = s[i];
-    if (valid) {
-      uint64_t *dst = ring + (size_t)g * LY::group_words + (size_t)(att % PP) * RW;
+    for (int i = 5; i < 25; i++) A[i] = 0;
+    if (half) A[16] = 0x80000000u;
+  };
+  // block r's output words go to an attempt's slot
+  auto squeeze = [&](const uint32_t (&A)[25], int slot, int r) {
+    uint32_t *dst = ring + (size_t)slot * LY::slot_words * 2 + half;
 #pragma unroll
-      for (int i = 0; i < 17; i++) {
-        const int w = 17 * r + i;
-        if (w < RW) dst[w] = s[i];
-      }
-      if (r == 0) {
-        st[0] = s[0];
-        st[1] = s[1];
-        st[2] = s[2];
-        st[3] = s[3];
-        attempt++;
-      }
+    for (int i = 0; i < 17; i++) {
+      const int w = 17 * r + i;
+      if (w < RW) dst[2 * w] = A[i];
     }
-    __syncwarp();
-    // attempts whose last block landed: filter, first t kept, repeats; one group at a time
-    uint32_t pend = __ballot_sync(0xffffffffu, valid && r == PP - 1);
-    uint32_t succ = 0;  // bit per group
-#pragma unroll 1
-    while (pend) {
-      const int L = __ffs(pend) - 1;
-      pend &= pend - 1;
-      const int gg = L / G, owner = gg * G;
-      const int a = __shfl_sync(0xffffffffu, att, L);
-      const uint16_t *raw = reinterpret_cast<const uint16_t *>(ring + (size_t)gg * LY::group_words + (size_t)(a % PP) * RW);
+  };
+  // one complete attempt in `slot` (warp-uniform arguments): filter, first t kept, repeats; a success writes e (and
+  // e[mt:n] or the syndrome)
+  auto check = [&](int slot, long long opr, int seg) -> bool {
+    const uint16_t *raw = reinterpret_cast<const uint16_t *>(ring + (size_t)slot * LY::slot_words * 2);
+    if constexpr (!p::full) {
       int total = 0;
 #pragma unroll
       for (int base = 0; base < ncand; base += 32) {
@@ -396,7 +382,7 @@ __global__ void __launch_bounds__(kSampleThreadsMax)
         bool keep = false;
         if (i < ncand) {
           v = raw[i] & mask;
-          keep = p::full || v < (uint32_t)p::n;
+          keep = v < (uint32_t)p::n;
         }
         const uint32_t bal = __ballot_sync(0xffffffffu, keep);
         const int idx = total + __popc(bal & ((1u << lane) - 1));
@@ -404,54 +390,172 @@ __global__ void __launch_bounds__(kSampleThreadsMax)
         total += __popc(bal);
       }
       __syncwarp();
-      if (total < p::t) continue;  // too few candidates below n: the attempt fails (warp-uniform)
-      uint32_t vv[NCW];
-      bool dup = false;
+      if (total < p::t) return false;  // too few candidates below n (warp-uniform)
+    }
+    auto pos_of = [&](int c) -> int { return p::full ? (int)(raw[c] & mask) : (int)cand[c]; };
+    uint32_t vv[NCW];
+    bool dup = false;
 #pragma unroll
-      for (int i = 0; i < NCW; i++) {
-        const int c = lane + 32 * i;
-        vv[i] = 0xFFFFFFFFu;
-        if (c < p::t) {
-          const uint32_t v = cand[c];
-          vv[i] = v;
-          const uint32_t bit = 1u << (v & 31);
-          dup |= (atomicOr(&bm[v >> 5], bit) & bit) != 0;
+    for (int i = 0; i < NCW; i++) {
+      const int c = lane + 32 * i;
+      vv[i] = 0xFFFFFFFFu;
+      if (c < p::t) {
+        const uint32_t v = (uint32_t)pos_of(c);
+        vv[i] = v;
+        const uint32_t bit = 1u << (v & 31);
+        dup |= (atomicOr(&bm[v >> 5], bit) & bit) != 0;
+      }
+    }
+    const bool good = !__any_sync(0xffffffffu, dup);
+    if (good) {
+      uint32_t *erow = E + opr * lde;
+      for (int w = lane; w < p::ew; w += 32) erow[w] = bm[w];
+      if (SPARSE) {
+        sparse_syndrome_row<SET>(pos_of, keys.TT[seg], keys.ldtt, S + opr * lds, lane);
+      } else {
+        uint32_t *xrow = Ens + opr * ldx;
+        for (int w = lane; w < p::kw; w += 32) {
+          const uint32_t lo = bm[w0 + w];
+          const uint32_t hi = (w0 + w + 1 < p::ew) ? bm[w0 + w + 1] : 0u;
+          xrow[w] = sh ? ((lo >> sh) | (hi << (32 - sh))) : lo;
         }
       }
-      const bool anydup = __any_sync(0xffffffffu, dup);
-      if (!anydup) {
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < NCW; i++)
+      if (vv[i] != 0xFFFFFFFFu) bm[vv[i] >> 5] = 0;
+    __syncwarp();
+    return good;
+  };
+
+  bool exhausted = false;
+  if (groups == 0) {
+    // pair per request
+    int blk = 0;  // the block of the current attempt this step permutes
+    uint32_t nst[4] = {0, 0, 0, 0};
+#pragma unroll 1
+    while (true) {
+      if (!fetch(!has && !exhausted)) exhausted = true;
+      const uint32_t live = __ballot_sync(0xffffffffu, has && half == 0);
+      if (__all_sync(0xffffffffu, exhausted || has) && __any_sync(0xffffffffu, exhausted) && __popc(live) <= NG) break;
+      if (!live) continue;
+      uint32_t A[25];
+      absorb(A);
+      if (blk) {
+#pragma unroll
+        for (int i = 0; i < 25; i++) A[i] = sts[i * 32 + lane];
+      }
+      keccak_f1600_pair(A, half);
+      squeeze(A, pair, blk);
+      if (blk == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) nst[i] = A[i];
+      }
+      blk++;
+      if (blk < PP) {
+#pragma unroll
+        for (int i = 0; i < 25; i++) sts[i * 32 + lane] = A[i];
+      }
+      __syncwarp();
+      uint32_t pend = __ballot_sync(0xffffffffu, has && blk == PP && half == 0);
+      uint32_t succ = 0;  // bit per pair's even lane
+#pragma unroll 1
+      while (pend) {
+        const int o = __ffs(pend) - 1;
+        pend &= pend - 1;
+        if (check(o >> 1, __shfl_sync(0xffffffffu, op, o), __shfl_sync(0xffffffffu, myseg, o))) succ |= 1u << o;
+      }
+      if (blk == PP || !has) {  // (an idle pair's next request starts at block 0)
+        blk = 0;
+        if ((succ >> (lane & ~1)) & 1) has = false;
+#pragma unroll
+        for (int i = 0; i < 4; i++) st[i] = nst[i];
+      }
+    }
+    // the warp's last requests as groups, each from the start of its current attempt
+    {
+      const uint32_t live = __ballot_sync(0xffffffffu, has && half == 0);
+      const int g = pair / PP, cnt = __popc(live);
+      int src = lane;
+      uint32_t l = live;
+      for (int i = 0; i < cnt; i++) {  // g-th live pair
+        if (i == g) src = (__ffs(l) - 1) | half;
+        l &= l - 1;
+      }
+      op = __shfl_sync(0xffffffffu, op, src);
+      myseg = __shfl_sync(0xffffffffu, myseg, src);
+#pragma unroll
+      for (int i = 0; i < 4; i++) st[i] = __shfl_sync(0xffffffffu, st[i], src);
+      has = pair == g * PP && g < cnt;
+      exhausted = true;
+    }
+    __syncwarp();
+  }
+
+  // group of PP pairs per request
+  const int g = pair / PP, r = pair - g * PP;
+  const bool chain = r == 0 && g < (groups ? groups : NG) && g < NG;  // the pair that owns the request and its chain
+  if (!chain) {
+    has = false;
+    exhausted = true;
+  }
+  int attempt = 0, att = 0;
+  bool valid = false;  // this pair holds block r of attempt att of the group's request
+#pragma unroll 1
+  while (true) {
+    const bool idle = !has;
+    if (!fetch(!has && !exhausted)) exhausted = true;
+    if (idle && has) attempt = 0;
+    if (!__any_sync(0xffffffffu, has || valid)) {
+      if (__all_sync(0xffffffffu, exhausted)) break;
+      continue;
+    }
+    // pair 0 of a group starts its request's next attempt; pair r > 0 continues the state pair r - 1 left a step
+    // earlier
+    uint32_t A[25];
+    absorb(A);
+    if (r == 0) {
+      valid = has;
+      att = attempt;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 25; i++) A[i] = sts[i * 32 + lane - 2];
+    }
+    __syncwarp();  // every predecessor state read before this step's states overwrite them
+    keccak_f1600_pair(A, half);
+#pragma unroll
+    for (int i = 0; i < 25; i++) sts[i * 32 + lane] = A[i];
+    if (valid) {
+      squeeze(A, g * PP + att % PP, r);
+      if (r == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) st[i] = A[i];
+        attempt++;
+      }
+    }
+    __syncwarp();
+    uint32_t pend = __ballot_sync(0xffffffffu, valid && r == PP - 1 && half == 0);
+    uint32_t succ = 0;  // bit per group
+#pragma unroll 1
+    while (pend) {
+      const int o = __ffs(pend) - 1;
+      pend &= pend - 1;
+      const int gg = (o >> 1) / PP, owner = gg * PP * 2;
+      const int a = __shfl_sync(0xffffffffu, att, o);
+      if (check(gg * PP + a % PP, __shfl_sync(0xffffffffu, op, owner), __shfl_sync(0xffffffffu, myseg, owner)))
         succ |= 1u << gg;
-        const long long opr = __shfl_sync(0xffffffffu, op, owner);
-        uint32_t *erow = E + opr * lde;
-        for (int w = lane; w < p::ew; w += 32) erow[w] = bm[w];
-        if (SPARSE) {
-          sparse_syndrome_row<SET>([&](int c) { return (int)cand[c]; },
-                                   keys.TT[__shfl_sync(0xffffffffu, myseg, owner)], keys.ldtt, S + opr * lds, lane);
-        } else {
-          uint32_t *xrow = Ens + opr * ldx;
-          for (int w = lane; w < p::kw; w += 32) {
-            const uint32_t lo = bm[w0 + w];
-            const uint32_t hi = (w0 + w + 1 < p::ew) ? bm[w0 + w + 1] : 0u;
-            xrow[w] = sh ? ((lo >> sh) | (hi << (32 - sh))) : lo;
-          }
-        }
-      }
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < NCW; i++)
-        if (vv[i] != 0xFFFFFFFFu) bm[vv[i] >> 5] = 0;
-      __syncwarp();
     }
     // a success ends the request: its younger attempts in flight are dropped
     if ((succ >> g) & 1) {
       valid = false;
       if (r == 0) has = false;
     }
-    // block r of an attempt moves one lane along the group (its state is in shared memory)
-    const bool vin = __shfl_up_sync(0xffffffffu, valid ? 1 : 0, 1, G) != 0;
-    const int ain = __shfl_up_sync(0xffffffffu, att, 1, G);
+    // block r of an attempt moves one pair along the group (its state is in shared memory)
+    const bool vin = __shfl_up_sync(0xffffffffu, valid ? 1 : 0, 2) != 0;
+    const int ain = __shfl_up_sync(0xffffffffu, att, 2);
     if (r > 0) {
-      valid = vin && r < PP;
+      valid = vin && g < NG;
       att = ain;
     }
   }
@@ -664,11 +768,9 @@ static cudaError_t launch_sample_mode(const uint8_t *seeds, const Segs &segs, ui
   // requests, so the last slow chains hold few warps (kSampleWarpsPerSM)
   const int warps = threads / 32;
   int per_sm_target = (kSampleWarpsPerSM + warps - 1) / warps;
-  // pipelined form (every set and batch size measured faster than the
-  // lane-per-request form: 348864 / 460896 / 6688128 / 6960119 / 8192128 at
-  // 65536 requests 0.31 / 0.63 / 0.89 / 0.77 / 0.57 ms against 0.37 / 0.80 /
-  // 1.00 / 0.82 / 0.70 ms, and up to 2.3x at 16384); groups take further
-  // requests when the batch outnumbers them
+  // pipelined form: 16 resident warps per SM while the batch fills them (8 / 12 / 16 / 20 / 24 warps, 8192128,
+  // 65536 requests: 490 / 404 / 377 / 384 / 398 us); as groups only, two warps per scheduler before a warp gets a
+  // further group (8192128, 3001 requests, one / two warps: 142 / 124 us)
   if (sample_pipelined()) {
     using PL = PipeLayout<SET>;
     auto kern = sample_pipe_kernel<SET, SPARSE>;
@@ -679,18 +781,15 @@ static cudaError_t launch_sample_mode(const uint8_t *seeds, const Segs &segs, ui
     int pper = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pper, kern, threads, psmem);
     if (pper < 1) pper = 1;
-    // the pipelined form fills the SMs (no tail cap: each warp's tail is one chain's)
-    const int ptarget = sample_sm_warps > 0 && (sample_sm_warps + warps - 1) / warps < pper
-                            ? (sample_sm_warps + warps - 1) / warps
-                            : pper;
-    const long long pslots = (long long)sms * ptarget * warps;
-    // active groups per warp: the smallest power of two with which the
-    // resident warps hold the whole batch at once, at most 32 / G
+    const int want_warps = sample_sm_warps > 0 ? sample_sm_warps : kSamplePipeWarps;
+    const int ptarget = (want_warps + warps - 1) / warps < pper ? (want_warps + warps - 1) / warps : pper;
+    const long long resident = (long long)sms * ptarget;  // blocks
+    // groups per warp where groups hold the whole batch: as many as keep one warp on every scheduler
     int groups = 1;
-    while (groups < PL::NG && (long long)groups * pslots < N) groups <<= 1;
-    const long long per_block = (long long)warps * groups;
+    while (groups < PL::NG && (long long)groups * 4 * sms * kSampleGroupWarps < N) groups++;
+    if ((long long)groups * resident * warps < N) groups = 0;  // pair per request
+    const long long per_block = (long long)warps * (groups ? groups : PL::NP);
     const long long need = (N + per_block - 1) / per_block;
-    const long long resident = (long long)sms * ptarget;
     const long long blocks = need < resident ? need : resident;
     kern<<<(unsigned)blocks, threads, psmem, st>>>(seeds, segs, E, lde, Ens, ldx, keys, S, lds, counter, groups);
     err = cudaGetLastError();

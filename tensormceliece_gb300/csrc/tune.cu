@@ -6,7 +6,7 @@
 // Candidates, tuned greedily in this order: the engine of the encapsulation
 // syndrome (sparse column gather in the sampler, or the tcgen05 GEMM) crossed
 // with the sampler's block size (32, 64, 128); the pipelined sampler's resident
-// warps per SM (as many as fit, 16 or 8); the GEMM engine of the
+// warps per SM (16 or 8); the GEMM engine of the
 // decapsulation front end (CUDA-core popcount or tcgen05); the tcgen05 GEMM's
 // pipeline depth (2, 3 or 4 A/X stages per CTA, when either op uses that
 // engine); and the requests per block of the two decoding kernels
@@ -243,9 +243,9 @@ extern "C" int gmc_autotune(int set, long long n, const char *cache_path) {
           best.sample_threads = threads[ti];
         }
       }
-    // resident warps per SM of the pipelined sampler (0: as many as fit)
-    const int smw[3] = {0, 16, 8};
-    for (int wi = 1; wi < 3; wi++) {
+    // resident warps per SM of the pipelined sampler (0: the default, 16)
+    const int smw[2] = {0, 8};
+    for (int wi = 1; wi < 2; wi++) {
       SetTune t = best;
       t.sample_sm_warps = smw[wi];
       tune_put(set, t);

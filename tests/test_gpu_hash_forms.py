@@ -1,6 +1,6 @@
 """The session-key hash runs as a warp per request up to four requests per SM and as two lanes per request
 (16 per warp) beyond: both forms against the oracle around that line, with a last warp that is not full, and
-with ciphertext and key buffers at odd, even and word-aligned addresses (byte, half-word and word stores)."""
+with seed, ciphertext and key buffers at odd, even and word-aligned addresses (byte, half-word and word accesses)."""
 import os
 
 import numpy as np
@@ -30,12 +30,13 @@ def test_hash_forms(keys, sid):
     cts = oc.copy()
     cts[::7, 3] ^= 4
     od, orc = O.dec_batch(sid, sk, cts, threads=THREADS)
-    d_seeds = torch.from_numpy(seeds).cuda()
+    d_seeds = torch.zeros(seeds.size + 8, dtype=torch.uint8, device="cuda")
     for n, off in ((1, 0), (1, 3), (33, 2), (line, 1), (line + 1, 0), (line + 17, 1), (line + 17, 2)):
         c = torch.zeros(n * cb + 8, dtype=torch.uint8, device="cuda")
         k = torch.zeros(n * 32 + 8, dtype=torch.uint8, device="cuda")
         rc = torch.full((n,), 7, dtype=torch.int32, device="cuda")
-        pub.enc_batch_dev(c.data_ptr() + off, k.data_ptr() + off, d_seeds.data_ptr(), n)
+        d_seeds[off:off + 32 * n] = torch.from_numpy(seeds[:n].reshape(-1)).cuda()
+        pub.enc_batch_dev(c.data_ptr() + off, k.data_ptr() + off, d_seeds.data_ptr() + off, n)
         torch.cuda.synchronize()
         ch, kh = c.cpu().numpy(), k.cpu().numpy()
         assert (ch[off:off + n * cb].reshape(n, cb) == oc[:n]).all(), (n, off)
