@@ -46,6 +46,7 @@ template <int SET, bool PC>
 __global__ void pack_ct_kernel(const uint8_t *__restrict__ C, const Segs segs, uint32_t *__restrict__ X, int ldx) {
   using p = P<SET>;
   constexpr int CB = p::synd_bytes + (PC ? 32 : 0);  // ciphertext row bytes
+  chain_trigger();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long op = idx / ldx;
   const int w = (int)(idx % ldx);
@@ -146,10 +147,12 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
   extern __shared__ __align__(16) uint32_t bsm[];
   uint16_t *gexp = reinterpret_cast<uint16_t *>(bsm) + LY::exp_off;
   uint16_t *glog = reinterpret_cast<uint16_t *>(bsm) + LY::log_off;
+  chain_trigger();
   copy_table(gexp, fd.gexp, Q);
   copy_table(glog, fd.glog, Q);
   for (int i = threadIdx.x; i < LY::zero_len; i += blockDim.x) bsm[LY::zero_off + i] = 0u;
   __syncthreads();
+  chain_wait();
   const uint32_t *ZP = bsm + LY::zero_off;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t *SP = bsm + LY::shared_u32 + warp * LY::warp_u32;
@@ -504,7 +507,9 @@ __global__ void __launch_bounds__((BMCtLayout<SET>::NS + 1) * 32, kBMCtBlocksPer
   const long long op = (long long)blockIdx.x * 32 + lane;
   int seg;
   const bool live = seg_live(segs, op, &seg);
+  chain_trigger();
   if (!__any_sync(0xffffffffu, live)) return;  // the same for every warp
+  chain_wait();
   const uint32_t *srow = S2 + op * lds2;
   for (int x = threadIdx.x; x < LY::s_off; x += THREADS) csm[x] = 0u;
   for (int w = warp; w < LY::s_len / 32; w += NS + 1) SP[32 * w + lane] = transpose32(live ? srow[w] : 0u, lane);
@@ -715,6 +720,7 @@ __global__ void __launch_bounds__(kBMLatWarps * 32, 2) dec_bm_lat_kernel(const u
   uint16_t *gexp = lsm + LY::exp_off;
   uint16_t *glog = lsm + LY::log_off;
   uint16_t *zech = lsm + LY::zech_off;
+  chain_trigger();
   copy_table(gexp, fd.gexp, 2 * Q);
   copy_table(glog, fd.glog, Q);
   copy_table(zech, fd.zech, Q);
@@ -729,6 +735,7 @@ __global__ void __launch_bounds__(kBMLatWarps * 32, 2) dec_bm_lat_kernel(const u
   }
   __syncthreads();
   if (warp >= nwb) return;  // warps that only help to copy the tables
+  chain_wait();
   const long long N = seg_rows(segs);
   const long long nwarps = (long long)gridDim.x * nwb;
   for (long long op = (long long)blockIdx.x * nwb + warp; op < N; op += nwarps) {
@@ -1017,6 +1024,7 @@ __global__ void __launch_bounds__(kRootWarps * 32, 2) dec_root_kernel(const uint
   uint16_t *frlo = sh16 + LY::frlo_off;
   uint32_t *abs_ = rsm + LY::abs_off;
   uint32_t *fhbs = rsm + LY::fhbs_off;
+  chain_trigger();
   if constexpr (CT) {
     copy_table(tlog, fd.fft_twist_cols, LY::twist_len);
   } else {
@@ -1028,6 +1036,7 @@ __global__ void __launch_bounds__(kRootWarps * 32, 2) dec_root_kernel(const uint
   copy_table(abs_, fd.fft_alpha_bs, 2 * (SIG - 1) * LY::abs_stride);
   copy_table(fhbs, fd.frob_hi_bs, 2 * NH * M);
   __syncthreads();
+  chain_wait();
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t *wbase = rsm + LY::shared_u32 + warp * LY::warp_u32;
@@ -1332,6 +1341,7 @@ __global__ void __launch_bounds__(kTailThreads, WARP ? 1 : PC ? kTailBlocksPerSM
   const bool live = seg_live(segs, op0 + r, &seg);
   const uint32_t livemask = __ballot_sync(0xffffffffu, live);
   if (!livemask) return;
+  chain_wait();
   // lanes of rows that are not live hash the warp's first live row and store nothing
   const int src_lane = live ? lane : __ffs(livemask) - 1;
   const long long op = op0 + (WARP ? 0 : src_lane >> 1);
@@ -1436,8 +1446,8 @@ cudaError_t launch_dec_bm(const uint32_t *S2, int lds2, FieldDev fd, const Segs 
     cudaError_t err =
         cudaFuncSetAttribute(dec_bm_ct_kernel<SET>, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::bytes);
     if (err != cudaSuccess) return err;
-    dec_bm_ct_kernel<SET><<<(unsigned)((N + 31) / 32), (LY::NS + 1) * 32, LY::bytes, st>>>(S2, lds2, segs, Sig);
-    return cudaGetLastError();
+    return launch_chained(segs, dec_bm_ct_kernel<SET>, (unsigned)((N + 31) / 32), (LY::NS + 1) * 32, LY::bytes, st, S2, lds2,
+                          segs, Sig);
   }
   if (N < kBMBitslicedMinRows) {  // small batch: warp per request (lower latency per request)
     // warps per block: as few rounds over two blocks per SM as kBMLatWarps
@@ -1454,8 +1464,7 @@ cudaError_t launch_dec_bm(const uint32_t *S2, int lds2, FieldDev fd, const Segs 
                                            BMLatLayout<SET>::bytes(kBMLatWarps));
     if (err != cudaSuccess) return err;
     const int gl = persistent_blocks(dec_bm_lat_kernel<SET>, threads, smem_l, N, lw);
-    dec_bm_lat_kernel<SET><<<gl, threads, smem_l, st>>>(S2, lds2, fd, segs, Sig, lw);
-    return cudaGetLastError();
+    return launch_chained(segs, dec_bm_lat_kernel<SET>, gl, threads, smem_l, st, S2, lds2, fd, segs, Sig, lw);
   }
   warps = bm_block_warps(N, warps);
   const int smem_bm = BMLayout<SET>::bytes(warps);
@@ -1463,8 +1472,7 @@ cudaError_t launch_dec_bm(const uint32_t *S2, int lds2, FieldDev fd, const Segs 
                                          BMLayout<SET>::bytes(kBMWarps));
   if (err != cudaSuccess) return err;
   const int gb = persistent_blocks(dec_bm_kernel<SET>, warps * 32, smem_bm, (N + 31) / 32, warps);
-  dec_bm_kernel<SET><<<gb, warps * 32, smem_bm, st>>>(S2, lds2, fd, segs, Sig);
-  return cudaGetLastError();
+  return launch_chained(segs, dec_bm_kernel<SET>, gb, warps * 32, smem_bm, st, S2, lds2, fd, segs, Sig);
 }
 
 template <int SET, bool CT>
@@ -1477,8 +1485,7 @@ static cudaError_t launch_dec_root_form(const uint16_t *Sig, const uint32_t *S2,
                                          RootLayout<SET, CT>::bytes(kRootWarps));
   if (err != cudaSuccess) return err;
   const int gr = persistent_blocks(dec_root_kernel<SET, CT>, warps * 32, smem_rt, N, warps);
-  dec_root_kernel<SET, CT><<<gr, warps * 32, smem_rt, st>>>(Sig, S2, lds2, keys, fd, segs, E, lde, ok);
-  return cudaGetLastError();
+  return launch_chained(segs, dec_root_kernel<SET, CT>, gr, warps * 32, smem_rt, st, Sig, S2, lds2, keys, fd, segs, E, lde, ok);
 }
 
 template <int SET>
@@ -1525,6 +1532,8 @@ __global__ void __launch_bounds__(256) benes_ct_kernel(uint32_t *__restrict__ E,
   constexpr int M = p::m, Q = p::q, T = p::t, N = p::n;
   constexpr int WPL = Q / 32 / 32;  // words per lane
   constexpr int LW = Q / 64;         // control words per layer
+  chain_trigger();
+  chain_wait();
   const int lane = threadIdx.x & 31;
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
   const long long NR = seg_rows(segs);
@@ -1596,6 +1605,8 @@ __global__ void ct_check_kernel(const uint32_t *__restrict__ S3, int lds3, const
                                 int *__restrict__ okio, const Segs segs) {
   using p = P<SET>;
   constexpr int TM = p::t * p::m, TW = (TM + 31) / 32;
+  chain_trigger();
+  chain_wait();
   const long long op = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   int seg;
   if (op >= seg_rows(segs) || !seg_live(segs, op, &seg)) return;
@@ -1621,14 +1632,12 @@ cudaError_t launch_dec_ct_finish(const DecKeys &keys, const GemmKeys &htt, int e
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long want = (N + 7) / 8;
   const int blocks = (int)(want < 8LL * sms ? want : 8LL * sms);
-  benes_ct_kernel<SET><<<blocks, 256, 0, st>>>(E, lde, ok, keys, segs);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_chained(segs, benes_ct_kernel<SET>, blocks, 256, 0, st, E, lde, ok, keys, segs);
   if (e != cudaSuccess) return e;
   e = launch_gf2_gemm_seg(engine, htt, segs, ct_htt_words(p::n), (p::t * p::m + kGemmRowTile - 1) / kGemmRowTile *
                           kGemmRowTile, E, lde, ct_htt_words(p::n), S3, lds3, (p::t * p::m + 31) / 32, err, st);
   if (e != cudaSuccess) return e;
-  ct_check_kernel<SET><<<(unsigned)((N + 127) / 128), 128, 0, st>>>(S3, lds3, S2, lds2, ok, segs);
-  return cudaGetLastError();
+  return launch_chained(segs, ct_check_kernel<SET>, (unsigned)((N + 127) / 128), 128, 0, st, S3, lds3, S2, lds2, ok, segs);
 }
 
 // HTT[r][w] bit b = bit r of HT[32 w + b] (r < t m, 32 w + b < n): the first t syndromes of every code position
@@ -1660,17 +1669,14 @@ cudaError_t launch_dec_tail(const uint32_t *E, int lde, const int *ok, const uin
   const long long N = seg_rows(segs);
   if (N <= 0) return cudaSuccess;
   auto launch = [&](auto kern, int rows_per_block) {
-    kern<<<(unsigned)((N + rows_per_block - 1) / rows_per_block), kTailThreads, 0, st>>>(E, lde, ok, C, keys, K, rc,
-                                                                                       segs);
+    return launch_chained(segs, kern, (unsigned)((N + rows_per_block - 1) / rows_per_block), kTailThreads, 0, st, E, lde, ok, C,
+                          keys, K, rc, segs);
   };
-  if (hash_warp_form(segs)) {
-    if (pc) launch(dec_tail_kernel<SET, true, true>, kTailThreads / 32);
-    else launch(dec_tail_kernel<SET, false, true>, kTailThreads / 32);
-  } else {
-    if (pc) launch(dec_tail_kernel<SET, true, false>, kTailThreads / 2);
-    else launch(dec_tail_kernel<SET, false, false>, kTailThreads / 2);
-  }
-  return cudaGetLastError();
+  if (hash_warp_form(segs))
+    return pc ? launch(dec_tail_kernel<SET, true, true>, kTailThreads / 32)
+              : launch(dec_tail_kernel<SET, false, true>, kTailThreads / 32);
+  return pc ? launch(dec_tail_kernel<SET, true, false>, kTailThreads / 2)
+            : launch(dec_tail_kernel<SET, false, false>, kTailThreads / 2);
 }
 
 #define GMC_INST_DEC(SET)                                                                                       \

@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(kSampleThreadsMax) sample_kernel(const uint8_t
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t *bm = sm + warp * (LY::warp_bytes / 4);
   uint16_t *cand = reinterpret_cast<uint16_t *>(bm + LY::bm_words);
+  chain_trigger();
   for (int w = lane; w < LY::bm_words; w += 32) bm[w] = 0;
   __syncwarp();
   const long long N = seg_rows(segs);
@@ -301,6 +302,7 @@ __global__ void __launch_bounds__(kSampleThreadsMax)
   uint16_t *cand = reinterpret_cast<uint16_t *>(wb + LY::cand_off);
   uint32_t *sts = reinterpret_cast<uint32_t *>(wb + LY::state_off);
   uint32_t *ring = reinterpret_cast<uint32_t *>(wb + LY::ring_off);
+  chain_trigger();
   for (int w = lane; w < LY::bm_words; w += 32) bm[w] = 0;
   __syncwarp();
   const long long N = seg_rows(segs);
@@ -615,6 +617,7 @@ __global__ void __launch_bounds__(kTailThreads, WARP ? 1 : PC ? kTailBlocksPerSM
   const bool live = seg_live(segs, op0 + r, &seg);
   const uint32_t livemask = __ballot_sync(0xffffffffu, live);
   if (!livemask) return;
+  chain_wait();
   const uint32_t badmask = __ballot_sync(0xffffffffu, (pk_bad_mask >> seg) & 1u);
   // lanes of rows that are not live hash the warp's first live row and store nothing
   const long long op = live ? op0 + r : op0 + (WARP ? 0 : (__ffs(livemask) - 1) >> 1);
@@ -734,9 +737,7 @@ bool hash_warp_form(const Segs &segs) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  long long live = 0;
-  for (int i = 0; i < segs.nseg; i++) live += segs.nreq[i];
-  return live <= (long long)kHashWarpsPerSM * sms;
+  return seg_live_rows(segs) <= (long long)kHashWarpsPerSM * sms;
 }
 
 // GMC_SAMPLE_PIPELINE=0 in the environment (read once per process) puts
@@ -837,17 +838,14 @@ cudaError_t launch_finalize(const uint32_t *E, int lde, const uint32_t *S, int l
   const long long N = seg_rows(segs);
   if (N <= 0) return cudaSuccess;
   auto launch = [&](auto kern, int rows_per_block) {
-    kern<<<(unsigned)((N + rows_per_block - 1) / rows_per_block), kTailThreads, 0, st>>>(E, lde, S, lds, C, K, segs,
-                                                                                       pk_bad_mask);
+    return launch_chained(segs, kern, (unsigned)((N + rows_per_block - 1) / rows_per_block), kTailThreads, 0, st, E, lde, S,
+                          lds, C, K, segs, pk_bad_mask);
   };
-  if (hash_warp_form(segs)) {
-    if (pc) launch(finalize_kernel<SET, true, true>, kTailThreads / 32);
-    else launch(finalize_kernel<SET, false, true>, kTailThreads / 32);
-  } else {
-    if (pc) launch(finalize_kernel<SET, true, false>, kTailThreads / 2);
-    else launch(finalize_kernel<SET, false, false>, kTailThreads / 2);
-  }
-  return cudaGetLastError();
+  if (hash_warp_form(segs))
+    return pc ? launch(finalize_kernel<SET, true, true>, kTailThreads / 32)
+              : launch(finalize_kernel<SET, false, true>, kTailThreads / 32);
+  return pc ? launch(finalize_kernel<SET, true, false>, kTailThreads / 2)
+            : launch(finalize_kernel<SET, false, false>, kTailThreads / 2);
 }
 
 #define GMC_INST_ENC(SET)                                                                                        \

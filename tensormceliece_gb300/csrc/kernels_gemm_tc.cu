@@ -191,6 +191,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gf2_gemm_tc(const GemmKeys keys
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   int *last_copy = reinterpret_cast<int *>(tmem_slot + 2);  // [STAGES]: last stage copied per buffer
 
+  chain_trigger();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ktiles = (mtiles + 1) >> 1;  // key tiles of 256 rows (the last one half when mtiles is odd)
   const long long ntile_all = (long long)ktiles * rtiles;
@@ -218,6 +219,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gf2_gemm_tc(const GemmKeys keys
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   constexpr uint32_t idesc = idesc_f8f6f4_e4m3(TC_REQ, TC_KEYN);
+  chain_wait();  // (the key image too may have been written just before: gmc_gf2_gemm_dev)
 
   if (warp < TC_EXP_WARPS) {
     // request stagers: SPLIT threads share each 128-bit stage row; thread tid
@@ -431,9 +433,8 @@ cudaError_t launch_gf2_gemm_tc(const GemmKeys &keys, const Segs &segs, int rows_
   const int mtiles = rows_pad / kTcM;
   const long long rtiles = rows / TC_REQ, tiles = rtiles * ((mtiles + 1) / 2);
   const int grid = (int)(tiles < sms ? tiles : sms);  // persistent: one CTA per SM (smem and TMEM bound)
-  kern<<<grid, TC_THREADS, smem, st>>>(keys, segs, kw_pad / (kTcKB / 32), mtiles, rtiles, X, ldx, Out, ldo,
-                                       out_words, err);
-  return cudaGetLastError();
+  return launch_chained(segs, kern, (unsigned)grid, TC_THREADS, smem, st, keys, segs, kw_pad / (kTcKB / 32), mtiles, rtiles, X,
+                        ldx, Out, ldo, out_words, err);
 }
 
 // ---------------------------------------------------------------- tcgen05 FP8 peak
