@@ -7,7 +7,7 @@
 // Decapsulation of n ciphertexts (one secret key):
 //   pack_ct                       ct bytes -> words
 //   gf2_gemm (F x c)              -> 2t syndromes of the Goppa code
-//   decode (one warp per request) BM, additive FFT, error, re-encryption check
+//   decode (one warp per request) BM, additive FFT, error, weight
 //   dec_tail (n threads)          K = H(b, e or s, c)
 // Reference flow: mceliece-gpu-params/main.cu:228-239 (encaps), 352-370 (decaps).
 #include <cuda_runtime.h>
@@ -344,8 +344,7 @@ extern "C" int gmc_sk_load(gmc_key **out, int id, const unsigned char *sk) {
   k->dk.LW2 = k->tabs + 2 * n;
   k->dk.invL = k->tabs + 3 * n;
   k->dk.s = k->s;
-  k->dk.HT = k->HT;
-  k->dk.ldh = h.ldh;
+  k->ldh = h.ldh;
   k->dk.cond = k->cond;
   *out = k;
   return GMC_OK;
@@ -362,8 +361,6 @@ extern "C" void gmc_key_free(gmc_key *key) {
   cudaFree(key->s);
   cudaFree(key->HT);
   cudaFree(key->cond);
-  cudaFree(key->htt);
-  cudaFree(key->htt8);
   delete key;
 }
 
@@ -515,52 +512,7 @@ static cudaError_t gemm_keys(const gmc_key *const *keys, int nkeys, int engine, 
 int gmc::dec_e_words(int set, bool ct) {
   const gmc_setinfo &S = set_info(set);
   const int tab = round_up((S.n + 31) / 32, 4);
-  return ct ? std::max(S.q / 32, ct_htt_words(S.n)) : tab;
-}
-
-// the first-t syndrome matrix of a secret key (and its FP8 image for the tensor-core engine), built on first use
-static cudaError_t key_ct(const gmc_key *kc, int engine, cudaStream_t st) {
-  gmc_key *k = const_cast<gmc_key *>(kc);
-  std::lock_guard<std::mutex> lk(*k->a8_mu);
-  if (!k->cond) return cudaErrorInvalidValue;  // a key without control bits (see gmc_key_import)
-  const gmc_setinfo &S = set_info(k->set);
-  const int tm = S.t * S.m, rows_pad = round_up(tm, kGemmRowTile), kwn = ct_htt_words(S.n);
-  cudaError_t e = cudaSuccess;
-  if (!k->htt) {
-    uint32_t *p = nullptr;
-    e = cudaMalloc(&p, (size_t)rows_pad * kwn * 4);
-    if (e == cudaSuccess) e = launch_ct_htt(k->HT, k->dk.ldh, S.n, tm, p, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) {
-      cudaFree(p);
-      return e;
-    }
-    k->htt = p;
-  }
-  if (engine == GEMM_TC && !k->htt8) {
-    uint8_t *p = nullptr;
-    e = cudaMalloc(&p, tc_a8_bytes(rows_pad, kwn));
-    if (e == cudaSuccess) e = launch_expand_a(k->htt, kwn, rows_pad, kwn, p, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) {
-      cudaFree(p);
-      return e;
-    }
-    k->htt8 = p;
-  }
-  return cudaSuccess;
-}
-
-cudaError_t gmc::ct_gemm_keys(const gmc_key *const *keys, int nkeys, int engine, cudaStream_t st, GemmKeys *gk) {
-  *gk = GemmKeys{};
-  if (nkeys > 0) gk->tc_stages = tune_get(keys[0]->set).gemm_stages;
-  for (int i = 0; i < nkeys; i++) {
-    cudaError_t e = key_ct(keys[i], engine, st);
-    if (e != cudaSuccess) return e;
-    gk->A[i] = keys[i]->htt;
-    gk->A8[i] = keys[i]->htt8;
-  }
-  return cudaSuccess;
+  return ct ? std::max(S.q / 32, round_up((S.n + 31) / 32, kGemmKTile)) : tab;
 }
 
 // encapsulation kernels for the segments of one set: seeds / c / k rows in padded row space
@@ -632,7 +584,7 @@ template <int SET>
 static cudaError_t dec_front_decode_seg(const Segs &segs, const gmc_key *ref, const GemmKeys &gk, const DecKeys &dk,
                                         int engine, int *err, const uint8_t *c, uint32_t *X, uint32_t *S2,
                                         uint16_t *Sig, uint32_t *E, int *ok, const DecDims &d, cudaStream_t st,
-                                        bool pc = false, const GemmKeys *ctk = nullptr) {
+                                        bool pc = false) {
   using p = P<SET>;
   FieldDev fd;
   if (get_field(SET, &fd) != GMC_OK) return cudaErrorUnknown;
@@ -648,13 +600,11 @@ static cudaError_t dec_front_decode_seg(const Segs &segs, const gmc_key *ref, co
   e = launch_dec_bm<SET>(S2, d.lds2, fd, segs, Sig, st, tune.bm_warps, d.ct);
   if (e != cudaSuccess) return e;
   prof_mark("dec_bm", st);
-  e = launch_dec_root<SET>(Sig, S2, d.lds2, dk, fd, segs, E, d.lde, ok, st, tune.root_warps, d.ct);
+  e = launch_dec_root<SET>(Sig, dk, fd, segs, E, d.lde, ok, st, tune.root_warps, d.ct);
   prof_mark("dec_fft_roots_reenc", st);
   if (e != cudaSuccess || !d.ct) return e;
-  // constant time: the Benes network to code positions, then the dense first-t syndrome check
-  // (the packed ciphertexts in X are no longer needed: X takes the check's syndromes)
-  if (!ctk) return cudaErrorInvalidValue;
-  e = launch_dec_ct_finish<SET>(dk, *ctk, engine, segs, E, d.lde, S2, d.lds2, X, d.ldx, ok, err, st);
+  // constant time: the Benes network to code positions
+  e = launch_dec_ct_finish<SET>(dk, segs, E, d.lde, ok, st);
   prof_mark("dec_ct_positions_check", st);
   return e;
 }
@@ -669,10 +619,8 @@ static cudaError_t dec_front_decode(const gmc_key *sk, const uint8_t *c, long lo
   if (e != cudaSuccess) return e;
   DecKeys dk{};
   dk.k[0] = sk->dk;
-  GemmKeys ctk;
-  if (d.ct && (e = ct_gemm_keys(&sk, 1, engine, st, &ctk)) != cudaSuccess) return e;
   return dec_front_decode_seg<SET>(one_segment(n), sk, gk, dk, engine, err, c, X, S2, Sig, E, ok, d, st,
-                                   sk->pc != 0, d.ct ? &ctk : nullptr);
+                                   sk->pc != 0);
 }
 
 template <int SET>
@@ -1180,11 +1128,9 @@ static cudaError_t plan_pipe_kernels(gmc_plan *p, PlanPipe &pp) {
     d.lde = dec_e_words(SET, pp.const_time);
     DecKeys dk{};
     for (size_t i = 0; i < pp.groups.size(); i++) dk.k[i] = keys[i]->dk;
-    GemmKeys ctk;
-    if (d.ct) e = ct_gemm_keys(keys, (int)pp.groups.size(), pp.engine, pp.st, &ctk);
     if (e == cudaSuccess)
       e = dec_front_decode_seg<SET>(pp.segs, ref, gk, dk, pp.engine, err, pp.in, pp.w0, pp.w1, pp.sig, pp.w2, pp.ok,
-                                    d, pp.st, pp.pc != 0, d.ct ? &ctk : nullptr);
+                                    d, pp.st, pp.pc != 0);
     if (e == cudaSuccess)
       e = launch_dec_tail<SET>(pp.w2, d.lde, pp.ok, pp.in, dk, pp.k, pp.rc, pp.segs, pp.pc != 0, pp.st);
   }
@@ -1273,12 +1219,6 @@ extern "C" int gmc_plan_create(gmc_plan **out, const gmc_group *groups, int ngro
         if ((e = key_a8(p->groups[gi].key, pp.st, &a8)) != cudaSuccess) break;
       }
     if (e == cudaSuccess && pp.engine == GEMM_TC && !tc_err_word()) e = cudaErrorMemoryAllocation;
-    if (e == cudaSuccess && pp.kind == 1 && pp.const_time) {  // the constant-time check's matrices, before capture
-      const gmc_key *ks[kMaxSegs];
-      for (size_t j = 0; j < pp.groups.size(); j++) ks[j] = p->groups[pp.groups[j]].key;
-      GemmKeys ctk;
-      e = ct_gemm_keys(ks, (int)pp.groups.size(), pp.engine, pp.st, &ctk);
-    }
   }
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->cap, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming);

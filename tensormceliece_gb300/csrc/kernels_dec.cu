@@ -3,8 +3,7 @@
 //  pack_ct     ciphertext bytes -> 32-bit words (the front-end GEMM operand)
 //  decode      one warp per request: 2t syndromes (from the front-end GEMM)
 //              -> Berlekamp-Massey -> additive FFT over all 2^m field
-//              elements -> error positions at the key's support -> weight
-//              and re-encryption (syndrome) check
+//              elements -> error positions at the key's support, weight
 //  dec_tail    K = SHAKE256(b || (e or s) || c), implicit rejection, and the
 //              6960119 ciphertext-padding rule
 //
@@ -308,7 +307,7 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
     }
     // sigma(x) = sum_deg C[t-deg] x^deg -> FFT coefficient slots (deg < 2^d);
     // coefficients are < 2^m <= 2^13, so bit 15 of the constant coefficient
-    // is free for the flag of a final length L > t
+    // is free for the flag of a final length L != t
 #pragma unroll
     for (int k = 0; k < NS; k++)
 #pragma unroll
@@ -324,7 +323,7 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
 #pragma unroll
           for (int b = 0; b < M; b++) v |= ((SP[i * M + b] >> lane) & 1u) << b;
         }
-        if (deg == 0 && L > T) v |= 0x8000u;
+        if (deg == 0 && L != T) v |= 0x8000u;
         sig[deg] = (uint16_t)v;
       }
     }
@@ -657,7 +656,7 @@ __global__ void __launch_bounds__((BMCtLayout<SET>::NS + 1) * 32, kBMCtBlocksPer
 #pragma unroll
           for (int b = 0; b < M; b++) v |= ((SP[ci * M + b] >> lane) & 1u) << b;
         }
-        v |= (deg == 0 && L > T) ? 0x8000u : 0u;
+        v |= (deg == 0 && L != T) ? 0x8000u : 0u;
         wd[e >> 1] |= v << (16 * (e & 1));
       }
       sig[u] = make_uint4(wd[0], wd[1], wd[2], wd[3]);
@@ -818,14 +817,14 @@ __global__ void __launch_bounds__(kBMLatWarps * 32, 2) dec_bm_lat_kernel(const u
     static_assert(NS >= 2 && NS <= 4, "one loop per number of active slots");
     // sigma(x) = sum_deg C[t-deg] x^deg -> FFT coefficient slots (deg < 2^d);
     // coefficients are < 2^m <= 2^13, so bit 15 of the constant coefficient
-    // is free for the flag of a final length L > t
+    // is free for the flag of a final length L != t
     uint16_t *sig = Sig + op * SIG;
     for (int x = T + lane; x < SIG; x += 32) sig[x] = x == T ? 1 : 0;
 #pragma unroll
     for (int k = 0; k < NS; k++) {
       const int i = 1 + lane + 32 * k;
       const uint32_t c = gexp[min(lC[k], (uint32_t)ZL)];
-      if (i <= T) sig[T - i] = (uint16_t)(c | ((i == T && L > T) ? 0x8000u : 0u));
+      if (i <= T) sig[T - i] = (uint16_t)(c | ((i == T && L != T) ? 0x8000u : 0u));
     }
     __syncwarp();
   }
@@ -834,7 +833,7 @@ __global__ void __launch_bounds__(kBMLatWarps * 32, 2) dec_bm_lat_kernel(const u
 // ---------------------------------------------------------------- root finding
 // One warp per request: additive FFT of sigma over all 2^m field elements
 // (Gao-Mateer, basis beta_i = 2^i so point c is the element c), the error
-// positions, the weight and the re-encryption check.
+// positions and the weight.
 // The top-down part (twist + radix conversion) turns the 2^d coefficients
 // into 2^d leaf constants. Every bottom-up butterfly level has stride < 2^d,
 // so the 2^m evaluations split into 2^(m-d) independent chunks of 2^d
@@ -1004,7 +1003,6 @@ __device__ __forceinline__ uint32_t gf_mul_cols(uint32_t v, const uint16_t *cols
 // tables indexed by coefficient values are not loaded)
 template <int SET, bool CT>
 __global__ void __launch_bounds__(kRootWarps * 32, 2) dec_root_kernel(const uint16_t *__restrict__ Sig,
-                                                                   const uint32_t *__restrict__ S2, int lds2,
                                                                    const DecKeys keys, FieldDev fd, const Segs segs,
                                                                    uint32_t *__restrict__ E, int lde,
                                                                    int *__restrict__ okout) {
@@ -1058,7 +1056,7 @@ __global__ void __launch_bounds__(kRootWarps * 32, 2) dec_root_kernel(const uint
     uint32_t vv[VPL];
 #pragma unroll
     for (int j = 0; j < VPL; j++) vv[j] = sig[lane + 32 * j];
-    const bool long_lfsr = (__shfl_sync(0xffffffffu, vv[0], 0) >> 15) != 0;  // BM ended with L > t
+    const bool bad_length = (__shfl_sync(0xffffffffu, vv[0], 0) >> 15) != 0;  // BM ended with L != t
     vv[0] &= 0x7FFFu;
 #pragma unroll 1
     for (int l = 0; l < D; l++) {
@@ -1211,7 +1209,7 @@ __global__ void __launch_bounds__(kRootWarps * 32, 2) dec_root_kernel(const uint
           erow[wb | b0] = rev5_bits(e32);
         }
       }
-      if (lane == 0) okout[op] = long_lfsr ? 0 : 1;  // weight and syndromes are checked after the Benes network
+      if (lane == 0) okout[op] = bad_length ? 0 : 1;  // the weight is checked after the Benes network
       __syncwarp();
       continue;
     }
@@ -1234,62 +1232,29 @@ __global__ void __launch_bounds__(kRootWarps * 32, 2) dec_root_kernel(const uint
         if (r < nroots && pos[k] < (uint32_t)p::n) {
           weight++;
           atomicOr(&esm[pos[k] >> 5], 1u << (pos[k] & 31));
-          roots[r] |= pos[k] << 16;
         }
       }
     }
     weight = __reduce_add_sync(0xffffffffu, weight);
     __syncwarp();
 
-    // Accept when the t roots lie in the support, BM's length is <= t and the
-    // first t syndromes of the found error equal the received ones. That is
-    // the library's full 2t-syndrome check: with L <= t, the connection
-    // polynomial C (sigma reversed) annihilates the received sequence from
-    // index t on, and also the found error's sequence sum_i w2_i L_i^j (sigma
-    // vanishes at every L_i), so the two sequences agree iff their first t
-    // terms do. With L > t no error of weight <= t has these syndromes (its
-    // locator would be a shorter LFSR), so the library's check fails as well.
-    bool ok = (weight == T) && !long_lfsr;
-    if (ok) {
-      // first t syndromes of the found error: XOR of the key's columns at the
-      // t positions (then every root is in the support and in the list). Each
-      // half-warp reads whole rows, lane c of a half the 16-byte chunk c, so a
-      // load instruction covers two rows contiguously; the halves are added by
-      // one shuffle and compared with the received words.
-      constexpr int TW = (T * M + 31) / 32;
-      constexpr int TW4 = (TW + 3) / 4;
-      static_assert(TW4 <= 16, "a row of the first t syndromes fits half a warp of 16-byte chunks");
-      const int c = lane & 15;
-      uint4 acc = make_uint4(0, 0, 0, 0);
-      if (c < TW4) {
-#pragma unroll 16
-        for (int r = lane >> 4; r < T; r += 2) {
-          const uint4 v = reinterpret_cast<const uint4 *>(key.HT + (size_t)(roots[r] >> 16) * key.ldh)[c];
-          acc.x ^= v.x;
-          acc.y ^= v.y;
-          acc.z ^= v.z;
-          acc.w ^= v.w;
-        }
-      }
-      acc.x ^= __shfl_xor_sync(0xffffffffu, acc.x, 16);
-      acc.y ^= __shfl_xor_sync(0xffffffffu, acc.y, 16);
-      acc.z ^= __shfl_xor_sync(0xffffffffu, acc.z, 16);
-      acc.w ^= __shfl_xor_sync(0xffffffffu, acc.w, 16);
-      uint32_t mism = 0;
-      if (lane < TW4) {
-        const uint32_t *srow = S2 + op * lds2;
-        const uint32_t q4[4] = {acc.x, acc.y, acc.z, acc.w};
-#pragma unroll
-        for (int e2 = 0; e2 < 4; e2++) {
-          const int word = 4 * lane + e2;
-          if (word < TW) {
-            const uint32_t msk = (word == TW - 1 && (T * M) % 32) ? ((1u << ((T * M) % 32)) - 1u) : 0xFFFFFFFFu;
-            mism |= (q4[e2] ^ srow[word]) & msk;
-          }
-        }
-      }
-      ok = !__any_sync(0xffffffffu, mism != 0);
-    }
+    // Accept when BM's length L is t and sigma's roots are t support elements.
+    // The library compares the 2t syndromes of the found error with the received
+    // ones as well; that comparison cannot fail then (and for L != t no error of
+    // weight t has these syndromes, whose complexity would be t):
+    // - The received word is binary: its syndromes are those of f' / f mod g^2, f
+    //   the product of x - L_i over its ones. With f = f0^2 + x f1^2 and s = a^2 +
+    //   x b^2, (s f)' = (a f1 + b f0)^2 in characteristic 2, so (s f)' = 0 mod g^2 iff
+    //   a f1 + b f0 = 0 mod g: t linear equations for the t + 1 coefficients of an s
+    //   of degree <= t. Some s != 0 solves them, and s f' / f = s' mod g^2.
+    // - L = t and distinct roots L_1 .. L_t of sigma: the syndromes are
+    //   sum_i c_i w2_i L_i^j with no c_i = 0 (else L < t), i.e. f' / f = w / sigma mod
+    //   g^2 with w coprime to sigma, deg w < t. So s w = s' sigma mod g^2, and exactly,
+    //   as both have degree < 2t: sigma divides s, s = k sigma, w = sigma' and every
+    //   c_i is 1, which is the found error's sequence.
+    // Reading the key's syndromes at the t positions for the comparison took 82 of
+    // 1062 us (8192128, 65536 requests; 27 KB per request from L2).
+    const bool ok = (weight == T) && !bad_length;
     uint32_t *erow = E + op * lde;
     for (int it = lane; it < NW; it += 32) erow[it] = esm[it];
     if (lane == 0) okout[op] = ok ? 1 : 0;
@@ -1476,7 +1441,7 @@ cudaError_t launch_dec_bm(const uint32_t *S2, int lds2, FieldDev fd, const Segs 
 }
 
 template <int SET, bool CT>
-static cudaError_t launch_dec_root_form(const uint16_t *Sig, const uint32_t *S2, int lds2, const DecKeys &keys,
+static cudaError_t launch_dec_root_form(const uint16_t *Sig, const DecKeys &keys,
                                         FieldDev fd, const Segs &segs, uint32_t *E, int lde, int *ok,
                                         cudaStream_t st, int warps) {
   const long long N = seg_rows(segs);
@@ -1485,11 +1450,11 @@ static cudaError_t launch_dec_root_form(const uint16_t *Sig, const uint32_t *S2,
                                          RootLayout<SET, CT>::bytes(kRootWarps));
   if (err != cudaSuccess) return err;
   const int gr = persistent_blocks(dec_root_kernel<SET, CT>, warps * 32, smem_rt, N, warps);
-  return launch_chained(segs, dec_root_kernel<SET, CT>, gr, warps * 32, smem_rt, st, Sig, S2, lds2, keys, fd, segs, E, lde, ok);
+  return launch_chained(segs, dec_root_kernel<SET, CT>, gr, warps * 32, smem_rt, st, Sig, keys, fd, segs, E, lde, ok);
 }
 
 template <int SET>
-cudaError_t launch_dec_root(const uint16_t *Sig, const uint32_t *S2, int lds2, const DecKeys &keys, FieldDev fd,
+cudaError_t launch_dec_root(const uint16_t *Sig, const DecKeys &keys, FieldDev fd,
                             const Segs &segs, uint32_t *E, int lde, int *ok, cudaStream_t st, int warps, bool ct) {
   const long long N = seg_rows(segs);
   if (N <= 0) return cudaSuccess;
@@ -1497,12 +1462,12 @@ cudaError_t launch_dec_root(const uint16_t *Sig, const uint32_t *S2, int lds2, c
   if (warps == 0) warps = kRootWarps;
   if (ct) {
     if (!fd.fft_twist_cols) return cudaErrorInvalidValue;
-    return launch_dec_root_form<SET, true>(Sig, S2, lds2, keys, fd, segs, E, lde, ok, st, warps);
+    return launch_dec_root_form<SET, true>(Sig, keys, fd, segs, E, lde, ok, st, warps);
   }
-  return launch_dec_root_form<SET, false>(Sig, S2, lds2, keys, fd, segs, E, lde, ok, st, warps);
+  return launch_dec_root_form<SET, false>(Sig, keys, fd, segs, E, lde, ok, st, warps);
 }
 
-// ---------------------------------------------------------------- constant-time positions and check
+// ---------------------------------------------------------------- constant-time positions
 // The key's Benes network (its sk control bits, 2m - 1 layers of conditional
 // swaps with strides 2^0 .. 2^(m-1) .. 2^0) applied to the field-order error
 // vector y (y[v] = e at field element bitrev_m(v)) gives x[i] = y[pi(i)] with
@@ -1511,6 +1476,8 @@ cudaError_t launch_dec_root(const uint16_t *Sig, const uint32_t *S2, int lds2, c
 // request, the q-bit vector in registers (word w = lane + 32 r); every layer
 // touches every word with the control words as masks, so nothing depends on the
 // error's positions. Then: bits >= n cleared, weight == t folded into ok.
+// (The dense product that compared the found error's syndromes, which cannot
+// differ, took 107 of the 150 us of this stage: 8192128, 8192 requests.)
 // a layer whose pairs are registers r and r + DR of one lane (stride 2^s, s >= 10)
 template <int WPL, int DR>
 __device__ __forceinline__ void benes_reg_layer(uint32_t (&x)[WPL], const uint32_t *cw, int lane, int s) {
@@ -1597,70 +1564,19 @@ __global__ void __launch_bounds__(256) benes_ct_kernel(uint32_t *__restrict__ E,
   }
 }
 
-// ok &= (first t syndromes of the decoded error == the received ones): S3 from
-// the dense product with the key's first-t syndrome matrix, S2 the received 2t
-// syndromes (same packing, m bits each). Thread per request, every word.
 template <int SET>
-__global__ void ct_check_kernel(const uint32_t *__restrict__ S3, int lds3, const uint32_t *__restrict__ S2, int lds2,
-                                int *__restrict__ okio, const Segs segs) {
-  using p = P<SET>;
-  constexpr int TM = p::t * p::m, TW = (TM + 31) / 32;
-  chain_trigger();
-  chain_wait();
-  const long long op = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  int seg;
-  if (op >= seg_rows(segs) || !seg_live(segs, op, &seg)) return;
-  uint32_t mism = 0;
-#pragma unroll 4
-  for (int w = 0; w < TW; w++) {
-    const uint32_t msk = (w == TW - 1 && (TM % 32)) ? ((1u << (TM % 32)) - 1u) : 0xFFFFFFFFu;
-    mism |= (S3[op * lds3 + w] ^ S2[op * lds2 + w]) & msk;
-  }
-  okio[op] = okio[op] & (mism == 0 ? 1 : 0);
-}
-
-template <int SET>
-cudaError_t launch_dec_ct_finish(const DecKeys &keys, const GemmKeys &htt, int engine, const Segs &segs, uint32_t *E,
-                                 int lde, const uint32_t *S2, int lds2, uint32_t *S3, int lds3, int *ok, int *err,
+cudaError_t launch_dec_ct_finish(const DecKeys &keys, const Segs &segs, uint32_t *E, int lde, int *ok,
                                  cudaStream_t st) {
   using p = P<SET>;
   const long long N = seg_rows(segs);
   if (N <= 0) return cudaSuccess;
-  if (lde < p::q / 32 || lde < ct_htt_words(p::n)) return cudaErrorInvalidValue;
+  if (lde < p::q / 32) return cudaErrorInvalidValue;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long want = (N + 7) / 8;
   const int blocks = (int)(want < 8LL * sms ? want : 8LL * sms);
-  cudaError_t e = launch_chained(segs, benes_ct_kernel<SET>, blocks, 256, 0, st, E, lde, ok, keys, segs);
-  if (e != cudaSuccess) return e;
-  e = launch_gf2_gemm_seg(engine, htt, segs, ct_htt_words(p::n), (p::t * p::m + kGemmRowTile - 1) / kGemmRowTile *
-                          kGemmRowTile, E, lde, ct_htt_words(p::n), S3, lds3, (p::t * p::m + 31) / 32, err, st);
-  if (e != cudaSuccess) return e;
-  return launch_chained(segs, ct_check_kernel<SET>, (unsigned)((N + 127) / 128), 128, 0, st, S3, lds3, S2, lds2, ok, segs);
-}
-
-// HTT[r][w] bit b = bit r of HT[32 w + b] (r < t m, 32 w + b < n): the first t syndromes of every code position
-// as a (t m) x n GF(2) matrix, rows_pad x kwn words
-__global__ void ct_htt_kernel(const uint32_t *__restrict__ HT, int ldh, int n, int tm, int rows_pad, int kwn,
-                              uint32_t *__restrict__ HTT) {
-  const long long item = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (item >= (long long)rows_pad * kwn) return;
-  const int r = (int)(item / kwn), w = (int)(item % kwn);
-  uint32_t v = 0;
-  if (r < tm)
-    for (int b = 0; b < 32; b++) {
-      const int i = 32 * w + b;
-      if (i < n) v |= ((HT[(size_t)i * ldh + (r >> 5)] >> (r & 31)) & 1u) << b;
-    }
-  HTT[item] = v;
-}
-
-cudaError_t launch_ct_htt(const uint32_t *HT, int ldh, int n, int tm, uint32_t *HTT, cudaStream_t st) {
-  const int rows_pad = (tm + kGemmRowTile - 1) / kGemmRowTile * kGemmRowTile, kwn = ct_htt_words(n);
-  const long long total = (long long)rows_pad * kwn;
-  ct_htt_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(HT, ldh, n, tm, rows_pad, kwn, HTT);
-  return cudaGetLastError();
+  return launch_chained(segs, benes_ct_kernel<SET>, blocks, 256, 0, st, E, lde, ok, keys, segs);
 }
 
 template <int SET>
@@ -1683,12 +1599,11 @@ cudaError_t launch_dec_tail(const uint32_t *E, int lde, const int *ok, const uin
   template cudaError_t launch_pack_ct<SET>(const uint8_t *, const Segs &, uint32_t *, int, bool, cudaStream_t);       \
   template cudaError_t launch_dec_bm<SET>(const uint32_t *, int, FieldDev, const Segs &, uint16_t *,             \
                                          cudaStream_t, int, bool);                                               \
-  template cudaError_t launch_dec_root<SET>(const uint16_t *, const uint32_t *, int, const DecKeys &, FieldDev,  \
-                                            const Segs &, uint32_t *, int, int *, cudaStream_t, int, bool);      \
+  template cudaError_t launch_dec_root<SET>(const uint16_t *, const DecKeys &, FieldDev, const Segs &,          \
+                                            uint32_t *, int, int *, cudaStream_t, int, bool);      \
   template cudaError_t launch_dec_tail<SET>(const uint32_t *, int, const int *, const uint8_t *, const DecKeys &, \
                                             uint8_t *, int *, const Segs &, bool, cudaStream_t);                 \
-  template cudaError_t launch_dec_ct_finish<SET>(const DecKeys &, const GemmKeys &, int, const Segs &, uint32_t *, \
-                                                 int, const uint32_t *, int, uint32_t *, int, int *, int *,      \
+  template cudaError_t launch_dec_ct_finish<SET>(const DecKeys &, const Segs &, uint32_t *, int, int *,            \
                                                  cudaStream_t);
 GMC_INST_DEC(0)
 GMC_INST_DEC(1)

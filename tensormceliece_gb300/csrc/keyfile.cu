@@ -176,7 +176,7 @@ extern "C" long long gmc_key_export(const gmc_key *key, unsigned char *buf, long
   h.variant = key->variant;
   h.kind = key->kind;
   h.lda = key->lda; h.rows_pad = key->rows_pad; h.kw_pad = key->kw_pad; h.pad_bad = key->pad_bad; h.ldtt = key->ldtt;
-  h.ldf = key->ldf; h.frows_pad = key->frows_pad; h.cw_pad = key->cw_pad; h.ldh = key->dk.ldh;
+  h.ldf = key->ldf; h.frows_pad = key->frows_pad; h.cw_pad = key->cw_pad; h.ldh = key->ldh;
   if (!section_sizes(h, h.section)) return kf_fail(GMC_EKEY, "gmc_key_export: key dimensions out of range");
   const long long total = (long long)sizeof(KeyHeader) +
                           (long long)(h.section[0] + h.section[1] + h.section[2] + h.section[3] + h.section[4]);
@@ -267,8 +267,7 @@ extern "C" int gmc_key_import(gmc_key **out, const unsigned char *buf, long long
     k->dk.LW2 = k->tabs + 2 * n;
     k->dk.invL = k->tabs + 3 * n;
     k->dk.s = k->s;
-    k->dk.HT = k->HT;
-    k->dk.ldh = h.ldh;
+    k->ldh = h.ldh;
     k->dk.cond = k->cond;
   }
   *out = k;

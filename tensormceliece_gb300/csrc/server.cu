@@ -290,14 +290,8 @@ cudaError_t run_pipe(Slot &sl, Pipe &pp, cudaStream_t pst) {
     e = launch_gf2_gemm_seg(engine, gk, pp.segs, ref->ldf, ref->frows_pad, X, cw, ref->cw_pad, S2, s2, p::s2w,
                             tc_err_word_ptr(), pst);
   if (e == cudaSuccess) e = launch_dec_bm<SET>(S2, s2, fd, pp.segs, Sig, pst, tune.bm_warps, ct);
-  if (e == cudaSuccess) e = launch_dec_root<SET>(Sig, S2, s2, dk, fd, pp.segs, E, ewd, ok, pst, tune.root_warps, ct);
-  if (e == cudaSuccess && ct) {
-    // the keys' first-t syndrome matrices are built on a key's first constant-time batch
-    GemmKeys ctk;
-    e = ct_gemm_keys(pp.keys.data(), (int)pp.keys.size(), engine, pst, &ctk);
-    if (e == cudaSuccess)
-      e = launch_dec_ct_finish<SET>(dk, ctk, engine, pp.segs, E, ewd, S2, s2, X, cw, ok, tc_err_word_ptr(), pst);
-  }
+  if (e == cudaSuccess) e = launch_dec_root<SET>(Sig, dk, fd, pp.segs, E, ewd, ok, pst, tune.root_warps, ct);
+  if (e == cudaSuccess && ct) e = launch_dec_ct_finish<SET>(dk, pp.segs, E, ewd, ok, pst);
   if (e == cudaSuccess)
     e = launch_dec_tail<SET>(E, ewd, ok, in, dk, kout, (int *)(sl.dev + pp.rc_off), pp.segs, pp.pc != 0, pst);
   return e;
