@@ -169,7 +169,8 @@ static int get_field(int set, FieldDev *out) {
   };
   const size_t o_exp = put(F.exp), o_log = put(F.log), o_twist = put(ft.twist_log), o_frlo = put(ft.frob_lo),
                o_abs = put(ft.alpha_bs), o_fhbs = put(ft.frob_hi_bs), o_zech = put(ft.zech),
-               o_tcols = put(ft.twist_cols);
+               o_tcols = put(ft.twist_cols), o_alpha = put(ft.alpha), o_lleaf = put(ft.lead_leaf),
+               o_lchunk = put(ft.lead_chunk);
   FieldEntry e;
   GMC_CUDA(cudaMalloc(&e.buf, all.size() * 2));
   GMC_CUDA(cudaMemcpy(e.buf, all.data(), all.size() * 2, cudaMemcpyHostToDevice));
@@ -181,6 +182,9 @@ static int get_field(int set, FieldDev *out) {
   e.fd.frob_hi_bs = reinterpret_cast<const uint32_t *>(e.buf + o_fhbs);
   e.fd.zech = e.buf + o_zech;
   e.fd.fft_twist_cols = e.buf + o_tcols;
+  e.fd.fft_alpha = e.buf + o_alpha;
+  e.fd.lead_leaf = e.buf + o_lleaf;
+  e.fd.lead_chunk = e.buf + o_lchunk;
   g_fields[key] = e;
   *out = e.fd;
   return GMC_OK;
@@ -427,7 +431,7 @@ static cudaStream_t host_call_stream() {
 struct Scratch {
   cudaStream_t st;
   void *base = nullptr;
-  size_t bytes = 0;
+  size_t bytes = 0, optional = 0;
   std::vector<std::pair<void **, size_t>> parts;
   explicit Scratch(cudaStream_t s) : st(s) {
     keep_pool_warm();
@@ -438,8 +442,20 @@ struct Scratch {
     parts.emplace_back(reinterpret_cast<void **>(p), bytes);
     bytes += (n + 255) / 256 * 256;
   }
+  // a part the caller can do without, wanted last; its pointer stays null when it does not fit
+  template <typename T>
+  void want_optional(T **p, size_t n) {
+    optional = bytes;
+    if (n) want(p, n);
+  }
   cudaError_t get() {
     cudaError_t e = cudaMallocAsync(&base, bytes ? bytes : 256, st);
+    if (e == cudaErrorMemoryAllocation && optional && optional < bytes) {
+      cudaGetLastError();
+      bytes = optional;
+      parts.pop_back();
+      e = cudaMallocAsync(&base, bytes, st);
+    }
     if (e != cudaSuccess) {
       base = nullptr;
       return e;
@@ -566,6 +582,7 @@ struct DecDims {
   int ldx, lds2, lde;
   long long n_pad;
   bool ct;  // constant-time kernels (the switch as read once for this batch)
+  uint8_t *root_work = nullptr;  // dec_root_work_bytes of scratch, where the caller has it
 };
 static DecDims dec_dims(int set, int cw_pad, long long rows) {
   const gmc_setinfo &S = set_info(set);
@@ -600,7 +617,7 @@ static cudaError_t dec_front_decode_seg(const Segs &segs, const gmc_key *ref, co
   e = launch_dec_bm<SET>(S2, d.lds2, fd, segs, Sig, st, tune.bm_warps, d.ct);
   if (e != cudaSuccess) return e;
   prof_mark("dec_bm", st);
-  e = launch_dec_root<SET>(Sig, dk, fd, segs, E, d.lde, ok, st, tune.root_warps, d.ct);
+  e = launch_dec_root<SET>(Sig, dk, fd, segs, E, d.lde, ok, st, tune.root_warps, d.ct, d.root_work);
   prof_mark("dec_fft_roots_reenc", st);
   if (e != cudaSuccess || !d.ct) return e;
   // constant time: the Benes network to code positions
@@ -636,6 +653,7 @@ static cudaError_t dec_run(const gmc_key *sk, uint8_t *k, const uint8_t *c, long
   scr.want(&Sig, (size_t)d.n_pad * (2u << P<SET>::fft_d));
   scr.want(&E, (size_t)d.n_pad * d.lde * 4);
   scr.want(&ok, (size_t)d.n_pad * 4);
+  scr.want_optional(&d.root_work, dec_root_work_bytes(SET, d.n_pad, d.ct));
   if ((e = scr.get()) != cudaSuccess) return e;
   if ((e = dec_front_decode<SET>(sk, c, n, X, S2, Sig, E, ok, d, st)) != cudaSuccess) return e;
   DecKeys dk{};
@@ -816,6 +834,7 @@ extern "C" int gmc_dec_stages_dev(const gmc_key *sk, const unsigned char *c, lon
     uint16_t *Sig = nullptr;
     scr.want(&X, (size_t)d.n_pad * d.ldx * 4);
     scr.want(&Sig, (size_t)d.n_pad * 256);
+    scr.want_optional(&d.root_work, dec_root_work_bytes(sk->set, d.n_pad, d.ct));
     e = scr.get();
     if (e == cudaSuccess) GMC_DISPATCH(sk->set, e = dec_front_decode<S_>(sk, c, n, X, synd, Sig, ev, ok, d, st));
     // (dec_front_decode packs C0 at the key's ciphertext stride: pc keys take C0 || C1 rows)
@@ -1075,6 +1094,7 @@ struct PlanPipe {
   int *rc = nullptr;
   uint32_t *w0 = nullptr, *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;  // intermediates
   uint16_t *sig = nullptr;
+  uint8_t *root_work = nullptr;
   int *ok = nullptr;
   cudaStream_t st = nullptr;
   cudaEvent_t done = nullptr;
@@ -1126,6 +1146,7 @@ static cudaError_t plan_pipe_kernels(gmc_plan *p, PlanPipe &pp) {
     DecDims d = dec_dims(SET, ref->cw_pad, rows);
     d.ct = pp.const_time;  // the buffers were laid out for the form chosen at creation
     d.lde = dec_e_words(SET, pp.const_time);
+    d.root_work = pp.root_work;
     DecKeys dk{};
     for (size_t i = 0; i < pp.groups.size(); i++) dk.k[i] = keys[i]->dk;
     if (e == cudaSuccess)
@@ -1219,6 +1240,13 @@ extern "C" int gmc_plan_create(gmc_plan **out, const gmc_group *groups, int ngro
         if ((e = key_a8(p->groups[gi].key, pp.st, &a8)) != cudaSuccess) break;
       }
     if (e == cudaSuccess && pp.engine == GEMM_TC && !tc_err_word()) e = cudaErrorMemoryAllocation;
+  }
+  for (auto &pp : p->pipes) {  // after everything a plan needs: without it a pipeline takes the other root finder
+    const size_t rw = pp.kind == 1 ? dec_root_work_bytes(pp.set, seg_rows(pp.segs), pp.const_time) : 0;
+    if (e == cudaSuccess && rw && plan_alloc(p, (void **)&pp.root_work, rw) != cudaSuccess) {
+      cudaGetLastError();
+      pp.root_work = nullptr;
+    }
   }
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->cap, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming);

@@ -165,6 +165,32 @@ FftTables build_fft_tables(int m, int d) {
   t.zech[0] = (uint16_t)(3 << m);
   for (int k = 1; k < (1 << m) - 1; k++) t.zech[k] = F.log[1 ^ F.exp[k]];
 
+  // request-sliced form. On the chunk of base a, x^(2^d) = P(x) + K(a) with P the polynomial of degree < 2^d that
+  // agrees with it on chunk 0: x^(2^d) - P(x) is a multiple of the vanishing polynomial of chunk 0's subspace, which is
+  // constant on every chunk. P's leaves come from its values on chunk 0 by the inverse butterflies.
+  t.alpha.resize(1 << m);
+  for (int i = 0; i < (1 << m); i++) t.alpha[i] = F.exp[t.alpha_log[i]];
+  {
+    const int n = 1 << d, chunks = 1 << (m - d);
+    auto off = [&](int l) { return (1 << m) - (1 << (m - l)); };
+    std::vector<uint16_t> f(t.frob_lo);
+    for (int l = 0; l < d; l++)
+      for (int x = 0; x < n; x++)
+        if (!((x >> l) & 1)) {
+          uint16_t &lo = f[x], &hi = f[x + (1 << l)];
+          hi ^= lo;
+          lo ^= F.mul(t.alpha[off(l) + (x >> (l + 1))], hi);
+        }
+    t.lead_leaf = f;
+    t.lead_chunk.resize(chunks);
+    for (int c = 0; c < chunks; c++) {
+      std::vector<uint16_t> v(f);
+      for (int l = d - 1; l >= 0; l--)  // the point c 2^d: slot 0's value
+        for (int x = 0; x < (1 << l); x++) v[x] ^= F.mul(t.alpha[off(l) + (c << (d - 1 - l))], v[x + (1 << l)]);
+      t.lead_chunk[c] = (uint16_t)(t.frob_hi[c] ^ v[0]);
+    }
+  }
+
   // bit-sliced forms: 32 chunks per word
   const int H = (1 << (m - d)) / 32;
   auto put_word = [](std::vector<uint16_t> &v, size_t w, uint32_t x) {

@@ -40,6 +40,11 @@ struct FftTables {
   //   frob_hi_bs[h * m + b]: frob_hi[c]
   std::vector<uint16_t> alpha_bs;
   std::vector<uint16_t> frob_hi_bs;
+  // request-sliced root finding: the butterfly constants as values, alpha[2^m - 2^(m-l) + c] for level l, and the
+  // x^(2^d) term (sets with t = 2^d): what it adds to every leaf, and to leaf 0 of chunk c
+  std::vector<uint16_t> alpha;
+  std::vector<uint16_t> lead_leaf;
+  std::vector<uint16_t> lead_chunk;
   // Zech logarithms: zech[k] = log(1 + g^k) for 0 < k < q-1; zech[0] (1 + 1 = 0)
   // is 3q, a log at or above the zero sentinel 2q-2 that stays below 2^16
   // after adding any log < q-1 and reducing once by q-1.

@@ -20,6 +20,10 @@ constexpr int kBMCtBlocksPerSM = 3;  // its constant-time form: blocks (groups o
 constexpr int kBMLatWarps = 24;  // Berlekamp-Massey latency form: largest warps per block (one request per warp)
 constexpr int kBMLatCopyWarps = 8;  // its smallest block: warps without a request help to copy the tables
 constexpr long long kBMBitslicedMinRows = 24576;  // smaller batches take the latency form
+// Root finding: smaller batches take the warp-per-request form. us, request-sliced / warp per request: 12288 rows
+// 205 / 205 (8192128), 201 / 201 (6960119), 95 / 90 (348864); 14336 rows 205 / 226, 202 / 222, 96 / 98; 65536 rows
+// 793 / 980, 778 / 970, 343 / 407.
+constexpr long long kRootSlicedMinRows = 14000;
 constexpr int kRootWarps = 8;  // root-finding kernel: default and largest warps per block
 
 // ---------------------------------------------------------------- segments
@@ -199,6 +203,9 @@ struct FieldDev {
   const uint32_t *fft_alpha_bs;   // [2^d - 2^(d-l) + xh][alpha_bs_stride(H m)], entry h m + b: alpha_{l, (c << (d-1-l)) + xh}
   const uint32_t *frob_hi_bs;     // [h][m]: (c 2^d)^(2^d)
   const uint16_t *zech;           // [q]: log(1 + g^k), zech[0] = 3q (zero)
+  // request-sliced root finding (null where not built): butterfly constants [q], level l from q - (q >> l); the x^t
+  // term's leaves [2^d] and per-chunk constants
+  const uint16_t *fft_alpha = nullptr, *lead_leaf = nullptr, *lead_chunk = nullptr;
   // [2^(d+1)][m]: for the twist constant c of each fft_twist_log entry, c x^i (i < m), so a product
   // with c needs no table indexed by the other factor (constant-time form); null where not built
   const uint16_t *fft_twist_cols = nullptr;
@@ -228,7 +235,11 @@ cudaError_t launch_dec_bm(const uint32_t *S2, int lds2, FieldDev fd, const Segs 
 // ct: the twist multiplies by table-free columns (needs fd.fft_twist_cols).
 template <int SET>
 cudaError_t launch_dec_root(const uint16_t *Sig, const DecKeys &keys, FieldDev fd, const Segs &segs, uint32_t *E,
-                            int lde, int *ok, cudaStream_t st, int warps = 0, bool ct = false);
+                            int lde, int *ok, cudaStream_t st, int warps = 0, bool ct = false,
+                            uint8_t *work = nullptr);
+// work (16-byte aligned): scratch of the request-sliced form for batches of `rows` padded rows; 0 bytes (or a null
+// pointer): the warp-per-request form
+size_t dec_root_work_bytes(int set, long long rows, bool ct);
 // Constant-time decapsulation, after launch_dec_root(ct = true) left the field-order error vectors in E and the
 // BM-length flag in ok: the key's Benes network to code order (E in place), weight == t into ok. E rows: lde >= q/32.
 template <int SET>

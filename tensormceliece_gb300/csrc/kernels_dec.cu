@@ -15,6 +15,7 @@
 // decoder yields the same session key. The BM update rule follows the
 // library's (mc:crypto_kem/348864/vec/bm.c:156), so locators agree with the
 // oracle's stage output as well.
+#include <algorithm>
 #include <type_traits>
 
 #include "kernels.h"
@@ -1262,6 +1263,375 @@ __global__ void __launch_bounds__(kRootWarps * 32, 2) dec_root_kernel(const uint
   }
 }
 
+// ---------------------------------------------------------------- root finding, request-sliced form
+// For large batches. dec_root_kernel slices over the 32 chunks of one request,
+// so every butterfly constant is a different element in every bit of a word
+// and lane and a product costs m^2 AND-XOR steps and the reduction (about 200
+// instructions). Here a word holds one plane of 32 requests and the lanes hold
+// 16 such groups (and two slots with the same constant), so a butterfly's
+// constant is one scalar for the whole warp and its product is a sum of shifted
+// planes: kSlicedWindow bits of the constant at a time select one of 8 sums by
+// branch, 62 XORs on average, 27 more for the reduction.
+// Three kernels: dec_leaf (top-down pass, eight groups per block), dec_fft (the
+// bottom-up butterflies of one chunk of 512 requests at a time in shared memory;
+// zero masks out) and dec_pos (zero masks to error vectors in code order, weight).
+// The x^t term of the sets with t = 2^d is folded into the leaves and one
+// constant per chunk (build_fft_tables).
+// 8192128, 65536 requests: 793 us against 980 us for dec_root_kernel; of 32768,
+// dec_fft takes 360 us (221 M warp instructions, 54% of them XORs, the rest
+// branches, moves and shared memory; 2.1 issued per cycle and SM, where its 16
+// warps wait for branch targets), dec_leaf 45 and dec_pos 31. Windows of 2 bits:
+// dec_fft 369 us. Selected sums instead of branches (what the compiler makes of
+// if chains): 481. The product's code once per butterfly, 14 times: 383, waiting
+// for instructions a third of the time.
+constexpr int kSlicedWindow = 3;
+
+template <int SET>
+struct SlicedLayout {
+  using p = P<SET>;
+  static constexpr int D = p::fft_d, M = p::m, POS = 1 << D, CHUNKS = p::q >> D;
+  static constexpr int GPS = 16;                    // groups of 32 requests per tile
+  static constexpr int tile_words = POS * M * GPS;  // [slot][plane][group]
+  static constexpr int LGPS = 8;                    // groups per block of dec_leaf
+  static constexpr int leaf_bytes = POS * M * LGPS * 4;
+  static constexpr int leaf_threads = 1024;
+  static constexpr int off(int l) { return p::q - (p::q >> l); }  // butterfly constants of level l
+  static_assert(D >= 6 && D <= 7 && CHUNKS == 64 && GPS % LGPS == 0 && LGPS % 4 == 0, "pass geometry");
+};
+
+// acc[w ..] += b V, V the value of a window of W bits of a constant
+template <int M, int W, int NB, int V>
+__device__ __forceinline__ void sliced_add(uint32_t (&acc)[NB][2 * M - 1], uint32_t (*const (&b)[NB])[M], int w) {
+#pragma unroll
+  for (int i = 0; i < NB; i++)
+#pragma unroll
+    for (int k = 0; k < M + W - 1; k++) {
+      uint32_t x = 0;
+#pragma unroll
+      for (int j = 0; j < W; j++)
+        if ((V >> j & 1) && k - j >= 0 && k - j < M) x ^= (*b[i])[k - j];
+      if (w + k < 2 * M - 1) {
+        acc[i][w + k] ^= x;
+        asm volatile("" : "+r"(acc[i][w + k]));  // stays in its branch (sunk below it: a move per branch)
+      }
+    }
+}
+
+// the same for a window f that is the same in the whole warp
+template <int M, int W, int NB>
+__device__ __forceinline__ void sliced_window(uint32_t (&acc)[NB][2 * M - 1], uint32_t (*const (&b)[NB])[M],
+                                              int w, uint32_t f) {
+  switch (f & ((1u << W) - 1)) {
+    case 0: asm volatile(""); break;
+    case 1: sliced_add<M, W, NB, 1>(acc, b, w); break;
+    case 2: sliced_add<M, W, NB, 2>(acc, b, w); break;
+    case 3: sliced_add<M, W, NB, 3>(acc, b, w); break;
+    case 4: sliced_add<M, W, NB, 4>(acc, b, w); break;
+    case 5: sliced_add<M, W, NB, 5>(acc, b, w); break;
+    case 6: sliced_add<M, W, NB, 6>(acc, b, w); break;
+    case 7: sliced_add<M, W, NB, 7>(acc, b, w); break;
+    default: break;
+  }
+}
+
+// acc += b c for NB elements and one constant
+template <int M, int NB>
+__device__ __forceinline__ void sliced_mul(uint32_t (&acc)[NB][2 * M - 1], uint32_t (*const (&b)[NB])[M], uint32_t c) {
+  constexpr int W = kSlicedWindow;
+#pragma unroll
+  for (int w = 0; w + W <= M; w += W) sliced_window<M, W, NB>(acc, b, w, (c >> w) & ((1u << W) - 1));
+  if (M % W) sliced_window<M, M % W ? M % W : 1, NB>(acc, b, M - M % W, c >> (M - M % W));
+}
+
+// NB butterflies with one constant: lo <- lo + c hi, hi <- lo + hi
+template <int M, int NB>
+__device__ __forceinline__ void sliced_butterflies(uint32_t (*const (&lo)[NB])[M], uint32_t (*const (&hi)[NB])[M],
+                                                   uint32_t c) {
+  uint32_t acc[NB][2 * M - 1];
+#pragma unroll
+  for (int i = 0; i < NB; i++)
+#pragma unroll
+    for (int k = 0; k < 2 * M - 1; k++) acc[i][k] = k < M ? (*lo[i])[k] : 0u;
+  sliced_mul<M, NB>(acc, hi, c);
+#pragma unroll
+  for (int i = 0; i < NB; i++) {
+    bs_reduce<M>(*lo[i], acc[i]);
+#pragma unroll
+    for (int k = 0; k < M; k++) (*hi[i])[k] ^= (*lo[i])[k];
+  }
+}
+
+// Block per LGPS groups of a tile: the coefficients transposed into planes in
+// shared memory, then level by level (twist, radix conversions) in place.
+template <int SET>
+__global__ void __launch_bounds__(SlicedLayout<SET>::leaf_threads, 1024 / SlicedLayout<SET>::leaf_threads) dec_leaf_kernel(const uint16_t *__restrict__ Sig, FieldDev fd, const Segs segs,
+                                                          uint32_t *__restrict__ Lf, int *__restrict__ okout) {
+  using p = P<SET>;
+  using LY = SlicedLayout<SET>;
+  constexpr int M = p::m, D = LY::D, POS = LY::POS, G = LY::LGPS, THREADS = LY::leaf_threads, WARPS = THREADS / 32;
+  extern __shared__ __align__(16) uint32_t tile[];  // [slot][plane][group]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long grp0 = (long long)blockIdx.x * G;
+  // units of four coefficients
+  for (int hu = warp; hu < POS / 4; hu += WARPS) {
+    const int u = hu >> 1, half = hu & 1;
+    {  // lane b of half e: plane b of coefficient 8 u + 4 half + 2 k + e
+      uint32_t x[2][G];
+#pragma unroll
+      for (int g = 0; g < G; g++) {
+        const long long op = 32 * (grp0 + g) + lane;
+        int seg;
+        const bool live = op < seg_rows(segs) && seg_live(segs, op, &seg);
+        const uint2 c = live ? reinterpret_cast<const uint2 *>(Sig + op * POS)[2 * u + half] : make_uint2(0, 0);
+        if (u == 0 && half == 0 && live) okout[op] = (c.x & 0x8000u) ? 0 : 1;  // BM ended with L != t
+        x[0][g] = transpose32(c.x, lane);
+        x[1][g] = transpose32(c.y, lane);
+      }
+      const int b = lane & 15;
+      if (b < M) {
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          uint4 *dst = reinterpret_cast<uint4 *>(tile + ((8 * u + 4 * half + 2 * k + (lane >> 4)) * M + b) * G);
+#pragma unroll
+          for (int g = 0; g < G; g += 4) dst[g / 4] = make_uint4(x[k][g], x[k][g + 1], x[k][g + 2], x[k][g + 3]);
+        }
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int l = 0; l < D; l++) {
+    if (l) {
+      // slot i times twist[i >> l]: the slots of a warp share the constant (two at l = 1, then 32 / G)
+      const uint16_t *tw = fd.fft_twist_log + (2 << D) - (2 << (D - l));
+      const int per = l == 1 ? 2 : 32 / G, e = lane / G;
+#pragma unroll 1
+      for (int i = warp * per; i < POS; i += WARPS * per) {
+        const uint32_t c = __reduce_or_sync(0xffffffffu, fd.gexp[tw[i >> l]]);
+        if (e < per) {
+          uint32_t *w = tile + (i + e) * (M * G) + lane % G;
+          uint32_t v[M], acc[1][2 * M - 1];
+#pragma unroll
+          for (int k = 0; k < 2 * M - 1; k++) acc[0][k] = 0;
+#pragma unroll
+          for (int k = 0; k < M; k++) v[k] = w[k * G];
+          sliced_mul<M, 1>(acc, {&v}, c);
+          bs_reduce<M>(v, acc[0]);
+#pragma unroll
+          for (int k = 0; k < M; k++) w[k * G] = v[k];
+        }
+      }
+      __syncthreads();
+    }
+#pragma unroll 1
+    for (int pb = D - 2; pb >= l; pb--) {
+      // quarters of every block of 4 2^pb slots: a2 += a3, a1 += a2
+      const int s = 1 << pb;
+      for (int t = threadIdx.x; t < POS / 4 * (M * G); t += THREADS) {
+        const int q = t / (M * G), i = ((q >> pb) << (pb + 2)) | (q & (s - 1));
+        uint32_t *w = tile + i * (M * G) + t % (M * G);
+        const uint32_t a2 = w[2 * s * (M * G)] ^ w[3 * s * (M * G)];
+        w[2 * s * (M * G)] = a2;
+        w[s * (M * G)] ^= a2;
+      }
+      __syncthreads();
+    }
+  }
+  uint32_t *out = Lf + (grp0 / LY::GPS) * LY::tile_words + grp0 % LY::GPS;
+  for (int t = threadIdx.x; t < POS * M * (G / 4); t += THREADS) {
+    const int row = t / (G / 4), c4 = t % (G / 4) * 4;
+    uint4 v = *reinterpret_cast<const uint4 *>(tile + row * G + c4);
+    if (p::lead) {
+      const uint32_t x = 0u - ((fd.lead_leaf[row / M] >> (row % M)) & 1u);
+      v.x ^= x;
+      v.y ^= x;
+      v.z ^= x;
+      v.w ^= x;
+    }
+    *reinterpret_cast<uint4 *>(out + row * LY::GPS + c4) = v;
+  }
+}
+
+// An item is one chunk of one tile; its levels run in three passes of tasks of
+// four slots in registers, through the tile in shared memory in between:
+//   pass 0  levels D-1, D-2: slots p0 + e 2^(D-2), from the leaves
+//   pass 1  levels D-3, D-4: block = the two top slot bits, slots p0 + e 2^(D-4)
+//   pass 2  the rest: block of 8 slots, slots p0 + 2 e, and level 0 across the
+//           half-warps; zero masks out
+// All levels share one loop body with two copies of the product's code (14 KB).
+template <int SET>
+__global__ void __launch_bounds__(256, 2) dec_fft_kernel(const uint32_t *__restrict__ Lf, FieldDev fd, long long items,
+                                                         long long ngroups, uint32_t *__restrict__ Z) {
+  using p = P<SET>;
+  using LY = SlicedLayout<SET>;
+  constexpr int M = p::m, D = LY::D, POS = LY::POS, GPS = LY::GPS, TASKS = POS / 8;
+  extern __shared__ __align__(16) uint32_t tile[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane & 15, h = lane >> 4;  // group of the tile; bit 0 of the slot
+  const uint32_t hm = h ? 0xFFFFFFFFu : 0u;
+  const uint16_t *__restrict__ alpha = fd.fft_alpha;
+  auto swap12 = [](uint32_t (&v)[4][M]) {
+#pragma unroll
+    for (int b = 0; b < M; b++) {
+      const uint32_t x = v[1][b];
+      v[1][b] = v[2][b];
+      v[2][b] = x;
+    }
+  };
+  const long long lo = items * blockIdx.x / gridDim.x, hi = items * (blockIdx.x + 1) / gridDim.x;
+  for (long long it = lo; it < hi; it++) {
+    const long long sg = it / LY::CHUNKS;
+    const int chunk = (int)(it % LY::CHUNKS);
+#pragma unroll 1
+    for (int pass = 0; pass < 3; pass++) {
+      if (pass) __syncthreads();
+#pragma unroll 1
+      for (int t = warp; t < TASKS; t += 8) {
+        constexpr int LOW = TASKS / 4;  // pass 1: tasks per block
+        const int blk = pass == 0 ? 0 : pass == 1 ? t / LOW : t;
+        const int p0 = pass == 0 ? 2 * t + h : pass == 1 ? blk * (POS / 4) + 2 * (t % LOW) + h : 8 * t + h;
+        const int s = pass == 0 ? POS / 4 : pass == 1 ? POS / 16 : 2;
+        const uint32_t *src = (pass == 0 ? Lf + sg * LY::tile_words : tile) + p0 * (M * GPS) + g;
+        uint32_t v[4][M];
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+#pragma unroll
+          for (int b = 0; b < M; b++) v[e][b] = src[(e * s * M + b) * GPS];
+        if (p::lead && pass == 0 && t == 0) {
+          const uint32_t kc = fd.lead_chunk[chunk];
+#pragma unroll
+          for (int b = 0; b < M; b++) v[0][b] ^= (0u - ((kc >> b) & 1u)) & ~hm;
+        }
+        // level of the first step and the index of its block's constant; the next level's are 2 i and 2 i + 1
+        const int l0 = D - 1 - 2 * pass;
+        const int i0 = pass == 0 ? chunk : pass == 1 ? 4 * chunk + blk : (chunk << (D - 3)) + blk;
+        const bool skip = D == 6 && pass == 2;  // (its second level is level 1)
+        if (skip) swap12(v);
+        const int steps = pass == 2 ? 3 : 2;
+#pragma unroll 1
+        for (int step = skip ? 1 : 0; step < steps; step++) {
+          uint32_t ca, cb;
+          if (step == 0) {
+            ca = cb = alpha[(p::q - (p::q >> l0)) + i0];
+          } else if (step == 1) {
+            const int l = pass == 2 ? 1 : l0 - 1;
+            ca = alpha[(p::q - (p::q >> l)) + 2 * i0];
+            cb = alpha[(p::q - (p::q >> l)) + 2 * i0 + 1];
+          } else {
+            // level 0 pairs the half-warps: half 0 takes the slot pairs e = 0, 1, half 1 the pairs 2, 3, whose
+            // constants are x^2 more (the level's constants are 2 i for the index i); v holds e = 0, 2, 1, 3
+            ca = alpha[(chunk << (D - 1)) + 4 * blk];
+            cb = alpha[(chunk << (D - 1)) + 4 * blk + 1];
+#pragma unroll
+            for (int b = 0; b < M; b++) {
+              const uint32_t g0 = __shfl_xor_sync(0xffffffffu, h ? v[0][b] : v[1][b], 16);
+              const uint32_t g1 = __shfl_xor_sync(0xffffffffu, h ? v[2][b] : v[3][b], 16);
+              const uint32_t lo0 = h ? g0 : v[0][b], hi0 = h ? v[1][b] : g0;
+              const uint32_t lo1 = h ? g1 : v[2][b], hi1 = h ? v[3][b] : g1;
+              v[0][b] = lo0;
+              v[2][b] = hi0;
+              v[1][b] = lo1;
+              v[3][b] = hi1;
+            }
+          }
+          ca = __reduce_or_sync(0xffffffffu, ca);  // uniform: branches, no masks
+          cb = __reduce_or_sync(0xffffffffu, cb);
+          sliced_butterflies<M, 1>({&v[0]}, {&v[2]}, ca);
+          sliced_butterflies<M, 1>({&v[1]}, {&v[3]}, cb);
+          if (step == 0) swap12(v);  // -> e = 0, 2, 1, 3: the pairs of the next level
+        }
+        if (pass < 2) {
+          uint32_t *dst = tile + p0 * (M * GPS) + g;
+#pragma unroll
+          for (int b = 0; b < M; b++) {
+            dst[b * GPS] = v[0][b];
+            dst[(s * M + b) * GPS] = v[2][b];
+            dst[(2 * s * M + b) * GPS] = v[1][b];
+            dst[(3 * s * M + b) * GPS] = v[3][b];
+          }
+        } else {
+          uint32_t z[4];
+#pragma unroll
+          for (int j = 0; j < 2; j++) {
+            // half 1: x^2 hi more on both outputs, hi = their sum
+            const int j0 = j, j1 = j + 2;
+            uint32_t f1[M], acc[2 * M - 1], fix[M], nu = 0, nv = 0;
+#pragma unroll
+            for (int k = 0; k < 2 * M - 1; k++) acc[k] = 0;
+#pragma unroll
+            for (int b = 0; b < M; b++) {
+              f1[b] = (v[j0][b] ^ v[j1][b]) & hm;
+              acc[b + 2] = f1[b];
+            }
+            bs_reduce<M>(fix, acc);
+#pragma unroll
+            for (int b = 0; b < M; b++) {
+              nu |= v[j0][b] ^ fix[b];
+              nv |= v[j1][b] ^ fix[b];
+            }
+            z[2 * j] = ~nu;
+            z[2 * j + 1] = ~nv;
+          }
+          const long long grp = sg * GPS + g;
+          if (grp < ngroups)
+            *reinterpret_cast<uint4 *>(Z + grp * p::q + chunk * POS + 8 * t + 4 * h) = make_uint4(z[0], z[1], z[2], z[3]);
+        }
+      }
+    }
+    __syncthreads();  // the tile is read no more
+  }
+}
+
+// Block per group: word w of 32 requests' error vectors is the transpose of the
+// zero masks at the support elements of positions 32 w .. 32 w + 31.
+template <int SET>
+__global__ void __launch_bounds__(256) dec_pos_kernel(const uint32_t *__restrict__ Z, const DecKeys keys,
+                                                      const Segs segs, uint32_t *__restrict__ E, int lde,
+                                                      int *__restrict__ okio) {
+  using p = P<SET>;
+  constexpr int Q = p::q, N = p::n, NW = (N + 31) / 32;
+  extern __shared__ __align__(16) uint32_t zs[];
+  __shared__ int wsum[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long op = 32LL * blockIdx.x + lane;
+  int seg;
+  const bool live = seg_live(segs, op, &seg);
+  if (!__any_sync(0xffffffffu, live)) return;  // the same for every warp
+  seg = seg_find(segs, 32LL * blockIdx.x);
+  for (int i = threadIdx.x; i < Q / 4; i += 256)
+    reinterpret_cast<uint4 *>(zs)[i] = reinterpret_cast<const uint4 *>(Z + (long long)blockIdx.x * Q)[i];
+  __syncthreads();
+  const uint16_t *__restrict__ L = keys.k[seg].L;
+  int weight = 0;
+  for (int w0 = 4 * warp; w0 < NW; w0 += 32) {
+    uint32_t x[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int pos = 32 * (w0 + k) + lane;
+      x[k] = transpose32(pos < N ? zs[L[pos]] : 0u, lane);
+      weight += __popc(x[k]);
+    }
+    if (live) {
+      uint32_t *row = E + op * lde + w0;
+      if (w0 + 4 <= NW) {
+        *reinterpret_cast<uint4 *>(row) = make_uint4(x[0], x[1], x[2], x[3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (w0 + k < NW) row[k] = x[k];
+      }
+    }
+  }
+  wsum[warp][lane] = weight;
+  __syncthreads();
+  if (warp == 0 && live) {
+    weight = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) weight += wsum[k][lane];
+    if (weight != p::t) okio[op] = 0;
+  }
+}
+
 // ---------------------------------------------------------------- tail
 // K = SHAKE256(b || (e or s) || c), s the key's n/8 bytes (stored zero-padded
 // to whole 16-byte units). The choice is a mask, not an address
@@ -1454,12 +1824,41 @@ static cudaError_t launch_dec_root_form(const uint16_t *Sig, const DecKeys &keys
 }
 
 template <int SET>
-cudaError_t launch_dec_root(const uint16_t *Sig, const DecKeys &keys, FieldDev fd,
-                            const Segs &segs, uint32_t *E, int lde, int *ok, cudaStream_t st, int warps, bool ct) {
+static cudaError_t launch_dec_root_sliced(const uint16_t *Sig, const DecKeys &keys, FieldDev fd, const Segs &segs,
+                                          uint32_t *E, int lde, int *ok,
+                                          cudaStream_t st, uint8_t *work) {
+  using p = P<SET>;
+  using LY = SlicedLayout<SET>;
+  const long long N = seg_rows(segs), ngroups = N / 32, nsg = (ngroups + LY::GPS - 1) / LY::GPS;
+  uint32_t *Lf = reinterpret_cast<uint32_t *>(work), *Z = Lf + nsg * LY::tile_words;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaError_t e = cudaFuncSetAttribute(dec_leaf_kernel<SET>, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::leaf_bytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(dec_fft_kernel<SET>, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::tile_words * 4);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(dec_pos_kernel<SET>, cudaFuncAttributeMaxDynamicSharedMemorySize, p::q * 4);
+  if (e != cudaSuccess) return e;
+  dec_leaf_kernel<SET><<<(unsigned)((ngroups + LY::LGPS - 1) / LY::LGPS), LY::leaf_threads, LY::leaf_bytes, st>>>(Sig, fd, segs, Lf, ok);
+  const long long items = nsg * LY::CHUNKS;
+  dec_fft_kernel<SET><<<(unsigned)std::min<long long>(items, 2LL * sms), 256, LY::tile_words * 4, st>>>(Lf, fd, items, ngroups,
+                                                                                                  Z);
+  dec_pos_kernel<SET><<<(unsigned)ngroups, 256, p::q * 4, st>>>(Z, keys, segs, E, lde, ok);
+  return cudaGetLastError();
+}
+
+template <int SET>
+cudaError_t launch_dec_root(const uint16_t *Sig, const DecKeys &keys, FieldDev fd, const Segs &segs, uint32_t *E,
+                            int lde, int *ok, cudaStream_t st, int warps, bool ct,
+                            uint8_t *work) {
   const long long N = seg_rows(segs);
   if (N <= 0) return cudaSuccess;
   if (warps < 0 || warps > kRootWarps) return cudaErrorInvalidValue;
   if (warps == 0) warps = kRootWarps;
+  if (work && dec_root_work_bytes(SET, N, ct)) {
+    if (!fd.fft_alpha || lde % 4) return cudaErrorInvalidValue;
+    return launch_dec_root_sliced<SET>(Sig, keys, fd, segs, E, lde, ok, st, work);
+  }
   if (ct) {
     if (!fd.fft_twist_cols) return cudaErrorInvalidValue;
     return launch_dec_root_form<SET, true>(Sig, keys, fd, segs, E, lde, ok, st, warps);
@@ -1595,12 +1994,27 @@ cudaError_t launch_dec_tail(const uint32_t *E, int lde, const int *ok, const uin
             : launch(dec_tail_kernel<SET, false, false>, kTailThreads / 2);
 }
 
+// scratch of the request-sliced root finder, 0 where the batch takes the chunk-sliced one
+size_t dec_root_work_bytes(int set, long long rows, bool ct) {
+  if (ct || rows < kRootSlicedMinRows) return 0;
+  auto bytes = [&](long long tile_words, long long q) {
+    return (size_t)((rows + 511) / 512 * tile_words * 4 + rows / 32 * q * 4);
+  };
+  switch (set) {
+    case 0: return bytes(SlicedLayout<0>::tile_words, P<0>::q);
+    case 1: return bytes(SlicedLayout<1>::tile_words, P<1>::q);
+    case 2: return bytes(SlicedLayout<2>::tile_words, P<2>::q);
+    case 3: return bytes(SlicedLayout<3>::tile_words, P<3>::q);
+    default: return bytes(SlicedLayout<4>::tile_words, P<4>::q);
+  }
+}
+
 #define GMC_INST_DEC(SET)                                                                                       \
   template cudaError_t launch_pack_ct<SET>(const uint8_t *, const Segs &, uint32_t *, int, bool, cudaStream_t);       \
   template cudaError_t launch_dec_bm<SET>(const uint32_t *, int, FieldDev, const Segs &, uint16_t *,             \
                                          cudaStream_t, int, bool);                                               \
   template cudaError_t launch_dec_root<SET>(const uint16_t *, const DecKeys &, FieldDev, const Segs &,          \
-                                            uint32_t *, int, int *, cudaStream_t, int, bool);      \
+                                            uint32_t *, int, int *, cudaStream_t, int, bool, uint8_t *);         \
   template cudaError_t launch_dec_tail<SET>(const uint32_t *, int, const int *, const uint8_t *, const DecKeys &, \
                                             uint8_t *, int *, const Segs &, bool, cudaStream_t);                 \
   template cudaError_t launch_dec_ct_finish<SET>(const DecKeys &, const Segs &, uint32_t *, int, int *,            \
