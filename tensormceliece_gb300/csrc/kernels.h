@@ -19,7 +19,11 @@ constexpr int kBMWarps = 14;    // Berlekamp-Massey kernel: default and largest 
 constexpr int kBMCtBlocksPerSM = 3;  // its constant-time form: blocks (groups of 32 requests) resident per SM
 constexpr int kBMLatWarps = 24;  // Berlekamp-Massey latency form: largest warps per block (one request per warp)
 constexpr int kBMLatCopyWarps = 8;  // its smallest block: warps without a request help to copy the tables
-constexpr long long kBMBitslicedMinRows = 24576;  // smaller batches take the latency form
+// Berlekamp-Massey: smaller batches take the latency form, a warp per request. The bit-sliced form, a warp per 32
+// requests, takes the same time until every SM has seven warps. us, bit-sliced / latency form: 348864 20000 rows
+// 197 / 174, 24576 198 / 217; 460896 28672 rows 428 / 404, 30720 430 / 464; 6960119 625 / 561, 622 / 641; 8192128
+// 682 / 625, 680 / 705, 36864 rows 679 / 845.
+constexpr long long bm_bitsliced_min_rows(int t) { return t <= 64 ? 22528 : 29696; }
 // Root finding: smaller batches take the warp-per-request form. us, request-sliced / warp per request: 12288 rows
 // 205 / 205 (8192128), 201 / 201 (6960119), 95 / 90 (348864); 14336 rows 205 / 226, 202 / 222, 96 / 98; 65536 rows
 // 793 / 980, 778 / 970, 343 / 407.

@@ -67,46 +67,64 @@ __global__ void pack_ct_kernel(const uint8_t *__restrict__ C, const Segs segs, u
 // ---------------------------------------------------------------- BM
 // One warp per group of 32 requests, bit-sliced: bit q of every word belongs
 // to request 32g + q, and a GF(2^m) value of all 32 requests is m words
-// (planes). Coefficient i of C (connection polynomial) lives in lane i%32,
-// slot i/32, as m plane registers; B and the syndromes sit in per-warp shared
-// memory as planes. Per iteration n:
-//   d = sum_i C_i s_{n-i}: carry-less plane products accumulated unreduced,
-//       one reduction, then one XOR reduction instruction per plane;
+// (planes). Coefficient i >= 1 of C (connection polynomial, C_0 = 1) lives in
+// lane (i-1)%32, slot (i-1)/32, as m plane registers; B and the syndromes sit in
+// per-warp shared memory as planes. Per iteration n:
+//   d = s_n + sum_i C_i s_{n-i}: carry-less plane products accumulated
+//       unreduced, one reduction, then one XOR reduction instruction per plane;
 //   f = d/b per request: lane q extracts its request's d, divides with the
 //       log tables (L and log b are per-request scalars in lane q) and the
 //       32 quotients are sliced back by ballot;
-//   C_i += f B_i (bit-sliced product), and B <- x (upd ? C_old : B) with the
-//       per-request update mask from a ballot.
+//   C_i += f B_i (bit-sliced product onto C_i, one reduction), and
+//       B <- x (upd ? C_old : B) with the per-request update mask from a ballot.
 // This is the library's update rule (mc:crypto_kem/348864/vec/bm.c:156) on
 // fixed arrays of t+1 coefficients, per request; the slot loops stop at the
 // largest degree bound of the group: before iteration n, deg C <= L and
 // deg B <= n+1-L, so the discrepancy needs i <= min(L, t) and the update
 // i <= min(max(L, n+1-L), t). Rows that are not live run with zero
 // syndromes (d = 0) and write nothing.
+// Both arrays are rings that turn with n: s_{n-i} and B_i have fixed entries for
+// the iterations that use them. Multiplying B by x moves nothing, so iterations
+// in which no request of the group takes the new B (every second one as long as
+// no discrepancy is 0) write nothing; entry i of B is read and replaced by the
+// lane that holds C_i, without barriers. The syndrome ring is filled 32 planes at
+// a time by a transpose of one word of every request's packed syndromes.
 // Shared memory per warp is what fourteen warps per SM can hold (one round
-// for 2048 groups on 152 SMs): iteration n reads s_{n-t} .. s_n only, so the
-// syndromes sit in a ring of t+1 entries, filled one syndrome per iteration
-// (its global load issued an iteration ahead); B keeps coefficients 0..t
-// (reads above t are zero); the exponent table keeps the q-1 entries the
-// division indexes. Lanes above deg C in an active discrepancy slot read
-// ring entries of other iterations: C_i = 0 there (coefficients above t are
-// never updated), so they add nothing.
+// for 2048 groups on 152 SMs): iteration n reads s_{n-t} .. s_n only, and a fill
+// reaches at most three syndromes ahead; B keeps coefficients 0..t; the exponent
+// table keeps the q-1 entries the division indexes. Lanes above deg C in an
+// active discrepancy slot read ring entries of other iterations: C_i = 0 there
+// (coefficients above t are never updated), so they add nothing.
+// 8192128: 65536 requests 1201 us (91% of the XOR pipe's rate), 32768 680 us; with B moved by one entry and
+// the coefficient C_0 computed with the others, 1335 and 782.
 template <int SET>
 struct BMLayout {
   using p = P<SET>;
   static constexpr int Q = p::q, T = p::t, M = p::m;
-  static constexpr int NS = (T + 1 + 31) / 32;
-  static constexpr int R = T + 1;                              // syndrome ring entries
+  static constexpr int NS = (T + 31) / 32;
+  static constexpr int R = T + 4;                              // syndrome ring entries
+  static constexpr int RB = T + 1;                             // B ring entries
   static constexpr int exp_off = 0, log_off = Q;               // u16 tables (exp: indexes 0..q-2)
-  static constexpr int zero_off = Q, zero_len = 16;            // u32: M zero planes (s_j, j < 0)
-  static constexpr int shared_u32 = zero_off + zero_len;
+  static constexpr int shared_u32 = Q;
   static constexpr int s_words = R * M;                        // syndrome planes [j mod R][b]
-  static constexpr int b_words = (T + 1) * M;                  // B planes [i][b], i <= t
+  static constexpr int b_words = RB * M;                       // B_i of iteration n: [(i - n) mod RB][b]
   static constexpr int warp_u32 = s_words + b_words;
   static constexpr int bytes(int warps) { return shared_u32 * 4 + warps * warp_u32 * 4; }
   static_assert(32 * NS * M <= warp_u32, "C planes are staged in the warp's area");
-  static_assert(2 * T <= 2 * R, "ring index j - R for j < 2t");
+  static_assert(32 + M - 1 <= 4 * M, "the planes of a fill at iteration n belong to s_n .. s_(n+3)");
 };
+
+// bit j of lane l -> bit l of lane j
+__device__ __forceinline__ uint32_t transpose32(uint32_t v, int lane) {
+  uint32_t m = 0x0000FFFFu;
+#pragma unroll
+  for (int s = 16; s; s >>= 1) {
+    const uint32_t o = __shfl_xor_sync(0xffffffffu, v, s);
+    v = (lane & s) ? ((o >> s) & m) | (v & ~m) : (v & m) | ((o & m) << s);
+    m ^= m << (s >> 1);
+  }
+  return v;
+}
 
 // acc (2M-1 planes, unreduced) -> r (M planes) mod the field polynomial, in
 // three-input XORs: with h_j the plane of x^(M+j), x^13 = x^4 + x^3 + x + 1
@@ -141,7 +159,7 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
   using p = P<SET>;
   using LY = BMLayout<SET>;
   constexpr int M = p::m, Q = p::q, T = p::t, D = p::fft_d;
-  constexpr int NS = LY::NS, R = LY::R;
+  constexpr int NS = LY::NS, R = LY::R, RB = LY::RB;
   constexpr int SIG = 1 << D;
   static_assert(M == 12 || M == 13, "field polynomial");
   extern __shared__ __align__(16) uint32_t bsm[];
@@ -150,10 +168,8 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
   chain_trigger();
   copy_table(gexp, fd.gexp, Q);
   copy_table(glog, fd.glog, Q);
-  for (int i = threadIdx.x; i < LY::zero_len; i += blockDim.x) bsm[LY::zero_off + i] = 0u;
   __syncthreads();
   chain_wait();
-  const uint32_t *ZP = bsm + LY::zero_off;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t *SP = bsm + LY::shared_u32 + warp * LY::warp_u32;
   uint32_t *BP = SP + LY::s_words;
@@ -168,56 +184,55 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
     const long long op = g * 32 + lane;
     int seg;
     const bool live = op < N && seg_live(segs, op, &seg);
+    constexpr int SW = (2 * T * M + 31) / 32;  // words of packed syndromes
     const uint32_t *srow = S2 + op * lds2;
-    // this lane's request's s_j (low M bits; 0 past the live rows)
-    auto synd = [&](int j) -> uint32_t {
-      uint32_t v = 0;
-      if (live) {
-        const int bb = j * M, w = bb >> 5, sh = bb & 31;
-        v = srow[w] >> sh;
-        if (sh + M > 32) v |= srow[w + 1] << (32 - sh);
-      }
-      return v;
-    };
-    // one syndrome of all 32 requests -> M planes in ring entry e (lane b < M stores plane b)
-    auto to_ring = [&](uint32_t v, int e) {
-      uint32_t pl[M];
-#pragma unroll
-      for (int b = 0; b < M; b++) pl[b] = __ballot_sync(0xffffffffu, (v >> b) & 1u);
-      if (lane == 0) {  // the planes are warp-uniform: one lane stores them (no per-lane selects)
-#pragma unroll
-        for (int b = 0; b < M; b++) SP[e * M + b] = pl[b];
-      }
-    };
-    to_ring(synd(0), 0);
     // C = 1, B = x
     uint32_t C[NS][M];
 #pragma unroll
     for (int k = 0; k < NS; k++)
 #pragma unroll
-      for (int b = 0; b < M; b++) C[k][b] = (k == 0 && lane == 0 && b == 0) ? 0xFFFFFFFFu : 0u;
+      for (int b = 0; b < M; b++) C[k][b] = 0u;
     for (int w = lane; w < LY::b_words; w += 32) BP[w] = (w == M) ? 0xFFFFFFFFu : 0u;
-    __syncwarp();
     int L = 0, lb = 0;  // this lane's request: LFSR length, log b
+    // this lane's request's packed syndromes: `have` bits of the current ones in sbits, word wn next (its value in
+    // word_n), of which the planes go to ring word 32 wn mod R M + lane
+    uint64_t sbits = 0;
+    int have = 0, wn = 0, fill = lane;
+    uint32_t word_n = live ? srow[0] : 0u;
+    int es = (R - 1 - lane) % R;  // ring entry of s_{n-1-lane}
+    int eb = 1 + lane;            // ring entry of B_{1+lane}
+    int e0 = 0;                   // ring entry of B_0
 #pragma unroll 1
     for (int n = 0; n < 2 * T; n++) {
-      const uint32_t s_next = n + 1 < 2 * T ? synd(n + 1) : 0u;  // consumed at the end of the iteration
+      if (have < M) {  // uniform
+        SP[fill] = transpose32(word_n, lane);
+        fill += 32;
+        if (fill >= R * M) fill -= R * M;
+        sbits |= (uint64_t)word_n << have;
+        have += 32;
+        wn++;
+        word_n = live && wn < SW ? srow[wn] : 0u;  // consumed two or three iterations later
+        __syncwarp();
+      }
+      uint32_t dq = (uint32_t)sbits & ((1u << M) - 1);  // s_n of this lane's request (C_0 = 1)
+      sbits >>= M;
+      have -= M;
       const int Lc = L < T ? L : T;
       int Lu = (L > n + 1 - L) ? L : n + 1 - L;
       Lu = Lu < T ? Lu : T;
       const int bd = (int)__reduce_max_sync(0xffffffffu, live ? (unsigned)Lc : 0u);
       const int bu = (int)__reduce_max_sync(0xffffffffu, live ? (unsigned)Lu : 0u);
-      // discrepancy planes
-      uint32_t d[M];
-      {
-        uint32_t acc[2 * M - 1];
+      // discrepancy planes of the other coefficients
+      if (bd > 0) {
+        uint32_t acc[2 * M - 1], d[M];
 #pragma unroll
         for (int k = 0; k < 2 * M - 1; k++) acc[k] = 0;
 #pragma unroll
         for (int k = 0; k < NS; k++) {
-          if (32 * k <= bd) {
-            const int j = n - lane - 32 * k;  // s_j (ring entry j mod R), j < 0 reads the zero planes
-            const uint32_t *sp = j >= 0 ? SP + (j >= R ? j - R : j) * M : ZP;
+          if (32 * k < bd) {
+            int e = es - 32 * k;
+            if (e < 0) e += R;
+            const uint32_t *sp = SP + e * M;
 #pragma unroll
             for (int b2 = 0; b2 < M; b2++) {
               const uint32_t sv = sp[b2];
@@ -229,11 +244,10 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
         bs_reduce<M>(d, acc);
 #pragma unroll
         for (int b = 0; b < M; b++) d[b] = __reduce_xor_sync(0xffffffffu, d[b]);
+#pragma unroll
+        for (int b = 0; b < M; b++) dq ^= ((d[b] >> lane) & 1u) << b;
       }
       // this lane's request: f = d / b, the update decision
-      uint32_t dq = 0;
-#pragma unroll
-      for (int b = 0; b < M; b++) dq += ((d[b] >> lane) & 1u) << b;  // disjoint bits: the add may fuse
       const bool upd = dq != 0 && 2 * L <= n;
       uint32_t fq = 0;
       int ld = 0;
@@ -252,58 +266,41 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
         L = n + 1 - L;
         lb = ld;
       }
-      // C_i += f B_i; B_{i+1} <- (U ? C_i(old) : B_i); slots in descending
-      // order so slot k's write of B_{32(k+1)} follows slot k+1's read of it
+      // C_i += f B_i; B_{i+1} <- (U ? C_i(old) : B_i) in B_i's entry
+      if (anyf) {
 #pragma unroll
-      for (int k = NS - 1; k >= 0; k--) {
-        if (32 * k <= bu) {
-          const int i = lane + 32 * k;
-          const uint32_t *bp = BP + i * M;
-          uint32_t bi[M];
+        for (int k = 0; k < NS; k++) {
+          if (32 * k < bu && 32 * k + lane < T) {  // coefficients above t stay zero
+            int e = eb + 32 * k;
+            if (e >= RB) e -= RB;
+            uint32_t *bp = BP + e * M;
+            uint32_t bi[M], acc[2 * M - 1];
 #pragma unroll
-          for (int b = 0; b < M; b++) bi[b] = i <= T ? bp[b] : 0u;
-          __syncwarp();  // every lane holds its B_i before B_{i+1} is replaced
-          const bool in = i <= T;  // coefficients above t stay zero
-          uint32_t r[M];
-          if (anyf) {
-            // r = f * B_i, Horner over the planes of f
+            for (int b = 0; b < M; b++) bi[b] = bp[b];
+            if (U) {
 #pragma unroll
-            for (int b = 0; b < M; b++) r[b] = bi[b] & f[M - 1];
-#pragma unroll
-            for (int jj = M - 2; jj >= 0; jj--) {
-              const uint32_t top = r[M - 1];
-#pragma unroll
-              for (int b = M - 1; b > 0; b--) r[b] = r[b - 1];
-              r[0] = top;
-              if (M == 13) {
-                r[1] ^= top;
-                r[3] ^= top;
-                r[4] ^= top;
-              } else {
-                r[3] ^= top;
-              }
-#pragma unroll
-              for (int b = 0; b < M; b++) r[b] ^= bi[b] & f[jj];
+              for (int b = 0; b < M; b++) bp[b] = (U & C[k][b]) | (~U & bi[b]);
             }
-          } else {
 #pragma unroll
-            for (int b = 0; b < M; b++) r[b] = 0;
-          }
-          uint32_t *bq = BP + (i + 1) * M;
+            for (int x = 0; x < 2 * M - 1; x++) acc[x] = x < M ? C[k][x] : 0u;
 #pragma unroll
-          for (int b = 0; b < M; b++) {
-            const uint32_t cold = C[k][b];
-            if (in) C[k][b] = cold ^ r[b];
-            if (i + 1 <= T) bq[b] = (U & cold) | (~U & bi[b]);
+            for (int j = 0; j < M; j++)
+#pragma unroll
+              for (int b = 0; b < M; b++) acc[j + b] ^= bi[b] & f[j];
+            bs_reduce<M>(C[k], acc);
           }
-          // no barrier before the next (lower) slot: its reads, B_{32(k-1)} ..
-          // B_{32k-1}, miss this slot's writes, B_{32k+1} .. B_{32k+32}, and
-          // its writes follow its own barrier above, after this slot's reads
         }
       }
-      if (lane < M) BP[lane] = 0;  // B_0 of x * (...) is zero (slot 0 read it before its barrier)
-      // s_{n+1} replaces s_{n-t}, the oldest entry (read above, before the update's warp barriers)
-      if (n + 1 < 2 * T) to_ring(s_next, n + 1 >= R ? n + 1 - R : n + 1);
+      // B_1 <- U ? C_0 : B_0 = 0 in B_0's entry; the next B_0 is 0, in the entry of B_t
+      const int et = e0 ? e0 - 1 : RB - 1;
+      __syncwarp();
+      if (lane < M) {
+        if (lane == 0) BP[e0 * M] = U;
+        BP[et * M + lane] = 0;
+      }
+      e0 = et;
+      eb = eb ? eb - 1 : RB - 1;
+      es = es + 1 < R ? es + 1 : 0;
       __syncwarp();
     }
     // sigma(x) = sum_deg C[t-deg] x^deg -> FFT coefficient slots (deg < 2^d);
@@ -313,20 +310,22 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
     for (int k = 0; k < NS; k++)
 #pragma unroll
       for (int b = 0; b < M; b++) SP[(lane + 32 * k) * M + b] = C[k][b];
+    const uint32_t flags = __ballot_sync(0xffffffffu, L != T);
     __syncwarp();
-    if (live) {
-      uint16_t *sig = Sig + op * SIG;
+    const int b = lane & 15;
 #pragma unroll 1
-      for (int deg = 0; deg < SIG; deg++) {
-        const int i = T - deg;
-        uint32_t v = 0;
-        if (i >= 0) {
+    for (int u = 0; u < SIG / 8; u++) {
+      uint32_t wd[4];
 #pragma unroll
-          for (int b = 0; b < M; b++) v |= ((SP[i * M + b] >> lane) & 1u) << b;
-        }
-        if (deg == 0 && L != T) v |= 0x8000u;
-        sig[deg] = (uint16_t)v;
+      for (int x = 0; x < 4; x++) {  // two coefficients: planes b of degree deg in the half-warps
+        const int deg = 8 * u + 2 * x + (lane >> 4), i = T - deg;
+        uint32_t v = 0;
+        if (b < M && i >= 1) v = SP[(i - 1) * M + b];
+        if (b == 0 && i == 0) v = 0xFFFFFFFFu;
+        if (b == 15 && deg == 0) v = flags;
+        wd[x] = transpose32(v, lane);
       }
+      if (live) reinterpret_cast<uint4 *>(Sig + op * SIG)[u] = make_uint4(wd[0], wd[1], wd[2], wd[3]);
     }
     __syncwarp();
   }
@@ -456,18 +455,6 @@ struct BMCtLayout {
   static constexpr int bytes = (b_off + b_len) * 4;
   static_assert((32 * NS + 1) * M <= s_len, "C planes are staged in the syndrome area");
 };
-
-// bit j of lane l -> bit l of lane j
-__device__ __forceinline__ uint32_t transpose32(uint32_t v, int lane) {
-  uint32_t m = 0x0000FFFFu;
-#pragma unroll
-  for (int s = 16; s; s >>= 1) {
-    const uint32_t o = __shfl_xor_sync(0xffffffffu, v, s);
-    v = (lane & s) ? ((o >> s) & m) | (v & ~m) : (v & m) | ((o & m) << s);
-    m ^= m << (s >> 1);
-  }
-  return v;
-}
 
 // the first M (at most 16) words of shared memory to d, four at a time
 template <int M>
@@ -1784,7 +1771,7 @@ cudaError_t launch_dec_bm(const uint32_t *S2, int lds2, FieldDev fd, const Segs 
     return launch_chained(segs, dec_bm_ct_kernel<SET>, (unsigned)((N + 31) / 32), (LY::NS + 1) * 32, LY::bytes, st, S2, lds2,
                           segs, Sig);
   }
-  if (N < kBMBitslicedMinRows) {  // small batch: warp per request (lower latency per request)
+  if (N < bm_bitsliced_min_rows(P<SET>::t)) {  // small batch: warp per request (lower latency per request)
     // warps per block: as few rounds over two blocks per SM as kBMLatWarps
     // allows, all of them full
     int dev = 0, sms = 0;

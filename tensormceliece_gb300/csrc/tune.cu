@@ -298,7 +298,7 @@ extern "C" int gmc_autotune(int set, long long n, const char *cache_path) {
     // requests per block of the decoding kernels
     const int bm_cand[3] = {kBMWarps, 8, 4};
     const int warp_cand[3] = {kRootWarps, 4, 2};
-    if (n >= kBMBitslicedMinRows)
+    if (n >= bm_bitsliced_min_rows(set_info(set).t))
       for (int wi = 1; wi < 3; wi++) {
         SetTune t = best;
         t.bm_warps = bm_cand[wi];
@@ -308,7 +308,7 @@ extern "C" int gmc_autotune(int set, long long n, const char *cache_path) {
           best.bm_warps = bm_cand[wi];
         }
       }
-    for (int wi = 1; wi < 3; wi++) {
+    for (int wi = 1; wi < 3 && n < kRootSlicedMinRows; wi++) {  // (larger batches take another root finder)
       SetTune t = best;
       t.root_warps = warp_cand[wi];
       const float ms = time_dec(t);
