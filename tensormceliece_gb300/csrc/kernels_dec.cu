@@ -673,10 +673,17 @@ __global__ void __launch_bounds__((BMCtLayout<SET>::NS + 1) * 32, kBMCtBlocksPer
 // slots, each with straight-line slot code: the slots' table lookups overlap.
 // With a test per slot their latencies added up: 8192128, 1 / 2048 / 8192 /
 // 20000 (6688128) requests 92 / 114 / 258 / 625 us, against 58 / 74 / 199 /
-// 459 us now. Four warps per request with a barrier an iteration were slower
+// 459 us with the straight loops. Four warps per request with a barrier an iteration were slower
 // (66 us for one request, 338 against 105 us for 4096).
-// Bound: the chain of one iteration up to about 2000 requests, above that the
-// bank conflicts of the table lookups (about 9 shared-memory wavefronts a slot).
+// AHEAD, for blocks of at most kBMLatCopyWarps requests: the chain of one
+// iteration is the bound there, and in it the discrepancy waits for the update
+// of C. d_{n+1} = e + f q with e = sum_i C_i s_{n+1-i} of the C before the update
+// and q = sum_i B_i s_{n+1-i}; when B becomes x C, q becomes that e, and else B is
+// multiplied by x while n grows by one, so q stays. So the dot product and the
+// update of C run at the same time, without branches on d. One request 58 -> 45
+// us, 2048 requests 74 -> 72; with full blocks the longer code loses (20000
+// requests 461 -> 508), where the bound is the bank conflicts of the table
+// lookups (about 9 shared-memory wavefronts a slot).
 template <int SET>
 struct BMLatLayout {
   using p = P<SET>;
@@ -692,8 +699,8 @@ struct BMLatLayout {
   static constexpr int bytes(int warps) { return shared_u16 * 2 + warps * warp_u16 * 2; }
 };
 
-template <int SET>
-__global__ void __launch_bounds__(kBMLatWarps * 32, 2) dec_bm_lat_kernel(const uint32_t *__restrict__ S2, int lds2,
+template <int SET, bool AHEAD>
+__global__ void __launch_bounds__((AHEAD ? kBMLatCopyWarps : kBMLatWarps) * 32, 2) dec_bm_lat_kernel(const uint32_t *__restrict__ S2, int lds2,
                                                                   FieldDev fd, const Segs segs,
                                                                   uint16_t *__restrict__ Sig, int nwb) {
   using p = P<SET>;
@@ -748,29 +755,33 @@ __global__ void __launch_bounds__(kBMLatWarps * 32, 2) dec_bm_lat_kernel(const u
 #pragma unroll
     for (int k = 0; k < NS; k++) lC[k] = ZL;
     int L = 0, sft = 1, n = 0;
-    uint32_t lb = 0;  // log b, b = 1
+    uint32_t lb = 0;        // log b, b = 1
+    uint32_t d = sraw[0];   // AHEAD: the discrepancy of iteration n
+    uint32_t lq = slog[0];  // AHEAD: log q, q = sum_i B_i s_{n+1-i}
     // the iterations that need K slots
     auto iterate = [&](auto slots) {
       constexpr int K = decltype(slots)::value;
 #pragma unroll 1
       for (; n < 2 * T; n++) {
         if (K < NS && (L > 32 * K || n + 1 - L > 32 * K)) return;
-        const uint16_t *sn = slog + n - 1 - lane, *bs = blog + 1 + lane - sft;
-        uint32_t dp = 0, lbi[K];
+        if constexpr (AHEAD) {
+          const uint16_t *sn = slog + n - lane, *bs = blog + 1 + lane - sft;
+          const uint32_t ld = glog[d];
+          const bool upd = d != 0 && n >= 2 * L;
+          uint32_t dp = 0, lbi[K], lco[K];
 #pragma unroll
-        for (int k = 0; k < K; k++) dp ^= gf_mul_log<M>(gexp, lC[k], sn[-32 * k]);
+          for (int k = 0; k < K; k++) dp ^= gf_mul_log<M>(gexp, lC[k], sn[-32 * k]);
 #pragma unroll
-        for (int k = 0; k < K; k++) lbi[k] = bs[32 * k];
-        const uint32_t d = __reduce_xor_sync(0xffffffffu, dp) ^ sraw[n];
-        if (d) {
-          const bool upd = (n >= 2 * L);
-          const int ld = glog[d];
-          int lf = ld - (int)lb;
-          if (lf < 0) lf += Q - 1;
-          uint32_t lco[K];
+          for (int k = 0; k < K; k++) lbi[k] = bs[32 * k];
+          // e = sum_i C_i s_{n+1-i} (of no use after the last iteration, where sraw[2t] is another array's)
+          uint32_t e = __reduce_xor_sync(0xffffffffu, dp);
+          // f = d / b; no f for d = 0
+          int lf = (int)ld - (int)lb;
+          lf += lf < 0 ? Q - 1 : 0;
+          const uint32_t fq = gf_mul_log<M>(gexp, d ? lf : (int)ZL, (int)lq);
 #pragma unroll
           for (int k = 0; k < K; k++) {
-            // log(C_i + f B_i): pl = log(f B_i); zero B_i keeps C_i, zero C_i takes pl
+            // log(C_i + f B_i): pl = log(f B_i); zero f B_i keeps C_i, zero C_i takes pl
             constexpr uint32_t Q1 = Q - 1;
             const uint32_t lc = lC[k];
             lco[k] = lc;
@@ -782,20 +793,68 @@ __global__ void __launch_bounds__(kBMLatWarps * 32, 2) dec_bm_lat_kernel(const u
             uint32_t nl = lc + z;
             nl = min(nl, nl - Q1);                      // >= 2q-2 when the sum is 0
             nl = (lc >= (uint32_t)ZL) ? pl : nl;
-            nl = (lbi[k] >= (uint32_t)ZL) ? lc : nl;
+            nl = (d == 0 || lbi[k] >= (uint32_t)ZL) ? lc : nl;
             if (32 * (k + 1) <= T || 1 + lane + 32 * k <= T) lC[k] = nl;  // coefficients above t stay zero
           }
-          if (upd) {
-            __syncwarp();  // every lane has read B' before it is replaced
+          __syncwarp();  // every lane has read B' before it is replaced
 #pragma unroll
-            for (int k = 0; k < K; k++) blog[1 + lane + 32 * k] = (uint16_t)lco[k];
-            __syncwarp();
+          for (int k = 0; k < K; k++)
+            if (upd) blog[1 + lane + 32 * k] = (uint16_t)lco[k];
+          __syncwarp();
+          e ^= sraw[n + 1];
+          const uint32_t dnext = e ^ fq;
+          const uint32_t le = glog[e & (Q - 1)];
+          if (upd) {
             L = n + 1 - L;
             lb = ld;
+            lq = le;  // B is x C_n from here on
             sft = 0;
           }
+          d = dnext;
+          sft++;
+        } else {
+          const uint16_t *sn = slog + n - 1 - lane, *bs = blog + 1 + lane - sft;
+          uint32_t dp = 0, lbi[K];
+#pragma unroll
+          for (int k = 0; k < K; k++) dp ^= gf_mul_log<M>(gexp, lC[k], sn[-32 * k]);
+#pragma unroll
+          for (int k = 0; k < K; k++) lbi[k] = bs[32 * k];
+          const uint32_t d = __reduce_xor_sync(0xffffffffu, dp) ^ sraw[n];
+          if (d) {
+            const bool upd = (n >= 2 * L);
+            const int ld = glog[d];
+            int lf = ld - (int)lb;
+            if (lf < 0) lf += Q - 1;
+            uint32_t lco[K];
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+              // log(C_i + f B_i): pl = log(f B_i); zero B_i keeps C_i, zero C_i takes pl
+              constexpr uint32_t Q1 = Q - 1;
+              const uint32_t lc = lC[k];
+              lco[k] = lc;
+              uint32_t pl = (uint32_t)lf + lbi[k];
+              pl = min(pl, pl - Q1);                      // < q-1 when B_i != 0
+              uint32_t kk = pl - lc;                      // log(f B_i / C_i) mod q-1
+              kk = min(kk + Q1, kk);
+              const uint32_t z = zech[min(kk, Q1 - 1)];   // index clamped for the zero cases
+              uint32_t nl = lc + z;
+              nl = min(nl, nl - Q1);                      // >= 2q-2 when the sum is 0
+              nl = (lc >= (uint32_t)ZL) ? pl : nl;
+              nl = (lbi[k] >= (uint32_t)ZL) ? lc : nl;
+              if (32 * (k + 1) <= T || 1 + lane + 32 * k <= T) lC[k] = nl;  // coefficients above t stay zero
+            }
+            if (upd) {
+              __syncwarp();  // every lane has read B' before it is replaced
+#pragma unroll
+              for (int k = 0; k < K; k++) blog[1 + lane + 32 * k] = (uint16_t)lco[k];
+              __syncwarp();
+              L = n + 1 - L;
+              lb = ld;
+              sft = 0;
+            }
+          }
+          sft++;
         }
-        sft++;
       }
     };
     iterate(std::integral_constant<int, 1>{});
@@ -1782,11 +1841,14 @@ cudaError_t launch_dec_bm(const uint32_t *S2, int lds2, FieldDev fd, const Segs 
     const int lw = (int)((N + blocks * rounds - 1) / (blocks * rounds));
     const int smem_l = BMLatLayout<SET>::bytes(lw);
     const int threads = 32 * (lw < kBMLatCopyWarps ? kBMLatCopyWarps : lw);
-    cudaError_t err = cudaFuncSetAttribute(dec_bm_lat_kernel<SET>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           BMLatLayout<SET>::bytes(kBMLatWarps));
-    if (err != cudaSuccess) return err;
-    const int gl = persistent_blocks(dec_bm_lat_kernel<SET>, threads, smem_l, N, lw);
-    return launch_chained(segs, dec_bm_lat_kernel<SET>, gl, threads, smem_l, st, S2, lds2, fd, segs, Sig, lw);
+    auto launch = [&](auto kern) {
+      cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             BMLatLayout<SET>::bytes(kBMLatWarps));
+      if (err != cudaSuccess) return err;
+      const int gl = persistent_blocks(kern, threads, smem_l, N, lw);
+      return launch_chained(segs, kern, gl, threads, smem_l, st, S2, lds2, fd, segs, Sig, lw);
+    };
+    return lw <= kBMLatCopyWarps ? launch(dec_bm_lat_kernel<SET, true>) : launch(dec_bm_lat_kernel<SET, false>);
   }
   warps = bm_block_warps(N, warps);
   const int smem_bm = BMLayout<SET>::bytes(warps);

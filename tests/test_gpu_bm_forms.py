@@ -44,3 +44,29 @@ def test_bm_forms_edges(keys, sid):
                 assert (k == ref[lo:hi]).all() and (r == rc[lo:hi]).all(), (on, lo, hi)
         finally:
             gmc.set_dec_constant_time(False)
+
+
+@pytest.mark.parametrize("sid", range(5), ids=SETS)
+def test_bm_latency_block_sizes(keys, sid):
+    """Both sides of the largest batch with at most eight requests per block (the look-ahead discrepancy)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import tensormceliece_gb300 as gmc
+
+    pk, sk = keys(sid)
+    z = O.sizes(sid)
+    base = 61
+    cts, _, _ = gmc.PublicKey(sid, pk).enc_batch(request_seeds(sid, base, b"blk"))
+    rng = np.random.default_rng(sid)
+    for i in range(0, base, 4):
+        cts[i, rng.integers(0, z["mt"] // 8)] ^= 1 << rng.integers(0, 8)
+    cts[3] = 0
+    cts[7] = 0
+    cts[7, 0] = 2  # discrepancies that vanish from some iteration on
+    ref, rc = O.dec_batch(sid, sk, cts, threads=THREADS)
+    sec = gmc.SecretKey(sid, sk)
+    edge = 16 * torch.cuda.get_device_properties(0).multi_processor_count
+    for n in (edge, edge + 1):
+        pick = np.arange(n) % base
+        k, r = sec.dec_batch(cts[pick])
+        assert (k == ref[pick]).all() and (r == rc[pick]).all(), n
