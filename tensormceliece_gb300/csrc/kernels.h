@@ -16,6 +16,8 @@ constexpr int kSampleThreadsMax = 128;  // sampler block size is a launch parame
 constexpr int kTailThreads = 64;
 constexpr int kTailBlocksPerSM = 14;
 constexpr int kBMWarps = 14;    // Berlekamp-Massey kernel: default and largest warps per block (32 requests per warp)
+constexpr int kBMBlockWarps = 16;  // its block: the warps that finish split groups are in addition
+constexpr int kBMCutNum = 11;      // a split group changes warps after this many sixteenths of its iterations
 constexpr int kBMCtBlocksPerSM = 3;  // its constant-time form: blocks (groups of 32 requests) resident per SM
 constexpr int kBMLatWarps = 24;  // Berlekamp-Massey latency form: largest warps per block (one request per warp)
 constexpr int kBMLatCopyWarps = 8;  // its smallest block: warps without a request help to copy the tables

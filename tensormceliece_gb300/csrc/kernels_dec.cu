@@ -95,8 +95,17 @@ __global__ void pack_ct_kernel(const uint8_t *__restrict__ C, const Segs segs, u
 // table keeps the q-1 entries the division indexes. Lanes above deg C in an
 // active discrepancy slot read ring entries of other iterations: C_i = 0 there
 // (coefficients above t are never updated), so they add nothing.
-// 8192128: 65536 requests 1201 us (91% of the XOR pipe's rate), 32768 680 us; with B moved by one entry and
-// the coefficient C_0 computed with the others, 1335 and 782.
+// A warp's instructions all go through one of the SM's four schedulers, so 13 or
+// 14 groups in a block take the time of 16. One or two groups more than a multiple
+// of four therefore change warps, to the two schedulers with fewer, after 11/16 of
+// their iterations (half of their work, and a little more because the second half
+// ends alone); C and the scalars pass through the group's rows of Sig. Not with
+// fewer than eight groups below them, where the second half alone is longer than
+// what the schedulers gain.
+// 8192128: 65536 requests 1072 us, 40000 822, 32768 680; without split groups
+// 1201 (91% of the XOR pipe's rate), 922 and 680; before, with B moved by one entry
+// and the coefficient C_0 computed with the others, 1335, 1024 and 782. Cut after
+// 10 / 12 / 13 sixteenths: 65536 1084 / 1094 / 1119.
 template <int SET>
 struct BMLayout {
   using p = P<SET>;
@@ -153,9 +162,9 @@ __device__ __forceinline__ void bs_reduce(uint32_t (&r)[M], const uint32_t (&acc
 }
 
 template <int SET>
-__global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t *__restrict__ S2, int lds2,
+__global__ void __launch_bounds__(kBMBlockWarps * 32, 1) dec_bm_kernel(const uint32_t *__restrict__ S2, int lds2,
                                                                   FieldDev fd, const Segs segs,
-                                                                  uint16_t *__restrict__ Sig) {
+                                                                  uint16_t *__restrict__ Sig, int nwb) {
   using p = P<SET>;
   using LY = BMLayout<SET>;
   constexpr int M = p::m, Q = p::q, T = p::t, D = p::fft_d;
@@ -171,16 +180,24 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
   __syncthreads();
   chain_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t *SP = bsm + LY::shared_u32 + warp * LY::warp_u32;
-  uint32_t *BP = SP + LY::s_words;
   const long long N = seg_rows(segs);
   const long long ngroups = (N + 31) / 32;
   // each block (one per SM) takes an equal contiguous share of the groups and
   // its warps stride over it: with a grid-wide stride, 2048 groups over 152 x 8
   // warps left 48 SMs with half the work of the others
-  const int nwb = blockDim.x >> 5;  // warps per block (a launch parameter up to kBMWarps)
   const long long g_lo = ngroups * blockIdx.x / gridDim.x, g_hi = ngroups * (blockIdx.x + 1) / gridDim.x;
-  for (long long g = g_lo + warp; g < g_hi; g += nwb) {
+  // one or two groups more than a multiple of four: their second half goes to the other two schedulers
+  const int mine = (int)(g_hi - g_lo), base = mine & ~3, extra = mine - base;
+  const bool halves = mine <= nwb && base >= 8 && (extra == 1 || extra == 2) &&
+                      32 * (base + 2 + extra) <= (int)blockDim.x;  // the block has the warps for it
+  const bool second = halves && warp >= base + 2;
+  const int area = second ? warp - 2 : warp;  // the group's index in the block and its shared memory
+  if (area >= nwb || (halves && area >= mine)) return;
+  uint32_t *SP = bsm + LY::shared_u32 + area * LY::warp_u32;
+  uint32_t *BP = SP + LY::s_words;
+  for (long long g = g_lo + area; g < g_hi; g += nwb) {
+    const bool split = halves && area >= base && 32 * (g + 1) <= N;
+    if (second && !split) return;
     const long long op = g * 32 + lane;
     int seg;
     const bool live = op < N && seg_live(segs, op, &seg);
@@ -192,7 +209,8 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
     for (int k = 0; k < NS; k++)
 #pragma unroll
       for (int b = 0; b < M; b++) C[k][b] = 0u;
-    for (int w = lane; w < LY::b_words; w += 32) BP[w] = (w == M) ? 0xFFFFFFFFu : 0u;
+    if (!second)
+      for (int w = lane; w < LY::b_words; w += 32) BP[w] = (w == M) ? 0xFFFFFFFFu : 0u;
     int L = 0, lb = 0;  // this lane's request: LFSR length, log b
     // this lane's request's packed syndromes: `have` bits of the current ones in sbits, word wn next (its value in
     // word_n), of which the planes go to ring word 32 wn mod R M + lane
@@ -202,8 +220,33 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
     int es = (R - 1 - lane) % R;  // ring entry of s_{n-1-lane}
     int eb = 1 + lane;            // ring entry of B_{1+lane}
     int e0 = 0;                   // ring entry of B_0
+    int n = 0;
+    // a split group's registers between its halves, in its rows of Sig: C, L, log b, the syndrome bits
+    uint32_t *save = reinterpret_cast<uint32_t *>(Sig + g * 32 * SIG) + lane;
+    static_assert((NS * M + 5) * 32 * 4 <= 32 * SIG * 2, "the registers fit the rows of 32 locators");
+    constexpr int CUT = 2 * T * kBMCutNum / 16;
+    if (second) {
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + area - base) : "memory");
+#pragma unroll
+      for (int k = 0; k < NS; k++)
+#pragma unroll
+        for (int b = 0; b < M; b++) C[k][b] = save[(k * M + b) * 32];
+      L = (int)save[(NS * M) * 32];
+      lb = (int)save[(NS * M + 1) * 32];
+      sbits = save[(NS * M + 2) * 32] | (uint64_t)save[(NS * M + 3) * 32] << 32;
+      word_n = save[(NS * M + 4) * 32];
+      // the rest follows from n: every syndrome bit below M n is used, in whole words
+      n = CUT;
+      wn = (CUT * M + 31) / 32;
+      have = 32 * wn - CUT * M;
+      fill = (32 * wn + lane) % (R * M);
+      es = (CUT + R - 1 - lane) % R;
+      e0 = (RB - CUT % RB) % RB;
+      eb = (e0 + 1 + lane) % RB;
+    }
+    const int n_end = split && !second ? CUT : 2 * T;
 #pragma unroll 1
-    for (int n = 0; n < 2 * T; n++) {
+    for (; n < n_end; n++) {
       if (have < M) {  // uniform
         SP[fill] = transpose32(word_n, lane);
         fill += 32;
@@ -302,6 +345,20 @@ __global__ void __launch_bounds__(kBMWarps * 32, 1) dec_bm_kernel(const uint32_t
       eb = eb ? eb - 1 : RB - 1;
       es = es + 1 < R ? es + 1 : 0;
       __syncwarp();
+    }
+    if (n_end < 2 * T) {  // the other warp goes on with this group
+#pragma unroll
+      for (int k = 0; k < NS; k++)
+#pragma unroll
+        for (int b = 0; b < M; b++) save[(k * M + b) * 32] = C[k][b];
+      save[(NS * M) * 32] = (uint32_t)L;
+      save[(NS * M + 1) * 32] = (uint32_t)lb;
+      save[(NS * M + 2) * 32] = (uint32_t)sbits;
+      save[(NS * M + 3) * 32] = (uint32_t)(sbits >> 32);
+      save[(NS * M + 4) * 32] = word_n;
+      __threadfence_block();
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + area - base) : "memory");
+      return;
     }
     // sigma(x) = sum_deg C[t-deg] x^deg -> FFT coefficient slots (deg < 2^d);
     // coefficients are < 2^m <= 2^13, so bit 15 of the constant coefficient
@@ -1851,12 +1908,12 @@ cudaError_t launch_dec_bm(const uint32_t *S2, int lds2, FieldDev fd, const Segs 
     return lw <= kBMLatCopyWarps ? launch(dec_bm_lat_kernel<SET, true>) : launch(dec_bm_lat_kernel<SET, false>);
   }
   warps = bm_block_warps(N, warps);
-  const int smem_bm = BMLayout<SET>::bytes(warps);
+  const int smem_bm = BMLayout<SET>::bytes(warps), threads = 32 * std::min((warps + 3) & ~3, kBMBlockWarps);
   cudaError_t err = cudaFuncSetAttribute(dec_bm_kernel<SET>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          BMLayout<SET>::bytes(kBMWarps));
   if (err != cudaSuccess) return err;
-  const int gb = persistent_blocks(dec_bm_kernel<SET>, warps * 32, smem_bm, (N + 31) / 32, warps);
-  return launch_chained(segs, dec_bm_kernel<SET>, gb, warps * 32, smem_bm, st, S2, lds2, fd, segs, Sig);
+  const int gb = persistent_blocks(dec_bm_kernel<SET>, threads, smem_bm, (N + 31) / 32, warps);
+  return launch_chained(segs, dec_bm_kernel<SET>, gb, threads, smem_bm, st, S2, lds2, fd, segs, Sig, warps);
 }
 
 template <int SET, bool CT>

@@ -70,3 +70,31 @@ def test_bm_latency_block_sizes(keys, sid):
         pick = np.arange(n) % base
         k, r = sec.dec_batch(cts[pick])
         assert (k == ref[pick]).all() and (r == rc[pick]).all(), n
+
+
+@pytest.mark.parametrize("sid", range(5), ids=SETS)
+def test_bm_split_groups(keys, sid):
+    """Blocks of the bit-sliced form with 9, 10, 13 and 14 groups of 32 requests, whose last one or two change warps
+    halfway, and with 12, which have none."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import tensormceliece_gb300 as gmc
+
+    pk, sk = keys(sid)
+    z = O.sizes(sid)
+    base = 89
+    cts, _, _ = gmc.PublicKey(sid, pk).enc_batch(request_seeds(sid, base, b"split"))
+    rng = np.random.default_rng(sid)
+    for i in range(0, base, 4):
+        cts[i, rng.integers(0, z["mt"] // 8)] ^= 1 << rng.integers(0, 8)
+    cts[3] = 0
+    cts[7] = 0
+    cts[7, 0] = 2
+    ref, rc = O.dec_batch(sid, sk, cts, threads=THREADS)
+    sec = gmc.SecretKey(sid, sk)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for groups in (9, 10, 12, 13, 14):
+        n = 32 * groups * sms - 300
+        pick = np.arange(n) % base
+        k, r = sec.dec_batch(cts[pick])
+        assert (k == ref[pick]).all() and (r == rc[pick]).all(), groups
