@@ -158,7 +158,7 @@ def algorithmic_bytes(kernel, z, n):
         "dec_pack_ct": ct + (ct + 3) // 4 * 4,
         "dec_front_gemm": (ct + 3) // 4 * 4 + s2,
         "dec_bm": s2 + 2 * (1 << (6 if z["t"] <= 64 else 7)),
-        "dec_fft_roots_reenc": 2 * (1 << (6 if z["t"] <= 64 else 7)) + s2 + ew + 4,
+        "dec_fft_roots_reenc": 2 * (1 << (6 if z["t"] <= 64 else 7)) + ew + 4,
         "dec_tail_hash": ew + 4 + ct + 32 + 4,
     }[kernel]
     fixed = {"enc_syndrome_gemm": z["mt"] * kw, "enc_sample_syndrome": z["k"] * mw,
@@ -180,8 +180,9 @@ def alu_lane_ops(kernel, z):
     i <= min(L, t) and the update C_i += f B_i over i <= min(max(L, n+1-L), t), one GF(2^m) product each, with
     the length profile L = ceil(n/2) of a full-rank syndrome sequence; 32 requests per lane operation.
     dec_fft_roots_reenc: the additive FFT's bottom-up pass, d = log2(2^d >= t) levels of 2^(m-1) butterflies,
-    each one product and two m-plane additions, 32 chunks per lane operation (the top-down pass, the root
-    extraction and the syndrome check are not counted)."""
+    each one product and two m-plane additions, 32 chunks or requests per lane operation (the top-down pass and
+    the root extraction are not counted; the request-sliced form of large batches multiplies by constants, which
+    takes about half of a product's steps)."""
     m, t = z["m"], z["t"]
     if kernel == "dec_bm":
         prods = 0
