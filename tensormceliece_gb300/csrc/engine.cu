@@ -606,11 +606,17 @@ static cudaError_t dec_front_decode_seg(const Segs &segs, const gmc_key *ref, co
   FieldDev fd;
   if (get_field(SET, &fd) != GMC_OK) return cudaErrorUnknown;
   prof_mark(nullptr, st);
-  cudaError_t e = launch_pack_ct<SET>(c, segs, X, d.ldx, pc, st);
-  if (e != cudaSuccess) return e;
-  prof_mark("dec_pack_ct", st);
-  e = launch_gf2_gemm_seg(engine, gk, segs, ref->ldf, ref->frows_pad, X, d.ldx, ref->cw_pad, S2, d.lds2, p::s2w, err,
-                          st);
+  cudaError_t e;
+  // (an engine set by the caller is kept)
+  if (g_engine_override < 0 && seg_live_rows(segs) * p::synd_bytes * p::s2w <= kFrontFewBytes) {
+    e = launch_dec_front_few<SET>(c, segs, gk, ref->ldf, S2, d.lds2, pc, st);
+  } else {
+    e = launch_pack_ct<SET>(c, segs, X, d.ldx, pc, st);
+    if (e != cudaSuccess) return e;
+    prof_mark("dec_pack_ct", st);
+    e = launch_gf2_gemm_seg(engine, gk, segs, ref->ldf, ref->frows_pad, X, d.ldx, ref->cw_pad, S2, d.lds2, p::s2w,
+                            err, st);
+  }
   if (e != cudaSuccess) return e;
   prof_mark("dec_front_gemm", st);
   const SetTune tune = tune_get(SET);

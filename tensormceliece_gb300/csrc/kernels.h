@@ -15,6 +15,12 @@ constexpr int kSampleThreadsMax = 128;  // sampler block size is a launch parame
 // blocks per SM
 constexpr int kTailThreads = 64;
 constexpr int kTailBlocksPerSM = 14;
+constexpr int kFrontFewWarps = 4;  // front end of small batches: warps per block
+// It is taken while live requests x ciphertext bytes x syndrome words, four times what its blocks read of the
+// ciphertexts, stay below this (145 requests of 8192128, 682 of 348864). On device buffers it would win up to about
+// 600 and 1000 requests, but the ciphertexts may lie in host memory: host calls of 8192128 with 128 / 256 / 600
+// requests 121 / 131 / 162 us, against 124 / 126 / 154 with the product, 348864 with 600 requests 89 / 91 us.
+constexpr long long kFrontFewBytes = 3 << 20;
 constexpr int kBMWarps = 14;    // Berlekamp-Massey kernel: default and largest warps per block (32 requests per warp)
 constexpr int kBMBlockWarps = 16;  // its block: the warps that finish split groups are in addition
 constexpr int kBMCutNum = 11;      // a split group changes warps after this many sixteenths of its iterations
@@ -227,6 +233,10 @@ struct DecKeys {
 // C rows of synd_bytes (+ 32 with pc); only C0 is packed.
 template <int SET>
 cudaError_t launch_pack_ct(const uint8_t *C, const Segs &segs, uint32_t *X, int ldx, bool pc, cudaStream_t st);
+// The 2t packed syndromes of a small batch from the ciphertext bytes (keys.A: the secret keys' F, rows of ldf words).
+template <int SET>
+cudaError_t launch_dec_front_few(const uint8_t *C, const Segs &segs, const GemmKeys &keys, int ldf, uint32_t *S2,
+                                 int lds2, bool pc, cudaStream_t st);
 // Berlekamp-Massey: S2 (2t packed syndromes) -> Sig [N][2^fft_d] u16, the
 // error locator's coefficients by degree (the leading x^t term is implicit
 // when t = 2^fft_d).

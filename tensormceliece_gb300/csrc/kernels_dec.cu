@@ -64,6 +64,73 @@ __global__ void pack_ct_kernel(const uint8_t *__restrict__ C, const Segs segs, u
   X[op * ldx + w] = v;
 }
 
+// ---------------------------------------------------------------- front end of small batches
+// The syndromes S2 = F C0 of a few live requests (kFrontFewBytes) straight from
+// the ciphertext bytes: a warp holds 32 rows of F (lane = row, the whole row
+// in registers) and goes through 16 requests whose words a block shares; a word
+// costs one LOP3 (acc ^= a & x) and the 32 parities of a request are one ballot.
+// Packing the ciphertexts and the tensor-core product take two launches, and
+// the product's tiles of 128 requests a fixed time: 8192128 20.6 us for up to
+// 1000 requests, against 6.1 for one request here, 8.1 for 64 and 11 for 256 (348864
+// 16.5, against 6.0, 6.4 and 7.5). Bound by the load of the rows and the launch.
+template <int SET, bool PC>
+__global__ void __launch_bounds__(kFrontFewWarps * 32) dec_front_few_kernel(const uint8_t *__restrict__ C, const Segs segs,
+                                                                           const GemmKeys keys, int ldf,
+                                                                           uint32_t *__restrict__ S2, int lds2) {
+  using p = P<SET>;
+  constexpr int CB = p::synd_bytes + (PC ? 32 : 0);  // ciphertext row bytes
+  constexpr int U = (p::synd_bytes + 15) / 16;       // 16-byte units of a row
+  constexpr int NW = p::s2w, RG = (NW + kFrontFewWarps - 1) / kFrontFewWarps, OPS = 16;
+  __shared__ __align__(16) uint32_t xs[OPS][4 * U];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  chain_trigger();
+  const long long op0 = (long long)(blockIdx.x / RG) * OPS;  // 16 rows never straddle segments
+  const int seg = seg_find(segs, op0);
+  const long long nlive = segs.row0[seg] + segs.nreq[seg] - op0;
+  if (nlive <= 0) return;
+  const int live = nlive < OPS ? (int)nlive : OPS;
+  const int w = blockIdx.x % RG * kFrontFewWarps + warp;  // word of the syndromes: rows 32 w .. 32 w + 31
+  uint4 a[U];
+  if (w < NW) {
+    const uint4 *row = reinterpret_cast<const uint4 *>(keys.A[seg] + (size_t)(32 * w + lane) * ldf);
+#pragma unroll
+    for (int u = 0; u < U; u++) a[u] = row[u];
+  }
+  // ciphertext rows on 4-byte boundaries (they may lie in host memory: few loads)
+  const bool words = p::synd_bytes % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 3) == 0;
+  for (int i = threadIdx.x; i < live * 4 * U; i += kFrontFewWarps * 32) {
+    const int r = i / (4 * U), x = i % (4 * U);
+    const uint8_t *c = C + (op0 + r) * CB;
+    uint32_t v = 0;
+    if (words) {
+      if (4 * x < p::synd_bytes) v = reinterpret_cast<const uint32_t *>(c)[x];
+    } else {
+#pragma unroll
+      for (int b = 0; b < 4; b++)
+        if (4 * x + b < p::synd_bytes) v |= (uint32_t)c[4 * x + b] << (8 * b);
+    }
+    xs[r][x] = v;
+  }
+  __syncthreads();
+  if (w >= NW) return;
+  uint32_t mine = 0;
+#pragma unroll 2
+  for (int r = 0; r < live; r++) {
+    uint32_t acc[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const uint4 x = reinterpret_cast<const uint4 *>(xs[r])[u];
+      acc[0] ^= a[u].x & x.x;
+      acc[1] ^= a[u].y & x.y;
+      acc[2] ^= a[u].z & x.z;
+      acc[3] ^= a[u].w & x.w;
+    }
+    const uint32_t par = __ballot_sync(0xffffffffu, __popc(acc[0] ^ acc[1] ^ acc[2] ^ acc[3]) & 1);
+    if (lane == r) mine = par;
+  }
+  if (lane < live) S2[(op0 + lane) * lds2 + w] = mine;
+}
+
 // ---------------------------------------------------------------- BM
 // One warp per group of 32 requests, bit-sliced: bit q of every word belongs
 // to request 32g + q, and a GF(2^m) value of all 32 requests is m words
@@ -1848,6 +1915,20 @@ cudaError_t launch_pack_ct(const uint8_t *C, const Segs &segs, uint32_t *X, int 
   return cudaGetLastError();
 }
 
+template <int SET>
+cudaError_t launch_dec_front_few(const uint8_t *C, const Segs &segs, const GemmKeys &keys, int ldf, uint32_t *S2,
+                                 int lds2, bool pc, cudaStream_t st) {
+  const long long N = seg_rows(segs);
+  if (N <= 0) return cudaSuccess;
+  constexpr int RG = (P<SET>::s2w + kFrontFewWarps - 1) / kFrontFewWarps;
+  const unsigned blocks = (unsigned)((N + 15) / 16 * RG);
+  if (pc)
+    dec_front_few_kernel<SET, true><<<blocks, kFrontFewWarps * 32, 0, st>>>(C, segs, keys, ldf, S2, lds2);
+  else
+    dec_front_few_kernel<SET, false><<<blocks, kFrontFewWarps * 32, 0, st>>>(C, segs, keys, ldf, S2, lds2);
+  return cudaGetLastError();
+}
+
 template <typename K>
 static int persistent_blocks(K kernel, int threads, int smem, long long work_items, int items_per_block) {
   int dev = 0, sms = 0, per_sm = 0;
@@ -2117,6 +2198,8 @@ size_t dec_root_work_bytes(int set, long long rows, bool ct) {
 
 #define GMC_INST_DEC(SET)                                                                                       \
   template cudaError_t launch_pack_ct<SET>(const uint8_t *, const Segs &, uint32_t *, int, bool, cudaStream_t);       \
+  template cudaError_t launch_dec_front_few<SET>(const uint8_t *, const Segs &, const GemmKeys &, int, uint32_t *, int, \
+                                                 bool, cudaStream_t);                                            \
   template cudaError_t launch_dec_bm<SET>(const uint32_t *, int, FieldDev, const Segs &, uint16_t *,             \
                                          cudaStream_t, int, bool);                                               \
   template cudaError_t launch_dec_root<SET>(const uint16_t *, const DecKeys &, FieldDev, const Segs &,          \
