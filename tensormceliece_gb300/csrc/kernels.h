@@ -7,6 +7,11 @@
 namespace gmc {
 
 constexpr int kSampleWarpsPerSM = 8;     // sampler: resident warps per SM (lanes fetch requests)
+// Sampler: requests per SM up to which a request gets a block (P Keccak blocks per attempt; full: n = 2^m, where an
+// attempt fails twice as often and the chains are longer). us, block per request / pairs and groups: 348864 (P = 2) 608
+// requests 36 / 44, 2000 55 / 61, 3001 73 / 71; 460896 (P = 3) 608 63 / 80, 2000 100 / 101; 6960119 (P = 4) 608
+// 87 / 113, 1200 108 / 119, 3001 165 / 130; 8192128 (P = 2, full) 608 75 / 109, 3001 98 / 122, 4500 116 / 131.
+constexpr int sample_few_per_sm(int perms, bool full) { return full ? 30 : 36 / perms; }
 constexpr int kSamplePipeWarps = 16;     // pipelined sampler: resident warps per SM unless tuned
 constexpr int kSampleGroupWarps = 2;     // its groups: warps per scheduler before a warp gets a further group
 constexpr int kSampleThreadsMax = 128;  // sampler block size is a launch parameter (32, 64 or 128)

@@ -18,8 +18,8 @@ namespace gmc {
 // bits; for n < 2^m the first t values below n are kept, else all t. A
 // repeated position rejects the attempt (only the set of positions matters,
 // as in the library's sort-and-compare).
-// Two forms: sample_pipe_kernel (below, the default) and this lane-per-request
-// sample_kernel (GMC_SAMPLE_PIPELINE=0), which share the check and gather steps.
+// Forms: sample_pipe_kernel and, for small batches, sample_few_kernel (below, the
+// defaults), and this lane-per-request sample_kernel (GMC_SAMPLE_PIPELINE=0).
 // Work split: each lane owns one request and runs its Keccak chain; lanes
 // take requests from a launch-wide counter whenever their previous request
 // is done, so a request that needs many attempts does not hold the warp's
@@ -281,6 +281,135 @@ struct PipeLayout {
   static_assert(raw_words <= 17 * perms && raw_words > 17 * (perms - 1) && raw_words > 4, "pipeline geometry");
 };
 
+// A complete attempt's candidates in raw (a warp, uniform arguments): filter, first t kept, repeats; a success writes e
+// (and e[mt:n] or the syndrome). bm is all zero before and after.
+template <int SET, bool SPARSE>
+__device__ __forceinline__ bool check_attempt(const uint16_t *raw, uint32_t *bm, uint16_t *cand, int lane,
+                                              uint32_t *__restrict__ E, int lde, uint32_t *__restrict__ Ens, int ldx,
+                                              const GemmKeys &keys, uint32_t *__restrict__ S, int lds, long long opr,
+                                              int seg) {
+  using p = P<SET>;
+  constexpr int NCW = (p::t + 31) / 32, ncand = p::cand_bytes / 2;
+  constexpr uint32_t mask = p::q - 1;
+  constexpr int sh = p::mt % 32, w0 = p::mt / 32;
+  if constexpr (!p::full) {
+    int total = 0;
+#pragma unroll
+    for (int base = 0; base < ncand; base += 32) {
+      const int i = base + lane;
+      uint32_t v = 0;
+      bool keep = false;
+      if (i < ncand) {
+        v = raw[i] & mask;
+        keep = v < (uint32_t)p::n;
+      }
+      const uint32_t bal = __ballot_sync(0xffffffffu, keep);
+      const int idx = total + __popc(bal & ((1u << lane) - 1));
+      if (keep && idx < p::t) cand[idx] = (uint16_t)v;
+      total += __popc(bal);
+    }
+    __syncwarp();
+    if (total < p::t) return false;  // too few candidates below n (warp-uniform)
+  }
+  auto pos_of = [&](int c) -> int { return p::full ? (int)(raw[c] & mask) : (int)cand[c]; };
+  uint32_t vv[NCW];
+  bool dup = false;
+#pragma unroll
+  for (int i = 0; i < NCW; i++) {
+    const int c = lane + 32 * i;
+    vv[i] = 0xFFFFFFFFu;
+    if (c < p::t) {
+      const uint32_t v = (uint32_t)pos_of(c);
+      vv[i] = v;
+      const uint32_t bit = 1u << (v & 31);
+      dup |= (atomicOr(&bm[v >> 5], bit) & bit) != 0;
+    }
+  }
+  const bool good = !__any_sync(0xffffffffu, dup);
+  if (good) {
+    uint32_t *erow = E + opr * lde;
+    for (int w = lane; w < p::ew; w += 32) erow[w] = bm[w];
+    if (SPARSE) {
+      sparse_syndrome_row<SET>(pos_of, keys.TT[seg], keys.ldtt, S + opr * lds, lane);
+    } else {
+      uint32_t *xrow = Ens + opr * ldx;
+      for (int w = lane; w < p::kw; w += 32) {
+        const uint32_t lo = bm[w0 + w];
+        const uint32_t hi = (w0 + w + 1 < p::ew) ? bm[w0 + w + 1] : 0u;
+        xrow[w] = sh ? ((lo >> sh) | (hi << (32 - sh))) : lo;
+      }
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < NCW; i++)
+    if (vv[i] != 0xFFFFFFFFu) bm[vv[i] >> 5] = 0;
+  __syncwarp();
+  return good;
+}
+
+// A block per request, for batches that leave most of the GPU idle: a warp per
+// block of an attempt, each on a whole Keccak state (KeccakWarp), and one that
+// checks. At step s warp r permutes block r of attempt s - r, warp 0 the seed chain
+// and each other warp the state that warp r - 1 left a step earlier; the last warp
+// checks attempt s - P, complete since the step before. A step is one permutation
+// of 24 x 207 cycles and a barrier, against about 9000 cycles in the kernels above,
+// at six times their instructions. 256 requests: 348864 34 us against 43, 6960119
+// 83 / 112, 8192128 74 / 108; the line to those forms: sample_few_per_sm.
+template <int SET, bool SPARSE>
+__global__ void __launch_bounds__((PipeLayout<SET>::perms + 1) * 32)
+    sample_few_kernel(const uint8_t *__restrict__ seeds, const Segs segs, uint32_t *__restrict__ E, int lde,
+                      uint32_t *__restrict__ Ens, int ldx, const GemmKeys keys, uint32_t *__restrict__ S, int lds) {
+  using p = P<SET>;
+  using LY = PipeLayout<SET>;
+  constexpr int PP = LY::perms, RW = LY::raw_words, SLOTS = PP + 1;
+  __shared__ __align__(16) uint64_t raw[SLOTS][LY::slot_words], state[PP][2][25];
+  __shared__ uint32_t bm[LY::bm_words];
+  __shared__ uint16_t cand[p::t];
+  __shared__ int done;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  chain_trigger();
+  const long long op = blockIdx.x;
+  int seg;
+  if (!seg_live(segs, op, &seg)) return;
+  for (int w = threadIdx.x; w < LY::bm_words; w += SLOTS * 32) bm[w] = 0;
+  if (threadIdx.x == 0) done = 0;
+  uint64_t st = 0;  // warp 0: word `lane` of the current attempt's state (lanes 0 .. 3)
+  if (warp == 0 && lane < 4) {
+    const uint8_t *sd = seeds + 32 * op + 8 * lane;
+#pragma unroll
+    for (int b = 0; b < 8; b++) st |= (uint64_t)sd[b] << (8 * b);
+  }
+  const KeccakWarp kw(lane);
+  __syncthreads();
+#pragma unroll 1
+  for (int s = 0;; s++) {
+    const int j = s - warp;  // the attempt this warp works on
+    if (j >= 0) {
+      if (warp < PP) {
+        uint64_t a;
+        if (warp == 0) {  // absorb {64} || state
+          const uint64_t below = __shfl_up_sync(0xffffffffu, st, 1);
+          a = lane < 4 ? st << 8 : lane == 4 ? 0x1F00ull : lane == 16 ? 0x8000000000000000ull : 0ull;
+          if (lane <= 4) a |= lane ? below >> 56 : 64ull;
+        } else {
+          a = state[warp - 1][(s - 1) & 1][lane < 25 ? lane : 0];
+        }
+        kw.permute(a);
+        if (warp == 0) st = a;
+        const int w = 17 * warp + lane;
+        if (lane < 17 && w < RW) raw[j % SLOTS][w] = a;
+        if (warp + 1 < PP && lane < 25) state[warp][s & 1][lane] = a;
+      } else if (check_attempt<SET, SPARSE>(reinterpret_cast<const uint16_t *>(raw[j % SLOTS]), bm, cand, lane, E, lde,
+                                            Ens, ldx, keys, S, lds, op, seg)) {
+        if (lane == 0) done = 1;
+      }
+    }
+    __syncthreads();
+    if (done) break;
+  }
+}
+
 // groups = 0: pair per request first, then the warp's last requests as groups; else only groups, at most `groups`
 // per warp
 template <int SET, bool SPARSE>
@@ -371,64 +500,9 @@ __global__ void __launch_bounds__(kSampleThreadsMax)
       if (w < RW) dst[2 * w] = A[i];
     }
   };
-  // one complete attempt in `slot` (warp-uniform arguments): filter, first t kept, repeats; a success writes e (and
-  // e[mt:n] or the syndrome)
   auto check = [&](int slot, long long opr, int seg) -> bool {
-    const uint16_t *raw = reinterpret_cast<const uint16_t *>(ring + (size_t)slot * LY::slot_words * 2);
-    if constexpr (!p::full) {
-      int total = 0;
-#pragma unroll
-      for (int base = 0; base < ncand; base += 32) {
-        const int i = base + lane;
-        uint32_t v = 0;
-        bool keep = false;
-        if (i < ncand) {
-          v = raw[i] & mask;
-          keep = v < (uint32_t)p::n;
-        }
-        const uint32_t bal = __ballot_sync(0xffffffffu, keep);
-        const int idx = total + __popc(bal & ((1u << lane) - 1));
-        if (keep && idx < p::t) cand[idx] = (uint16_t)v;
-        total += __popc(bal);
-      }
-      __syncwarp();
-      if (total < p::t) return false;  // too few candidates below n (warp-uniform)
-    }
-    auto pos_of = [&](int c) -> int { return p::full ? (int)(raw[c] & mask) : (int)cand[c]; };
-    uint32_t vv[NCW];
-    bool dup = false;
-#pragma unroll
-    for (int i = 0; i < NCW; i++) {
-      const int c = lane + 32 * i;
-      vv[i] = 0xFFFFFFFFu;
-      if (c < p::t) {
-        const uint32_t v = (uint32_t)pos_of(c);
-        vv[i] = v;
-        const uint32_t bit = 1u << (v & 31);
-        dup |= (atomicOr(&bm[v >> 5], bit) & bit) != 0;
-      }
-    }
-    const bool good = !__any_sync(0xffffffffu, dup);
-    if (good) {
-      uint32_t *erow = E + opr * lde;
-      for (int w = lane; w < p::ew; w += 32) erow[w] = bm[w];
-      if (SPARSE) {
-        sparse_syndrome_row<SET>(pos_of, keys.TT[seg], keys.ldtt, S + opr * lds, lane);
-      } else {
-        uint32_t *xrow = Ens + opr * ldx;
-        for (int w = lane; w < p::kw; w += 32) {
-          const uint32_t lo = bm[w0 + w];
-          const uint32_t hi = (w0 + w + 1 < p::ew) ? bm[w0 + w + 1] : 0u;
-          xrow[w] = sh ? ((lo >> sh) | (hi << (32 - sh))) : lo;
-        }
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < NCW; i++)
-      if (vv[i] != 0xFFFFFFFFu) bm[vv[i] >> 5] = 0;
-    __syncwarp();
-    return good;
+    return check_attempt<SET, SPARSE>(reinterpret_cast<const uint16_t *>(ring + (size_t)slot * LY::slot_words * 2), bm,
+                                      cand, lane, E, lde, Ens, ldx, keys, S, lds, opr, seg);
   };
 
   bool exhausted = false;
@@ -774,6 +848,13 @@ static cudaError_t launch_sample_mode(const uint8_t *seeds, const Segs &segs, ui
   // further group (8192128, 3001 requests, one / two warps: 142 / 124 us)
   if (sample_pipelined()) {
     using PL = PipeLayout<SET>;
+    if (seg_live_rows(segs) <= (long long)sample_few_per_sm(PL::perms, P<SET>::full) * sms) {
+      sample_few_kernel<SET, SPARSE><<<(unsigned)N, (PL::perms + 1) * 32, 0, st>>>(seeds, segs, E, lde, Ens, ldx, keys, S,
+                                                                                   lds);
+      err = cudaGetLastError();
+      if (mark) mark(SPARSE ? "enc_sample_syndrome" : "enc_sample", st);
+      return err;
+    }
     auto kern = sample_pipe_kernel<SET, SPARSE>;
     const int psmem = warps * PL::warp_bytes;
     err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
