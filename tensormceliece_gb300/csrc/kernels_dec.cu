@@ -2042,8 +2042,9 @@ cudaError_t launch_dec_root(const uint16_t *Sig, const DecKeys &keys, FieldDev f
   if (N <= 0) return cudaSuccess;
   if (warps < 0 || warps > kRootWarps) return cudaErrorInvalidValue;
   if (warps == 0) warps = kRootWarps;
-  if (work && dec_root_work_bytes(SET, N, ct)) {
-    if (!fd.fft_alpha || lde % 4) return cudaErrorInvalidValue;
+  // (rows of E are written in 16-byte units)
+  if (work && dec_root_work_bytes(SET, N, ct) && lde % 4 == 0 && (reinterpret_cast<uintptr_t>(E) & 15) == 0) {
+    if (!fd.fft_alpha) return cudaErrorInvalidValue;
     return launch_dec_root_sliced<SET>(Sig, keys, fd, segs, E, lde, ok, st, work);
   }
   if (ct) {

@@ -37,3 +37,32 @@ def test_sliced_roots(keys, sid):
         pick = np.arange(n) % base
         k, r = sec.dec_batch(cts[pick])
         assert (k == ref[pick]).all() and (r == rc[pick]).all(), n
+
+
+def test_sliced_roots_stage_rows_at_any_word(keys):
+    """Error-vector rows of the caller that start between 16-byte boundaries (the stage outputs take any word)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import tensormceliece_gb300 as gmc
+
+    sid = 0
+    pk, sk = keys(sid)
+    z = O.sizes(sid)
+    cts, _, _ = gmc.PublicKey(sid, pk).enc_batch(request_seeds(sid, 50, b"rows"))
+    n = FIRST + 1
+    d_c = torch.from_numpy(cts[np.arange(n) % 50]).cuda()
+    lds2 = ((2 * z["t"] * z["m"] + 31) // 32 + 3) // 4 * 4
+    lde = ((z["n"] + 31) // 32 + 3) // 4 * 4
+    sec = gmc.SecretKey(sid, sk)
+    rows = []
+    for off in (0, 1):
+        s2 = torch.zeros(n * lds2 + 1, dtype=torch.int32, device="cuda")
+        e = torch.zeros(n * lde + 1, dtype=torch.int32, device="cuda")
+        ok = torch.zeros(n, dtype=torch.int32, device="cuda")
+        assert gmc.lib().gmc_dec_stages_dev(sec.handle, d_c.data_ptr(), n, s2.data_ptr() + 4 * off, lds2,
+                                            e.data_ptr() + 4 * off, lde, ok.data_ptr(), 0) == 0
+        torch.cuda.synchronize()
+        assert int(ok.sum()) == n
+        words = (z["n"] + 31) // 32
+        rows.append(e[off : off + n * lde].view(n, lde)[:, :words].cpu())
+    assert torch.equal(rows[0], rows[1])
