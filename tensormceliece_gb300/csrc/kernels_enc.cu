@@ -829,14 +829,23 @@ static cudaError_t launch_sample_mode(const uint8_t *seeds, const Segs &segs, ui
                                      unsigned int *counter, cudaStream_t st, int sample_sm_warps,
                                      void (*mark)(const char *, cudaStream_t)) {
   const long long N = seg_rows(segs);
-  const int smem = (threads / 32) * SampleLayout<SET>::warp_bytes;
-  cudaError_t err = cudaFuncSetAttribute(sample_kernel<SET, SPARSE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (kSampleThreadsMax / 32) * SampleLayout<SET>::warp_bytes);
-  if (err != cudaSuccess) return err;
-  if ((err = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st)) != cudaSuccess) return err;
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaError_t err;
+  constexpr int PP = PipeLayout<SET>::perms;
+  if (sample_pipelined() && seg_live_rows(segs) <= (long long)sample_few_per_sm(PP, P<SET>::full) * sms) {
+    sample_few_kernel<SET, SPARSE>
+        <<<(unsigned)N, (PP + 1) * 32, 0, st>>>(seeds, segs, E, lde, Ens, ldx, keys, S, lds);
+    err = cudaGetLastError();
+    if (mark) mark(SPARSE ? "enc_sample_syndrome" : "enc_sample", st);
+    return err;
+  }
+  const int smem = (threads / 32) * SampleLayout<SET>::warp_bytes;
+  err = cudaFuncSetAttribute(sample_kernel<SET, SPARSE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (kSampleThreadsMax / 32) * SampleLayout<SET>::warp_bytes);
+  if (err != cudaSuccess) return err;
+  if ((err = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st)) != cudaSuccess) return err;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sample_kernel<SET, SPARSE>, threads, smem);
   if (per_sm < 1) per_sm = 1;
   // fewer lanes than requests: a lane that finishes early takes further
@@ -848,13 +857,6 @@ static cudaError_t launch_sample_mode(const uint8_t *seeds, const Segs &segs, ui
   // further group (8192128, 3001 requests, one / two warps: 142 / 124 us)
   if (sample_pipelined()) {
     using PL = PipeLayout<SET>;
-    if (seg_live_rows(segs) <= (long long)sample_few_per_sm(PL::perms, P<SET>::full) * sms) {
-      sample_few_kernel<SET, SPARSE><<<(unsigned)N, (PL::perms + 1) * 32, 0, st>>>(seeds, segs, E, lde, Ens, ldx, keys, S,
-                                                                                   lds);
-      err = cudaGetLastError();
-      if (mark) mark(SPARSE ? "enc_sample_syndrome" : "enc_sample", st);
-      return err;
-    }
     auto kern = sample_pipe_kernel<SET, SPARSE>;
     const int psmem = warps * PL::warp_bytes;
     err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
