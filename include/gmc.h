@@ -301,7 +301,8 @@ int gmc_get_dec_constant_time(void);
  * (gemm_stages 2..4 A/X buffers per CTA, default 4) and the requests per block
  * of the decoding kernels (bm_warps: Berlekamp-Massey warps of 32 requests,
  * 1..14, default 14, not used by the constant-time form; root_warps:
- * root-finding warps of one request, 1..8, default 8) and the
+ * root-finding warps of one request, 1..8, default 8, for batches below
+ * 14000 rows) and the
  * pipelined sampler's resident warps per SM (sample_sm_warps, 0 = the
  * default, 16); gmc_tune_set_launch / gmc_tune_get_launch set and read
  * them by hand. */
