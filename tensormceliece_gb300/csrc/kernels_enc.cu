@@ -366,14 +366,12 @@ __global__ void __launch_bounds__((PipeLayout<SET>::perms + 1) * 32)
   __shared__ __align__(16) uint64_t raw[SLOTS][LY::slot_words], state[PP][2][25];
   __shared__ uint32_t bm[LY::bm_words];
   __shared__ uint16_t cand[p::t];
-  __shared__ int done;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   chain_trigger();
   const long long op = blockIdx.x;
   int seg;
   if (!seg_live(segs, op, &seg)) return;
   for (int w = threadIdx.x; w < LY::bm_words; w += SLOTS * 32) bm[w] = 0;
-  if (threadIdx.x == 0) done = 0;
   uint64_t st = 0;  // warp 0: word `lane` of the current attempt's state (lanes 0 .. 3)
   if (warp == 0 && lane < 4) {
     const uint8_t *sd = seeds + 32 * op + 8 * lane;
@@ -385,6 +383,7 @@ __global__ void __launch_bounds__((PipeLayout<SET>::perms + 1) * 32)
 #pragma unroll 1
   for (int s = 0;; s++) {
     const int j = s - warp;  // the attempt this warp works on
+    int good = 0;
     if (j >= 0) {
       if (warp < PP) {
         uint64_t a;
@@ -400,13 +399,14 @@ __global__ void __launch_bounds__((PipeLayout<SET>::perms + 1) * 32)
         const int w = 17 * warp + lane;
         if (lane < 17 && w < RW) raw[j % SLOTS][w] = a;
         if (warp + 1 < PP && lane < 25) state[warp][s & 1][lane] = a;
-      } else if (check_attempt<SET, SPARSE>(reinterpret_cast<const uint16_t *>(raw[j % SLOTS]), bm, cand, lane, E, lde,
-                                            Ens, ldx, keys, S, lds, op, seg)) {
-        if (lane == 0) done = 1;
+      } else {
+        good = check_attempt<SET, SPARSE>(reinterpret_cast<const uint16_t *>(raw[j % SLOTS]), bm, cand, lane, E, lde,
+                                          Ens, ldx, keys, S, lds, op, seg);
       }
     }
-    __syncthreads();
-    if (done) break;
+    // every warp leaves after the same step: a flag in shared memory could be set by the checking warp's next step
+    // before a late warp has read it
+    if (__syncthreads_or(good)) break;
   }
 }
 
