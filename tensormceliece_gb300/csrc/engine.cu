@@ -608,7 +608,7 @@ static cudaError_t dec_front_decode_seg(const Segs &segs, const gmc_key *ref, co
   prof_mark(nullptr, st);
   cudaError_t e;
   // (an engine set by the caller is kept)
-  if (g_engine_override < 0 && seg_live_rows(segs) * p::synd_bytes * p::s2w <= kFrontFewBytes) {
+  if (g_engine_override < 0 && dec_front_few_form(SET, segs)) {
     e = launch_dec_front_few<SET>(c, segs, gk, ref->ldf, S2, d.lds2, pc, st);
   } else {
     e = launch_pack_ct<SET>(c, segs, X, d.ldx, pc, st);

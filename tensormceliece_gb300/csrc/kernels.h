@@ -171,6 +171,12 @@ cudaError_t launch_gf2_gemm_b1(const GemmKeys &keys, const Segs &segs, int lda, 
 Segs one_segment(long long n);
 // hash kernels: whether a launch takes a warp per request (kernels_enc.cu)
 bool hash_warp_form(const Segs &segs);
+// the forms that a batch takes, shared by the launchers and the autotuner (which times only parameters that its
+// batch's forms read): the block-per-request sampler (kernels_enc.cu), the front end of a few decapsulations
+// (kernels_dec.cu; not with an engine set by the caller) and the bit-sliced Berlekamp-Massey
+bool sample_few_form(int set, const Segs &segs);
+bool dec_front_few_form(int set, const Segs &segs);
+bool dec_bm_bitsliced_form(int set, long long rows, bool ct);
 
 // Encapsulation: seeds / C / K rows in padded row space; E, Ens, S have
 // seg_rows(segs) rows. pk_bad_mask bit s: segment s's public key has

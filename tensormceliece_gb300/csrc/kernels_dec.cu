@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "host_keys.h"
 #include "kernels.h"
 #include "device_common.cuh"
 
@@ -1968,7 +1969,7 @@ cudaError_t launch_dec_bm(const uint32_t *S2, int lds2, FieldDev fd, const Segs 
     return launch_chained(segs, dec_bm_ct_kernel<SET>, (unsigned)((N + 31) / 32), (LY::NS + 1) * 32, LY::bytes, st, S2, lds2,
                           segs, Sig);
   }
-  if (N < bm_bitsliced_min_rows(P<SET>::t)) {  // small batch: warp per request (lower latency per request)
+  if (!dec_bm_bitsliced_form(SET, N, ct)) {  // small batch: warp per request (lower latency per request)
     // warps per block: as few rounds over two blocks per SM as kBMLatWarps
     // allows, all of them full
     int dev = 0, sms = 0;
@@ -2180,6 +2181,15 @@ cudaError_t launch_dec_tail(const uint32_t *E, int lde, const int *ok, const uin
               : launch(dec_tail_kernel<SET, false, true>, kTailThreads / 32);
   return pc ? launch(dec_tail_kernel<SET, true, false>, kTailThreads / 2)
             : launch(dec_tail_kernel<SET, false, false>, kTailThreads / 2);
+}
+
+bool dec_front_few_form(int set, const Segs &segs) {
+  const gmc_setinfo &S = set_info(set);
+  return seg_live_rows(segs) * S.synd_bytes * ((2 * S.t * S.m + 31) / 32) <= kFrontFewBytes;
+}
+
+bool dec_bm_bitsliced_form(int set, long long rows, bool ct) {
+  return !ct && rows >= bm_bitsliced_min_rows(set_info(set).t);
 }
 
 // scratch of the request-sliced root finder, 0 where the batch takes the chunk-sliced one

@@ -6,6 +6,7 @@
 // mc:crypto_kem/348864/vec/encrypt.c:41-132, kem_enc.c:18).
 #include <stdlib.h>
 
+#include "host_keys.h"
 #include "kernels.h"
 #include "device_common.cuh"
 
@@ -823,6 +824,16 @@ static bool sample_pipelined() {
   }();
   return on;
 }
+// whether a batch takes the block-per-request sampler (which has no tuned parameters)
+bool sample_few_form(int set, const Segs &segs) {
+  const gmc_setinfo &S = set_info(set);
+  const bool full = S.n == S.q;
+  const int perms = ((full ? 2 : 4) * S.t + 135) / 136;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sample_pipelined() && seg_live_rows(segs) <= (long long)sample_few_per_sm(perms, full) * sms;
+}
 template <int SET, bool SPARSE>
 static cudaError_t launch_sample_mode(const uint8_t *seeds, const Segs &segs, uint32_t *E, int lde, uint32_t *Ens,
                                      int ldx, const GemmKeys &keys, uint32_t *S, int lds, int threads,
@@ -834,7 +845,7 @@ static cudaError_t launch_sample_mode(const uint8_t *seeds, const Segs &segs, ui
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaError_t err;
   constexpr int PP = PipeLayout<SET>::perms;
-  if (sample_pipelined() && seg_live_rows(segs) <= (long long)sample_few_per_sm(PP, P<SET>::full) * sms) {
+  if (sample_few_form(SET, segs)) {
     sample_few_kernel<SET, SPARSE>
         <<<(unsigned)N, (PP + 1) * 32, 0, st>>>(seeds, segs, E, lde, Ens, ldx, keys, S, lds);
     err = cudaGetLastError();

@@ -11,8 +11,10 @@
 // pipeline depth (2, 3 or 4 A/X stages per CTA, when either op uses that
 // engine); and the requests per block of the two decoding kernels
 // (Berlekamp-Massey: at most 14, 8 or 4 warps of 32 requests per block, fewer
-// when the groups spread over every SM with fewer, timed only when the batch
-// takes its bit-sliced form; root finding: 8, 4 or 2 warps of one request).
+// when the groups spread over every SM with fewer; root finding: 8, 4 or 2
+// warps of one request). A parameter is timed only when the batch takes a form
+// that reads it (sample_few_form and its neighbours in kernels.h); else it
+// keeps its value.
 // The GEMM tile is fixed at 128 x 256 (one tcgen05 M=128 instruction shape
 // and a TMEM accumulator pair) and K is never split: every CTA owns whole
 // output tiles, so there is no split-K reduction to tune. A later candidate
@@ -229,23 +231,28 @@ extern "C" int gmc_autotune(int set, long long n, const char *cache_path) {
     const int enc_engines[2] = {GEMM_SPARSE, GEMM_TC};
     const int engines[2] = {GEMM_POPC, GEMM_TC};
     const int threads[3] = {32, 64, 128};
+    // small batches take forms of the sampler and the front end that read neither the block size, the resident
+    // warps nor the engine: the values other batch sizes use stay as they are
+    const Segs segs = one_segment(n);
+    const bool enc_few = sample_few_form(set, segs), dec_few = dec_front_few_form(set, segs);
+    const bool const_time = dec_constant_time();
     for (int ei = 0; ei < 2; ei++)
-      for (int ti = 0; ti < 3; ti++) {
+      for (int ti = 0; ti < (enc_few ? 1 : 3); ti++) {
         SetTune t = best;
         t.enc_engine = enc_engines[ei];
-        t.sample_threads = threads[ti];
+        if (!enc_few) t.sample_threads = threads[ti];
         tune_put(set, t);
         const float ms =
             time_median([&] { return gmc_enc_batch_dev(P, ct, key, seeds, n, nullptr, st); }, st, a, b, &rc);
         if (ms < best_enc) {
           best_enc = ms;
-          best.enc_engine = enc_engines[ei];
-          best.sample_threads = threads[ti];
+          best.enc_engine = t.enc_engine;
+          best.sample_threads = t.sample_threads;
         }
       }
     // resident warps per SM of the pipelined sampler (0: the default, 16)
     const int smw[2] = {0, 8};
-    for (int wi = 1; wi < 2; wi++) {
+    for (int wi = 1; wi < 2 && !enc_few; wi++) {
       SetTune t = best;
       t.sample_sm_warps = smw[wi];
       tune_put(set, t);
@@ -258,14 +265,14 @@ extern "C" int gmc_autotune(int set, long long n, const char *cache_path) {
     }
     tune_put(set, best);
     rc |= gmc_enc_batch_dev(P, ct, key, seeds, n, nullptr, st);  // valid ciphertexts for the dec timing
-    for (int ei = 0; ei < 2; ei++) {
+    for (int ei = 0; ei < (dec_few ? 1 : 2); ei++) {
       SetTune t = best;
-      t.dec_engine = engines[ei];
+      if (!dec_few) t.dec_engine = engines[ei];
       tune_put(set, t);
       const float ms = time_median([&] { return gmc_dec_batch_dev(K, key2, ct, n, nullptr, st); }, st, a, b, &rc);
       if (ms < best_dec) {
         best_dec = ms;
-        best.dec_engine = engines[ei];
+        best.dec_engine = t.dec_engine;
       }
     }
     auto time_dec = [&](const SetTune &t) {
@@ -273,7 +280,8 @@ extern "C" int gmc_autotune(int set, long long n, const char *cache_path) {
       return time_median([&] { return gmc_dec_batch_dev(K, key2, ct, n, nullptr, st); }, st, a, b, &rc);
     };
     // pipeline depth of the tcgen05 GEMM (both ops share it)
-    if (best.enc_engine == GEMM_TC || best.dec_engine == GEMM_TC) {
+    const bool enc_tc = best.enc_engine == GEMM_TC, dec_tc = best.dec_engine == GEMM_TC && !dec_few;
+    if (enc_tc || dec_tc) {
       const int stage_cand[3] = {4, 3, 2};
       float best_sum = 1e30f;
       for (int si = 0; si < 3; si++) {
@@ -281,10 +289,10 @@ extern "C" int gmc_autotune(int set, long long n, const char *cache_path) {
         t.gemm_stages = stage_cand[si];
         tune_put(set, t);
         const float me =
-            best.enc_engine == GEMM_TC
+            enc_tc
                 ? time_median([&] { return gmc_enc_batch_dev(P, ct, key, seeds, n, nullptr, st); }, st, a, b, &rc)
                 : best_enc;
-        const float md = best.dec_engine == GEMM_TC ? time_dec(t) : best_dec;
+        const float md = dec_tc ? time_dec(t) : best_dec;
         if (si == 0 || me + md < 0.99f * best_sum) {
           best_sum = me + md;
           best.gemm_stages = stage_cand[si];
@@ -298,7 +306,7 @@ extern "C" int gmc_autotune(int set, long long n, const char *cache_path) {
     // requests per block of the decoding kernels
     const int bm_cand[3] = {kBMWarps, 8, 4};
     const int warp_cand[3] = {kRootWarps, 4, 2};
-    if (n >= bm_bitsliced_min_rows(set_info(set).t))
+    if (dec_bm_bitsliced_form(set, seg_rows(segs), const_time))
       for (int wi = 1; wi < 3; wi++) {
         SetTune t = best;
         t.bm_warps = bm_cand[wi];
