@@ -302,9 +302,10 @@ int gmc_get_dec_constant_time(void);
  * of the decoding kernels (bm_warps: Berlekamp-Massey warps of 32 requests,
  * 1..14, default 14, not used by the constant-time form; root_warps:
  * root-finding warps of one request, 1..8, default 8, for batches below
- * 14000 rows) and the
+ * 14000 rows, and for constant-time and the server's batches of any size) and the
  * pipelined sampler's resident warps per SM (sample_sm_warps, 0 = the
- * default, 16); gmc_tune_set_launch / gmc_tune_get_launch set and read
+ * default, 16). A parameter that a batch of n requests does not use keeps its
+ * value (root_warps is timed on a smaller batch then). gmc_tune_set_launch / gmc_tune_get_launch set and read
  * them by hand. */
 int gmc_autotune(int set, long long n, const char *cache_path);
 int gmc_autotune_load(const char *cache_path);

@@ -316,15 +316,25 @@ extern "C" int gmc_autotune(int set, long long n, const char *cache_path) {
           best.bm_warps = bm_cand[wi];
         }
       }
-    for (int wi = 1; wi < 3 && n < kRootSlicedMinRows; wi++) {  // (larger batches take another root finder)
+    // A batch of the request-sliced root finder does not read root_warps, but a serving batch of its size does, and one
+    // whose scratch did not fit: it is timed on the largest batch of the warp-per-request form.
+    const bool sliced = dec_root_work_bytes(set, seg_rows(segs), const_time) != 0;
+    const long long n_root = sliced ? (kRootSlicedMinRows - 1) / kGemmOpPad * kGemmOpPad : n;
+    auto time_root = [&](const SetTune &t) {
+      tune_put(set, t);
+      return time_median([&] { return gmc_dec_batch_dev(K, key2, ct, n_root, nullptr, st); }, st, a, b, &rc);
+    };
+    float best_root = sliced ? time_root(best) : best_dec;
+    for (int wi = 1; wi < 3; wi++) {
       SetTune t = best;
       t.root_warps = warp_cand[wi];
-      const float ms = time_dec(t);
-      if (ms < 0.99f * best_dec) {
-        best_dec = ms;
+      const float ms = time_root(t);
+      if (ms < 0.99f * best_root) {
+        best_root = ms;
         best.root_warps = warp_cand[wi];
       }
     }
+    if (!sliced) best_dec = best_root;
     best.tuned = 1;
     best.enc_ms = best_enc;
     best.dec_ms = best_dec;

@@ -28,3 +28,10 @@ def test_small_batch_keeps_unread_parameters(gmc, sid, dec_engine):
     assert got["sample_sm_warps"] == 12 and got["bm_warps"] == 11
     if got["enc_engine"] != "tc":
         assert got["gemm_stages"] == 3
+
+
+def test_root_warps_above_the_sliced_line(gmc):
+    """Batches from 14000 rows take the request-sliced root finder, but the server's still read root_warps: a tune at
+    such a size replaces one warp per block (about a third of the speed of four)."""
+    gmc.tune_set(0, "sparse", "tc", 128, gemm_stages=4, bm_warps=14, root_warps=1, sample_sm_warps=0)
+    assert gmc.autotune(0, 16384)["root_warps"] > 1
