@@ -80,7 +80,10 @@ int gmc_key_import(gmc_key **out, const unsigned char *buf, long long len);
  * -1 only for a 6960119 key with nonzero padding bits, as the library).
  * _dev: all pointers are device pointers, work is queued on `stream`
  * (a cudaStream_t, 0 = default stream) and the call returns without waiting.
- * Without _dev: host pointers; the call copies in, runs and copies out.
+ * Without _dev: host pointers; the call copies in, runs and copies out. Small
+ * calls pass through a page-locked buffer of the calling thread (256 KB, kept
+ * until the thread ends), whose seeds and session keys are cleared before the
+ * call returns, also when it fails.
  * GMC_SAMPLE_PIPELINE=0 in the environment (read once) selects the
  * lane-per-request sampler instead of the pipelined one (same outputs). */
 int gmc_enc_batch_dev(const gmc_key *pk, unsigned char *c, unsigned char *k, const unsigned char *seeds,
@@ -336,6 +339,10 @@ int gmc_b1mma_peak(double *mac_per_s);
  * and the decode flags. For the staged parity tests. */
 int gmc_dec_stages_dev(const gmc_key *sk, const unsigned char *c, long long n, unsigned int *synd,
                        int synd_words, unsigned int *e, int e_words, int *ok, void *stream);
+/* Bytes that are not zero where the calling thread's last small host-pointer
+ * call had its seeds and session keys in the thread's page-locked buffer: 0
+ * between calls. For the tests. */
+long long gmc_host_stage_residue(void);
 /* Stage outputs of an encapsulation batch: error vectors and raw syndromes
  * T*e[mt:n] (device pointers). */
 int gmc_enc_stages_dev(const gmc_key *pk, const unsigned char *seeds, long long n, unsigned int *e,

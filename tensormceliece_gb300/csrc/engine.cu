@@ -473,22 +473,46 @@ struct Scratch {
 // lets the kernels read and write it in place: a batch of one spends longer in
 // four pageable copies than in its kernels (one encapsulation of 348864 88 us
 // with copies and separate allocations, 50 us now; one decapsulation call of
-// 8192128 163 / 136 us).
+// 8192128 163 / 136 us). The seeds and session keys in it are cleared before
+// the call returns (StageWipe).
 constexpr size_t kHostStageBytes = 256 * 1024;
+struct HostStage {
+  uint8_t *p = nullptr;
+  size_t secret_at = 0, secret_bytes = 0;  // the seeds and session keys of this thread's last staged call
+  ~HostStage() {
+    if (p) cudaFreeHost(p);
+  }
+};
+static thread_local HostStage t_stage;
 static uint8_t *host_stage(size_t bytes) {
-  struct Holder {
-    uint8_t *p = nullptr;
-    ~Holder() {
-      if (p) cudaFreeHost(p);
-    }
-  };
-  thread_local Holder h;
+  HostStage &h = t_stage;
   if (bytes > kHostStageBytes) return nullptr;
   if (!h.p && cudaHostAlloc((void **)&h.p, kHostStageBytes, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
     cudaGetLastError();
     h.p = nullptr;
   }
   return h.p;
+}
+// clears [at, at + bytes) of the staging buffer at the end of a call, on error returns too (after its last wait for
+// the stream)
+struct StageWipe {
+  StageWipe(size_t at, size_t bytes) {
+    t_stage.secret_at = at;
+    t_stage.secret_bytes = bytes;
+  }
+  ~StageWipe() {
+    uint8_t *p = t_stage.p + t_stage.secret_at;
+    memset(p, 0, t_stage.secret_bytes);
+    asm volatile("" : : "r"(p) : "memory");  // the stores are not dead
+  }
+  StageWipe(const StageWipe &) = delete;
+  StageWipe &operator=(const StageWipe &) = delete;
+};
+
+extern "C" long long gmc_host_stage_residue(void) {
+  long long n = 0;
+  for (size_t i = 0; i < t_stage.secret_bytes; i++) n += t_stage.p[t_stage.secret_at + i] != 0;
+  return n;
 }
 
 struct EncDims {
@@ -742,6 +766,7 @@ extern "C" int gmc_enc_batch(const gmc_key *pk, unsigned char *c, unsigned char 
   };
   const size_t k_at = (ct_b + 15) / 16 * 16;
   if (uint8_t *stage = host_stage(k_at + k_b + in_b)) {
+    const StageWipe wipe(k_at, k_b + in_b);
     uint8_t *s_k = stage + k_at, *s_in = s_k + k_b;
     memcpy(s_in, seeds, in_b);
     const int res = gmc_enc_batch_dev(pk, stage, s_k, s_in, n, nullptr, st);
@@ -787,6 +812,7 @@ extern "C" int gmc_dec_batch(const gmc_key *sk, unsigned char *k, const unsigned
   if (!st) return fail(GMC_ECUDA, "gmc_dec_batch: stream");
   const size_t k_at = (ct_b + 15) / 16 * 16, rc_at = k_at + k_b;
   if (uint8_t *stage = host_stage(rc_at + rc_b)) {
+    const StageWipe wipe(k_at, k_b);
     uint8_t *s_k = stage + k_at;
     int *s_rc = reinterpret_cast<int *>(stage + rc_at);
     memcpy(stage, c, ct_b);
