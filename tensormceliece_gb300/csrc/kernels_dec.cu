@@ -804,8 +804,10 @@ __global__ void __launch_bounds__((BMCtLayout<SET>::NS + 1) * 32, kBMCtBlocksPer
 // iteration is the bound there, and in it the discrepancy waits for the update
 // of C. d_{n+1} = e + f q with e = sum_i C_i s_{n+1-i} of the C before the update
 // and q = sum_i B_i s_{n+1-i}; when B becomes x C, q becomes that e, and else B is
-// multiplied by x while n grows by one, so q stays. So the dot product and the
-// update of C run at the same time, without branches on d. One request 58 -> 45
+// multiplied by x while n grows by one, so q stays, but for the term of a B_t that
+// the multiplication moves out of the fixed arrays (deg B <= n+1-L; it counts only
+// in sequences whose length ends above t: the next update makes L = n+1-L). So the
+// dot product and the update of C run at the same time, without branches on d. One request 58 -> 45
 // us, 2048 requests 74 -> 72; with full blocks the longer code loses (20000
 // requests 461 -> 508), where the bound is the bank conflicts of the table
 // lookups (about 9 shared-memory wavefronts a slot).
@@ -890,6 +892,10 @@ __global__ void __launch_bounds__((AHEAD ? kBMLatCopyWarps : kBMLatWarps) * 32, 
       for (; n < 2 * T; n++) {
         if (K < NS && (L > 32 * K || n + 1 - L > 32 * K)) return;
         if constexpr (AHEAD) {
+          if (K == NS && n - L >= T) {  // x moved B_t out of the array: its term leaves q
+            const uint32_t q = gexp[min(lq, (uint32_t)ZL)] ^ gf_mul_log<M>(gexp, blog[T + 1 - sft], slog[n - T]);
+            lq = glog[q];
+          }
           const uint16_t *sn = slog + n - lane, *bs = blog + 1 + lane - sft;
           const uint32_t ld = glog[d];
           const bool upd = d != 0 && n >= 2 * L;
