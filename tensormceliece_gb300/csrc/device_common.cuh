@@ -313,20 +313,4 @@ __device__ __forceinline__ uint16_t gf_mul_log(const uint16_t *__restrict__ ex, 
   return ex[s];
 }
 
-template <int M>
-__device__ __forceinline__ uint16_t gf_mul(const uint16_t *__restrict__ ex, const uint16_t *__restrict__ lg,
-                                           uint16_t a, uint16_t b) {
-  return gf_mul_log<M>(ex, lg[a], lg[b]);
-}
-
-// x mod (2^M - 1) for x < 2^(2M+?) small: two folds leave a value <= 2^M,
-// and exp[] is periodic with period 2^M - 1 over its first 2q-2 entries.
-template <int M>
-__device__ __forceinline__ int fold_mod(int x) {
-  constexpr int mask = (1 << M) - 1;
-  x = (x & mask) + (x >> M);
-  x = (x & mask) + (x >> M);
-  return x;
-}
-
 }  // namespace gmc

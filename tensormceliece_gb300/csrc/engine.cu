@@ -344,8 +344,6 @@ extern "C" int gmc_sk_load(gmc_key **out, int id, const unsigned char *sk) {
     return cuda_fail(e, "gmc_sk_load");
   }
   k->dk.L = k->tabs;
-  k->dk.LL = k->tabs + n;
-  k->dk.LW2 = k->tabs + 2 * n;
   k->dk.invL = k->tabs + 3 * n;
   k->dk.s = k->s;
   k->ldh = h.ldh;
@@ -552,7 +550,7 @@ static cudaError_t gemm_keys(const gmc_key *const *keys, int nkeys, int engine, 
 int gmc::dec_e_words(int set, bool ct) {
   const gmc_setinfo &S = set_info(set);
   const int tab = round_up((S.n + 31) / 32, 4);
-  return ct ? std::max(S.q / 32, round_up((S.n + 31) / 32, kGemmKTile)) : tab;
+  return ct ? S.q / 32 : tab;
 }
 
 // encapsulation kernels for the segments of one set: seeds / c / k rows in padded row space
@@ -648,6 +646,7 @@ static cudaError_t dec_front_decode_seg(const Segs &segs, const gmc_key *ref, co
   if (e != cudaSuccess) return e;
   prof_mark("dec_bm", st);
   e = launch_dec_root<SET>(Sig, dk, fd, segs, E, d.lde, ok, st, tune.root_warps, d.ct, d.root_work);
+  // (the labels of this stage and the next are kept for readers of gmc_prof_report; neither compares syndromes)
   prof_mark("dec_fft_roots_reenc", st);
   if (e != cudaSuccess || !d.ct) return e;
   // constant time: the Benes network to code positions

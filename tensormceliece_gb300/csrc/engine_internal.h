@@ -20,7 +20,8 @@ struct gmc_key {
   // secret key
   uint32_t *F = nullptr;
   int ldf = 0, frows_pad = 0, cw_pad = 0;
-  uint16_t *tabs = nullptr;  // L | LL | LW2 (n each) | invL (2^m)
+  // L | log L | log of 1/g(L)^2 (n each) | invL (2^m); the kernels read L and invL, exported key strings hold all
+  uint16_t *tabs = nullptr;
   uint8_t *a8 = nullptr;     // FP8 stage images of T (public) or F (secret) for the tensor-core engine
   std::mutex *a8_mu = nullptr;
   uint8_t *s = nullptr;
@@ -62,6 +63,6 @@ int field_tables(int set, FieldDev *out);
 // (FP8 image of its matrix, per-set tables), so later launches allocate nothing for it
 int key_prepare_resident(const gmc_key *key);
 // decapsulation rows of the error-vector buffer: the table form needs ceil(n/32) words, the constant-time form
-// the field-order vector (q/32 words); the latter's rows are whole GEMM K tiles
+// the field-order vector (q/32 words)
 int dec_e_words(int set, bool ct);
 }  // namespace gmc

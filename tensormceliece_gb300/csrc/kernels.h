@@ -206,8 +206,6 @@ cudaError_t launch_finalize(const uint32_t *E, int lde, const uint32_t *S, int l
 // Per-key decapsulation state on the device (built once per secret key).
 struct DecKeyDev {
   const uint16_t *L;     // support element of each code position [n]
-  const uint16_t *LL;    // log L_i (zero sentinel when L_i = 0) [n]
-  const uint16_t *LW2;   // log of 1/g(L_i)^2 [n]
   const uint16_t *invL;  // code position of each field element, 0xFFFF off the support [2^m]
   const uint8_t *s;      // implicit-rejection string [n/8]
   const uint32_t *cond;  // the sk's Benes control bits ((2m - 1) 2^(m-1) bits, as 32-bit words)

@@ -1,9 +1,11 @@
 // Decapsulation kernels.
 //
 //  pack_ct     ciphertext bytes -> 32-bit words (the front-end GEMM operand)
-//  decode      one warp per request: 2t syndromes (from the front-end GEMM)
-//              -> Berlekamp-Massey -> additive FFT over all 2^m field
-//              elements -> error positions at the key's support, weight
+//  decode      2t syndromes (from the front-end GEMM, or straight from the
+//              ciphertext bytes in small batches) -> Berlekamp-Massey ->
+//              additive FFT over all 2^m field elements -> error positions
+//              at the key's support, weight; a warp per request, or 32
+//              requests per word, by batch size
 //  dec_tail    K = SHAKE256(b || (e or s) || c), implicit rejection, and the
 //              6960119 ciphertext-padding rule
 //
@@ -13,8 +15,8 @@
 // mc:crypto_kem/6960119/vec/kem_dec.c:21-78). Only the outcome is defined
 // there: a weight-t error with the received syndrome is unique, so any exact
 // decoder yields the same session key. The BM update rule follows the
-// library's (mc:crypto_kem/348864/vec/bm.c:156), so locators agree with the
-// oracle's stage output as well.
+// library's (mc:crypto_kem/348864/vec/bm.c:156) on its fixed arrays of t + 1
+// coefficients, so locators agree with the oracle's stage output as well.
 #include <algorithm>
 #include <type_traits>
 
@@ -23,12 +25,6 @@
 #include "device_common.cuh"
 
 namespace gmc {
-
-__device__ __forceinline__ uint32_t warp_xor(uint32_t v) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) v ^= __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 
 // Copies a field table of n 16-bit entries to shared memory by the whole block,
 // 16 bytes a thread (both sides 16-byte aligned; n is rounded up to whole

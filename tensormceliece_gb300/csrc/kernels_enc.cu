@@ -420,10 +420,7 @@ __global__ void __launch_bounds__(kSampleThreadsMax)
                        unsigned int *__restrict__ counter, int groups) {
   using p = P<SET>;
   using LY = PipeLayout<SET>;
-  constexpr int PP = LY::perms, NG = LY::NG, RW = LY::raw_words, NCW = (p::t + 31) / 32;
-  constexpr int ncand = p::cand_bytes / 2;
-  constexpr uint32_t mask = p::q - 1;
-  constexpr int sh = p::mt % 32, w0 = p::mt / 32;
+  constexpr int PP = LY::perms, NG = LY::NG, RW = LY::raw_words;
   extern __shared__ __align__(16) uint32_t sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int half = lane & 1, pair = lane >> 1;

@@ -263,8 +263,6 @@ extern "C" int gmc_key_import(gmc_key **out, const unsigned char *buf, long long
   if (h.kind == 1) {
     const size_t n = S.n;
     k->dk.L = k->tabs;
-    k->dk.LL = k->tabs + n;
-    k->dk.LW2 = k->tabs + 2 * n;
     k->dk.invL = k->tabs + 3 * n;
     k->dk.s = k->s;
     k->ldh = h.ldh;
