@@ -1405,7 +1405,7 @@ done:
 // Semi-systematic keys: almost every attempt succeeds (the last 32 pivots come
 // from 64 columns), so a round gives every key one attempt and takes it
 // straight to the full elimination, control bits and assembly, and one link is
-// expanded ahead. 460896f, 200 keys: 17.2 ms, against 37.8 ms with 3 speculative
+// expanded ahead. 460896f, 200 keys: 15.1 ms, against 35.9 ms with 3 speculative
 // attempts per key, rank tests and 24 links expanded and waited for.
 template <int SET>
 int keypair_batch(uint8_t *pk, uint8_t *sk, const uint8_t *seeds, long long nkeys, bool semi, cudaStream_t s0,
